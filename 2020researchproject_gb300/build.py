@@ -27,6 +27,7 @@ CUDA_SOURCES = {
     "step32_kernels.cu": [],
     "krylov.cu": [],
     "multigrid.cu": [],
+    "fastpoisson.cu": [],
     "setup_kernels.cu": ["-fmad=false"],
     "solver.cu": [],
 }

@@ -22,6 +22,7 @@
 #include "geo3d.h"
 #include "kernels.h"
 #include "krylov.h"
+#include "fastpoisson.h"
 #include "multigrid.h"
 #include "ncfile.h"
 #include "prof.h"
@@ -117,7 +118,11 @@ struct ibm3d_device {
     IRWork irmom, irpres;
     GMG<double> *mg = nullptr;
     GMG<float> *mg32 = nullptr;
-    WidenedPreconditioner pc64;   // FP32 multigrid under an FP64 Krylov solve
+    // Fast-diagonalisation preconditioners, null where the multigrid serves
+    // the case (pres_pc32, pres_pc64).
+    FastPoisson<double> *fp64 = nullptr;
+    FastPoisson<float> *fp32 = nullptr;
+    WidenedPreconditioner pc64;   // FP32 preconditioner under an FP64 Krylov solve
     // IBM3D_MIXED32 pressure solve on double-float vectors: a view of
     // kpres's buffers, the solution vector and the FP32 multigrid behind it.
     KrylovWork<dfloat> kpres_df;
@@ -307,6 +312,10 @@ void release_device(ibm3d_device *d) {
     d->mg = nullptr;
     delete d->mg32;
     d->mg32 = nullptr;
+    delete d->fp64;
+    d->fp64 = nullptr;
+    delete d->fp32;
+    d->fp32 = nullptr;
     d->pc64.release();
     d->gm.release();
     d->kmom.release();
@@ -831,6 +840,49 @@ bool build_ops(IBMSolver *sv) {
     return cuda_check(sv, cudaStreamSynchronize(d->s), "operator tables");
 }
 
+// Fast-diagonalisation preconditioners (fastpoisson.h): in FP32 for every
+// case its axes allow, in FP64 without a body.
+bool build_fast_poisson(IBMSolver *sv) {
+    ibm3d_device *d = sv->dev;
+    const Grid &g = d->g;
+    const int Ns[3] = {sv->Nx, sv->Ny, sv->Nz};
+    const double *KM[3] = {sv->kx_W, sv->ky_S, sv->kz_D}, *KP[3] = {sv->kx_E, sv->ky_N, sv->kz_U};
+    const double *D[3] = {sv->dx, sv->dy, sv->dz};
+    FastPoissonGeom h;
+    for (int a = 0; a < 3; a++) {
+        h.km[a].assign(KM[a] + 2, KM[a] + 2 + Ns[a]);
+        h.kp[a].assign(KP[a] + 2, KP[a] + 2 + Ns[a]);
+        h.d[a].assign(D[a] + 2, D[a] + 2 + Ns[a]);
+    }
+    h.flag.resize(g.ncell);
+    bool body = false;
+    for (long long P = 0; P < g.ncell; P++) {
+        h.flag[P] = (uint8_t)sv->flag[P];
+        body = body || h.flag[P] != FLUID;
+    }
+    const int ng = d->nghost;
+    h.gcell.resize(ng);
+    h.gidx.resize(8 * (size_t)ng);
+    h.gwself.resize(ng);
+    if (ng > 0) {
+        cudaMemcpyAsync(h.gcell.data(), d->gargs.cell, sizeof(int) * ng, cudaMemcpyDeviceToHost, d->s);
+        cudaMemcpyAsync(h.gidx.data(), d->g_gidx, sizeof(int) * 8 * ng, cudaMemcpyDeviceToHost, d->s);
+        cudaMemcpyAsync(h.gwself.data(), d->g_gwself, sizeof(double) * ng, cudaMemcpyDeviceToHost, d->s);
+        if (!cuda_check(sv, cudaStreamSynchronize(d->s), "preconditioner tables")) return false;
+    }
+    auto make = [&](auto *&fp, auto &A) {
+        fp = new std::remove_reference_t<decltype(*fp)>();
+        const int rc = fp->setup(d->s, d->A64, A, h);
+        if (rc != 0) {
+            delete fp;
+            fp = nullptr;
+        }
+        if (rc < 0) set_status(sv, IBM3D_ECUDA, "preconditioner setup failed");
+        return rc >= 0;
+    };
+    return make(d->fp32, d->A32) && (body || make(d->fp64, d->A64));
+}
+
 void swap3(double *a[3], double *b[3]) {
     for (int l = 0; l < 3; l++) std::swap(a[l], b[l]);
 }
@@ -1071,11 +1123,17 @@ bool pres_df(const IBMSolver *sv) {
 }
 Preconditioner<dfloat> *pres_pcdf(IBMSolver *sv) { return &sv->dev->pcdf; }
 
+// FP32 preconditioner of the mixed modes' pressure solves.
+Preconditioner<float> *pres_pc32(const ibm3d_device *d) {
+    return d->fp32 ? (Preconditioner<float> *)d->fp32 : (Preconditioner<float> *)d->mg32;
+}
+
 // Preconditioner of an FP64 pressure Krylov solve.
 Preconditioner<double> *pres_pc64(IBMSolver *sv) {
     ibm3d_device *d = sv->dev;
     if (!use_mg(sv)) return nullptr;
-    return d->precision != IBM3D_FP64 ? (Preconditioner<double> *)&d->pc64 : (Preconditioner<double> *)d->mg;
+    if (d->precision != IBM3D_FP64) return &d->pc64;
+    return d->fp64 ? (Preconditioner<double> *)d->fp64 : (Preconditioner<double> *)d->mg;
 }
 
 void stage_rhs(IBMSolver *sv) {
@@ -1222,7 +1280,7 @@ void one_step(IBMSolver *sv) {
     if (pres_gmres(sv))
         rc = gmres(d->s, d->A64, OP_PRES, d->gm, d->b, d->pp, pp, pres_pc64(sv), d->rep_p);
     else if (pres_ir(sv))
-        rc = solve_ir(d->s, d->A64, d->A32, OP_PRES, d->irpres, d->b, d->pp, pp, use_mg(sv) ? d->mg32 : nullptr,
+        rc = solve_ir(d->s, d->A64, d->A32, OP_PRES, d->irpres, d->b, d->pp, pp, use_mg(sv) ? pres_pc32(d) : nullptr,
                       d->rep_p);
     else if (pres_df(sv))
         rc = bicgstab_df(d->s, d->Adf, OP_PRES, d->kpres_df, d->pp_df, d->b, d->pp, pp, pres_pcdf(sv), d->rep_p);
@@ -1293,7 +1351,7 @@ bool record_step_into(IBMSolver *sv, StepGraph &G) {
                               &pi) == 0;
         else if (pres_ir(sv))
             ok = record_ir(d->s, d->aux, d->A64, d->A32, OP_PRES, d->irpres, d->b, d->pp, pp,
-                           use_mg(sv) ? d->mg32 : nullptr, &pf, &po, &pi) == 0;
+                           use_mg(sv) ? pres_pc32(d) : nullptr, &pf, &po, &pi) == 0;
         else if (pres_df(sv))
             ok = record_bicgstab_df(d->s, d->aux, d->Adf, OP_PRES, d->kpres_df, d->pp_df, d->b, d->pp, pp,
                                     pres_pcdf(sv), &pf, &pi) == 0;
@@ -1755,7 +1813,8 @@ void IBMSolver_assemble(IBMSolver *s) {
     }
     d->mg->set_prof(&d->prof);
     d->mg32->set_prof(&d->prof);
-    if (d->pc64.allocate(g.ncell, d->mg32) != 0) {
+    if (!build_fast_poisson(s)) return;
+    if (d->pc64.allocate(g.ncell, pres_pc32(d)) != 0) {
         set_status(s, IBM3D_ECUDA, "preconditioner workspace allocation failed");
         return;
     }
