@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "krylov.h"
+#include "momsweep.h"
 #include "prof.h"
 
 namespace ibm {
@@ -234,12 +235,18 @@ __device__ __forceinline__ void sweep_rows(const OpT<T> &A, const bool (&run)[NC
 // reach), ||r||^2 and the divergence max of r; a guess that already passes
 // the stopping test ends the solve before its first iteration.  b as in
 // k_bicg_init.
+// after (momentum only): the sweeps that came before; when they ended the
+// solve nothing runs, else their count starts the iteration count.  outer
+// (increment solves): the norms that fix the stopping test, as in
+// k_bicg_init.
 template <typename T, int NC, typename B = T>
 __global__ void __launch_bounds__(SW_THREADS, std::is_same<T, dfloat>::value ? 4 : 1)
 k_bicg_init_guess(const OpT<T> A, const int op, const long long n, const B *__restrict__ b, const T *__restrict__ x,
                   T *r, KScal *sc, double *partials, unsigned int *counter, const double tol,
-                  const double divtol, const LoopCtl lc) {
+                  const double divtol, const LoopCtl lc, const MScal *__restrict__ after,
+                  const IRScal *__restrict__ outer, const double outer_tol, const int maxit) {
     pdl_enter();
+    if (after && (after->state == MS_A || after->state == MS_B)) return;
     __shared__ double smem[32 * (2 * NC + 1)];
     typename AccT<T>::type a[2 * NC + 1];
     bool run[NC];
@@ -276,14 +283,16 @@ k_bicg_init_guess(const OpT<T> A, const int op, const long long n, const B *__re
             s.alpha = 1.0;
             s.omega = 1.0;
             s.beta = 0.0;
-            s.iters = 0;
+            s.iters = after ? after->sweeps : 0;
             s.tol = tol;
+            if (outer && outer[c].rnorm2 > 0)
+                s.tol = fmax(tol, 0.5 * outer_tol * sqrt(outer[c].bnorm2 / outer[c].rnorm2));
             s.divtol = divtol;
             s.divmax = tot[2 * NC];
             s.restart = 1;   // the first p update sets p = r0 = r
-            const bool done = tot[NC + c] == 0.0 || converged(tot[NC + c], s.bnorm2, tot[2 * NC], tol, divtol);
+            const bool done = tot[NC + c] == 0.0 || converged(tot[NC + c], s.bnorm2, tot[2 * NC], s.tol, divtol);
             s.state = done ? KS_DONE : KS_RUN;
-            go = go || !done;
+            go = go || (!done && s.iters < maxit);
         }
         set_loop(lc, go);
     });
@@ -837,13 +846,14 @@ static void launch_init(cudaStream_t st, KrylovWork<T> &w, const B *b, T *x, dou
 
 template <typename T, typename B>
 static void launch_init_guess(cudaStream_t st, const OpT<T> &A, int op, KrylovWork<T> &w, const B *b, const T *x,
-                              double tol, double divtol, LoopCtl lc) {
+                              double tol, double divtol, LoopCtl lc, int maxit, const MScal *after = nullptr,
+                              const IRScal *outer = nullptr, double outer_tol = 0.0) {
     if (w.nc == 3)
         launch_pdl(k_bicg_init_guess<T, 3, B>, A.sw.nblocks, SW_THREADS, 0, st, A, op, w.n, b, x, w.r, w.scal,
-                   w.partials, w.counter, tol, divtol, lc);
+                   w.partials, w.counter, tol, divtol, lc, after, outer, outer_tol, maxit);
     else
         launch_pdl(k_bicg_init_guess<T, 1, B>, A.sw.nblocks, SW_THREADS, 0, st, A, op, w.n, b, x, w.r, w.scal,
-                   w.partials, w.counter, tol, divtol, lc);
+                   w.partials, w.counter, tol, divtol, lc, after, outer, outer_tol, maxit);
     note_launches(1);
 }
 
@@ -1092,7 +1102,7 @@ static void host_loop(cudaStream_t st, const OpT<T> &A, int op, KrylovWork<T> &w
 template <typename T>
 int bicgstab(cudaStream_t st, const OpT<T> &A, int op, KrylovWork<T> &w, const T *b, T *x, const SolveParams &prm,
              Preconditioner<T> *M, SolveReport &rep) {
-    if (prm.x_given) launch_init_guess(st, A, op, w, b, x, prm.tol, prm.divtol, LoopCtl());
+    if (prm.x_given) launch_init_guess(st, A, op, w, b, x, prm.tol, prm.divtol, LoopCtl(), prm.maxit);
     else launch_init(st, w, b, x, prm.tol, prm.divtol, nullptr, 0.0, 0.0, LoopCtl());
     host_loop(st, A, op, w, x, prm.maxit, M, prm.prof);
     return report(w, rep);
@@ -1119,7 +1129,7 @@ int bicgstab_df(cudaStream_t st, const OpT<dfloat> &A, int op, KrylovWork<dfloat
     const long long m = w.n * w.nc;
     if (prm.x_given) {
         launch_to_dfloat(st, m, x, xw);
-        launch_init_guess(st, A, op, w, b, xw, prm.tol, prm.divtol, LoopCtl());
+        launch_init_guess(st, A, op, w, b, xw, prm.tol, prm.divtol, LoopCtl(), prm.maxit);
     } else {
         launch_init(st, w, b, xw, prm.tol, prm.divtol, nullptr, 0.0, 0.0, LoopCtl());
     }
@@ -1241,7 +1251,7 @@ int record_bicgstab(cudaStream_t st, const cudaStream_t *aux, const OpT<T> &A, i
                     T *x, const SolveParams &prm, Preconditioner<T> *M, int *fixed, int *per_iter) {
     LoopCtl lc;
     if (new_loop(st, lc) != 0) return -1;
-    if (prm.x_given) launch_init_guess(st, A, op, w, b, x, prm.tol, prm.divtol, lc);
+    if (prm.x_given) launch_init_guess(st, A, op, w, b, x, prm.tol, prm.divtol, lc, prm.maxit);
     else launch_init(st, w, b, x, prm.tol, prm.divtol, nullptr, 0.0, 0.0, lc);
     if (record_loop(st, aux[0], A, op, w, x, prm.maxit, M, lc, per_iter) != 0) return -1;
     cudaMemcpyAsync(w.scal_h, w.scal, sizeof(KScal) * w.nc, cudaMemcpyDeviceToHost, st);
@@ -1265,7 +1275,7 @@ int record_bicgstab_df(cudaStream_t st, const cudaStream_t *aux, const OpT<dfloa
     if (new_loop(st, lc) != 0) return -1;
     if (prm.x_given) {
         launch_to_dfloat(st, m, x, xw);
-        launch_init_guess(st, A, op, w, b, xw, prm.tol, prm.divtol, lc);
+        launch_init_guess(st, A, op, w, b, xw, prm.tol, prm.divtol, lc, prm.maxit);
     } else {
         launch_init(st, w, b, xw, prm.tol, prm.divtol, nullptr, 0.0, 0.0, lc);
     }
@@ -1323,6 +1333,414 @@ void apply_operator(cudaStream_t st, const OpT<T> &A, int op, int comp, const T 
 
 template void apply_operator<double>(cudaStream_t, const OpT<double> &, int, int, const double *, double *);
 template void apply_operator<float>(cudaStream_t, const OpT<float> &, int, int, const float *, float *);
+
+// ============================================ Jacobi sweeps (momentum) ==
+// Design and choice: momsweep.h.  A sweep is two launches: k_mom_sweep
+// updates the fluid (and solid) rows of the three components from one
+// buffer into the other and reduces the residual of the values it read;
+// k_mom_rows then sets the new buffer's ghost and outer values.  The
+// buffers alternate; the result always ends in the first one.
+
+// Value of an outer cell that solves its row (outer_row with OP_MOM), from
+// interior values: the coordinates outside are resolved z, then y, then x,
+// the order in which the faces own the outer cells.
+template <typename T, int AX>
+__device__ __forceinline__ T mom_outer(const OpT<T> &c, const int comp, const T *x, const T *b, int i, int j, int k) {
+    if constexpr (AX < 0) {
+        return x[cidx(c.g, i, j, k)];
+    } else {
+        const int q = AX == 0 ? i : AX == 1 ? j : k, n = AX == 0 ? c.g.nx : AX == 1 ? c.g.ny : c.g.nz;
+        if (q >= 0 && q < n) return mom_outer<T, AX - 1>(c, comp, x, b, i, j, k);
+        const bool low = q < 0;
+        const int L = low ? -q : q - n + 1;
+        const BCRow<T> &F = c.bc[AX == 0 ? (low ? F_W : F_E) : AX == 1 ? (low ? F_S : F_N) : (low ? F_D : F_U)];
+        const T rv = b[cidx(c.g, i, j, k)];
+        auto at = [&](int p) {
+            return mom_outer<T, AX - 1>(c, comp, x, b, AX == 0 ? p : i, AX == 1 ? p : j, AX == 2 ? p : k);
+        };
+        const int m = low ? L - 1 : n - L;   // the mirror cell
+        switch (outer_row_kind(OP_MOM, F.type, comp, AX)) {
+        case ROW_DIR: return (rv - F.dir_m[L - 1] * at(m)) / F.dir_o[L - 1];
+        case ROW_NEU: return rv + at(m);
+        case ROW_PER: return rv + x[periodic_image(c.g, i, j, k)];
+        default: break;
+        }
+        // Three-point extrapolation; layer 2 from layer 1.
+        const T a0 = at(low ? 0 : n - 1), a1 = at(low ? 1 : n - 2);
+        const int q1 = low ? -1 : n;
+        const T r1 = b[cidx(c.g, AX == 0 ? q1 : i, AX == 1 ? q1 : j, AX == 2 ? q1 : k)];
+        const T x1 = (r1 + a0 - F.ext_2[0] * a1) / F.ext_o[0];
+        return L == 1 ? x1 : (rv + x1 - F.ext_2[1] * a0) / F.ext_o[1];
+    }
+}
+
+// Ghost rows, blocks [0, gblocks), and the outer rows of the list, the
+// other blocks; one thread per row and component.  Ghost entries that are
+// ghosts or outer cells are read from the old buffer xo (null: zeros).
+// ends: the launch belongs to a sweep into the first buffer, which is
+// completed even when that sweep's test has just ended the solve; always:
+// no gate.
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_mom_rows(const OpT<T> c, const long long n, const T *__restrict__ b, const T *__restrict__ xo, T *xn,
+           const int *__restrict__ gcell, const uint8_t *__restrict__ gold, const int ng, const int gblocks,
+           const int *__restrict__ outer, const int nout, const MScal *ms, const int ends, const int always) {
+    pdl_enter();
+    const int state = ms->state;
+    if (!always && state != MS_RUN && !(ends && (state == MS_B || state == MS_FALL_B))) return;
+    if ((int)blockIdx.x < gblocks) {
+        const int t = blockIdx.x * 256 + threadIdx.x;
+        if (t >= 3 * ng) return;
+        const int l = t / ng, g = t - l * ng;
+        const long long o = l * n;
+        T sum = 0;
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            const int q = c.gidx[8 * g + e];
+            if (q < 0) continue;
+            const T v = !gold[8 * g + e] ? xn[o + q] : xo ? xo[o + q] : (T)0;
+            sum += c.gw[8 * g + e] * v;
+        }
+        const int P = gcell[g];
+        xn[o + P] = (b[o + P] - sum) / ((T)1 + c.gwself[g]);
+        return;
+    }
+    const int t = (blockIdx.x - gblocks) * 256 + threadIdx.x;
+    if (t >= 3 * nout) return;
+    const int l = t / nout, P = outer[t - l * nout];
+    int i, j, k;
+    cijk_fast(c.g, c.fdx, c.fdy, P, i, j, k);
+    const long long o = l * n;
+    xn[o + P] = mom_outer<T, 2>(c, l, xn + o, b + o, i, j, k);
+}
+
+__device__ __forceinline__ float ms_rcp(float d) { return __frcp_rn(d); }
+// A relaxation weight needs no more than FP32 accuracy; formed off the FP64
+// pipe.
+__device__ __forceinline__ double ms_rcp(double d) { return f2d_int(__frcp_rn(d2f_int(d))); }
+
+// MODE 0: a sweep xo -> xn with the test on xo.  MODE 1: the first sweep
+// from x = 0 (xn = c / D; ||b||^2, unless ir has the norms).  MODE 2: the
+// first sweep from a guess, which also sums ||b||^2 and the outer rows'
+// residual.  Threads march over planes of i as in sweep_rows, the three
+// components together: the flag, the diagonal and its reciprocal serve all
+// three, x's planes stay in registers.  FP32: bound by its bytes (36 per
+// cell); FP64: by the FP64 pipe (28 operations per cell).
+template <typename T, int MODE>
+__global__ void __launch_bounds__(SW_THREADS)
+k_mom_sweep(const OpT<T> A, const long long n, const T *__restrict__ b, const T *__restrict__ xo, T *__restrict__ xn,
+            MScal *ms, KScal *sc, const IRScal *__restrict__ ir, const double tol, const double outer_tol,
+            const int limit, const int into_first, double *partials, unsigned int *counter, const LoopCtl lc) {
+    pdl_enter();
+    if (MODE == 0 && ms->state != MS_RUN) return;
+    constexpr int NV = MODE == 2 ? 6 : 3;
+    __shared__ double smem[32 * NV];
+    typename AccT<T>::type a[NV];
+#pragma unroll
+    for (int q = 0; q < NV; q++) a[q] = 0;
+    int i0, i1, j, k;
+    if (sweep_column(A.sw, A.g, i0, i1, j, k)) {
+        if (j < A.g.ny && k < A.g.nz) {
+            const Column<T> q = column(A, j, k);
+            const T d0 = (T)1 + q.ksy + q.ksz;
+            const long long sx = A.g.sx, sy = A.g.sy;
+            long long P = cidx(A.g, i0, j, k);
+            T xw[3], xc[3];
+            if (MODE != 1) {
+#pragma unroll
+                for (int l = 0; l < 3; l++) {
+                    xw[l] = xo[l * n + P - sx];
+                    xc[l] = xo[l * n + P];
+                }
+            }
+            for (int i = i0; i < i1; i++, P += sx) {
+                const uint8_t fl = A.flag[P];
+                const T D = d0 + A.ks[0][i + 2], W = ms_rcp(D);
+                const T kmx = A.km[0][i + 2], kpx = A.kp[0][i + 2];
+                T y[3], r[3];
+#pragma unroll
+                for (int l = 0; l < 3; l++) {
+                    const long long o = l * n + P;
+                    const T bv = b[o];
+                    if (MODE == 1) {
+                        r[l] = bv;
+                        y[l] = fl == FLUID ? W * bv : bv;
+                    } else {
+                        const T xe = xo[o + sx];
+                        const T nb = sum6(kmx, xw[l], kpx, xe, q.kmy, xo[o - sy], q.kpy, xo[o + sy], q.kmz, xo[o - 1],
+                                          q.kpz, xo[o + 1]);
+                        r[l] = bv + (nb - D * xc[l]);
+                        y[l] = xc[l] + W * r[l];
+                        if (fl != FLUID) {
+                            r[l] = bv - xc[l];
+                            y[l] = bv;
+                        }
+                        if (fl == GHOST) {
+                            const int g = A.gid[P];
+                            T sum = 0;
+#pragma unroll
+                            for (int e = 0; e < 8; e++) {
+                                const int m = A.gidx[8 * g + e];
+                                if (m >= 0) sum += A.gw[8 * g + e] * xo[l * n + m];
+                            }
+                            r[l] = bv - (((T)1 + A.gwself[g]) * xc[l] + sum);
+                        }
+                        xw[l] = xc[l];
+                        xc[l] = xe;
+                        if (MODE == 2) mac(a[3 + l], bv, bv);
+                    }
+                    mac(a[l], r[l], r[l]);
+                }
+                if (fl != GHOST) {
+#pragma unroll
+                    for (int l = 0; l < 3; l++) xn[l * n + P] = y[l];
+                }
+            }
+        }
+    } else {
+        const int t = sweep_outer(A.sw);
+        if (t < A.sw.nout) {
+            const long long P = A.sw.outer[t];
+#pragma unroll
+            for (int l = 0; l < 3; l++) {
+                const T bv = b[l * n + P];
+                const T r = MODE == 1 ? bv : bv - op_row(A, OP_MOM, l, xo + l * n, P);
+                mac(a[l], r, r);
+                if (MODE == 2) mac(a[3 + l], bv, bv);
+            }
+        }
+    }
+    reduce_and_finish<NV, NV>(a, smem, partials, counter, [&](const double *tot) {
+        MScal &s = *ms;
+        if (MODE != 0) {
+            s.sweeps = 0;
+            s.state = MS_RUN;
+            for (int c = 0; c < 3; c++) {
+                s.iters[c] = -1;
+                s.bn2[c] = ir ? ir[c].rnorm2 : MODE == 2 ? tot[3 + c] : tot[c];
+                if (MODE == 2 && s.bn2[c] == 0.0) s.bn2[c] = tot[c];
+            }
+        }
+        bool all = true, finite = true;
+        for (int c = 0; c < 3; c++) {
+            double t = ir ? tol : fmax(MS_MARGIN * tol, fmin(tol, 1e-13));
+            if (ir && ir[c].rnorm2 > 0) t = fmax(tol, MS_MARGIN * outer_tol * sqrt(ir[c].bnorm2 / ir[c].rnorm2));
+            s.rn2[c] = MODE == 1 ? s.bn2[c] : tot[c];
+            const bool ok = s.bn2[c] == 0.0 || (MODE != 1 && converged(s.rn2[c], s.bn2[c], 0.0, t, 0.0));
+            if (ok && s.iters[c] < 0) s.iters[c] = s.sweeps;
+            all = all && ok;
+            finite = finite && isfinite(s.rn2[c]);
+        }
+        if (all) {
+            s.state = MODE == 1 || into_first ? MS_B : MS_A;
+            for (int c = 0; c < 3; c++) {
+                KScal &q = sc[c];
+                q.bnorm2 = s.bn2[c];
+                q.rnorm2 = s.rn2[c];
+                q.iters = s.iters[c];
+                q.state = KS_DONE;
+                q.divmax = 0.0;
+            }
+        } else if (s.sweeps >= limit || !finite) {
+            s.state = into_first ? MS_FALL_B : MS_FALL;
+        }
+        if (s.state != MS_A && s.state != MS_FALL) s.sweeps++;
+        set_loop(lc, s.state == MS_RUN);
+    });
+}
+
+void MomSweep::release() {
+    if (outer1) cudaFree(outer1);
+    if (gold) cudaFree(gold);
+    if (scal) cudaFree(scal);
+    outer1 = nullptr;
+    gold = nullptr;
+    scal = nullptr;
+    use = false;
+}
+
+int MomSweep::setup(cudaStream_t s, const Grid &g, const double *const ks[3], const uint8_t *flag,
+                    const int *gcell_dev, const int *gc, const int *gidx, int nghost) {
+    release();
+    const int n[3] = {g.nx, g.ny, g.nz};
+    double sum = 0;
+    for (int a = 0; a < 3; a++) sum += *std::max_element(ks[a], ks[a] + n[a]);
+    rho = sum / (1 + sum);
+    use = rho <= MS_RHO;
+    if (!use) return 0;
+    ng = nghost;
+    gcell = gcell_dev;
+    split = full = false;
+    // The faces' first layer: one coordinate one cell outside, the others
+    // inside (the outer cells fluid rows read).
+    auto layer1 = [&](long long P) {
+        int i, j, k;
+        cijk(g, P, i, j, k);
+        const int q[3] = {i, j, k};
+        int out = 0, far = 0;
+        for (int a = 0; a < 3; a++) {
+            out += q[a] < 0 || q[a] >= n[a];
+            far += q[a] < -1 || q[a] > n[a];
+        }
+        return out == 1 && far == 0;
+    };
+    std::vector<int> o1;
+    for (long long P = 0; P < g.ncell; P++) {
+        const int k = (int)(P % g.sy);
+        if (k == 2 && n[2] > 4) {   // inside along k: only rows at the other faces matter
+            const long long row = P / g.sy;
+            const int J = (int)(row % (g.ny + 4)), I = (int)(row / (g.ny + 4));
+            if (I >= 2 && I < g.nx + 2 && J >= 2 && J < g.ny + 2) {
+                P += n[2] - 1;
+                continue;
+            }
+        }
+        if (layer1(P)) o1.push_back((int)P);
+    }
+    nout1 = (int)o1.size();
+    std::vector<uint8_t> old(8 * (size_t)ng, 0);
+    for (int q = 0; q < ng; q++) {
+        int i, j, k;
+        cijk(g, gc[q], i, j, k);
+        split = split || i < 2 || i >= n[0] - 2 || j < 2 || j >= n[1] - 2 || k < 2 || k >= n[2] - 2;
+        for (int e = 0; e < 8; e++) {
+            const int P = gidx[8 * (size_t)q + e];
+            if (P < 0) continue;
+            cijk(g, P, i, j, k);
+            const bool in = i >= 0 && i < n[0] && j >= 0 && j < n[1] && k >= 0 && k < n[2];
+            old[8 * (size_t)q + e] = !in || flag[P] == GHOST;
+            full = full || (!in && !layer1(P));
+        }
+    }
+    if (cudaMalloc(&outer1, sizeof(int) * std::max<size_t>(1, o1.size())) != cudaSuccess ||
+        cudaMalloc(&gold, std::max<size_t>(1, old.size())) != cudaSuccess ||
+        cudaMalloc(&scal, sizeof(MScal)) != cudaSuccess)
+        return -1;
+    cudaMemsetAsync(scal, 0, sizeof(MScal), s);
+    cudaMemcpyAsync(outer1, o1.data(), sizeof(int) * o1.size(), cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(gold, old.data(), old.size(), cudaMemcpyHostToDevice, s);
+    return cudaStreamSynchronize(s) == cudaSuccess ? 0 : -1;
+}
+
+// Ghost and outer rows of the buffer a sweep has just written; returns the
+// number of launches.
+template <typename T>
+static int launch_rows(cudaStream_t st, const OpT<T> &A, const MomSweep &ms, const KrylovWork<T> &w, const T *b,
+                       const T *xo, T *xn, int ends, int always) {
+    const int gb = (3 * ms.ng + 255) / 256;
+    const int *outer = ms.full ? A.sw.outer : ms.outer1;
+    const int no = ms.full ? A.sw.nout : ms.nout1, ob = (3 * no + 255) / 256;
+    if (ms.split && gb > 0) {
+        launch_pdl(k_mom_rows<T>, gb, 256, 0, st, A, w.n, b, xo, xn, ms.gcell, (const uint8_t *)ms.gold, ms.ng, gb,
+                   outer, 0, (const MScal *)ms.scal, ends, always);
+        launch_pdl(k_mom_rows<T>, ob, 256, 0, st, A, w.n, b, xo, xn, ms.gcell, (const uint8_t *)ms.gold, 0, 0, outer,
+                   no, (const MScal *)ms.scal, ends, always);
+        return 2;
+    }
+    launch_pdl(k_mom_rows<T>, gb + ob, 256, 0, st, A, w.n, b, xo, xn, ms.gcell, (const uint8_t *)ms.gold, ms.ng, gb,
+               outer, no, (const MScal *)ms.scal, ends, always);
+    return 1;
+}
+
+// The sweep that starts the solve; true when it wrote the first buffer x.
+template <typename T>
+static bool launch_first(cudaStream_t st, const OpT<T> &A, MomSweep &ms, KrylovWork<T> &w, const T *b, T *x,
+                         const SolveParams &prm, const IRScal *ir, int limit, LoopCtl lc, int *k) {
+    const double tol = ir ? prm.inner_tol : prm.tol;
+    if (prm.x_given && !ir) {
+        launch_pdl(k_mom_sweep<T, 2>, A.sw.nblocks, SW_THREADS, 0, st, A, w.n, b, (const T *)x, w.r, ms.scal, w.scal,
+                   ir, tol, prm.tol, limit, 0, w.partials, w.counter, lc);
+        *k += 1 + launch_rows(st, A, ms, w, b, (const T *)x, w.r, 0, 0);
+        return false;
+    }
+    launch_pdl(k_mom_sweep<T, 1>, ir ? A.sw.nint : A.sw.nblocks, SW_THREADS, 0, st, A, w.n, b, (const T *)nullptr, x,
+               ms.scal, w.scal, ir, tol, prm.tol, limit, 1, w.partials, w.counter, lc);
+    *k += 1 + launch_rows(st, A, ms, w, b, (const T *)nullptr, x, 1, 1);
+    return true;
+}
+
+template <typename T>
+static int launch_sweep(cudaStream_t st, const OpT<T> &A, MomSweep &ms, KrylovWork<T> &w, const T *b, T *x,
+                        const SolveParams &prm, const IRScal *ir, int limit, bool into_first, LoopCtl lc) {
+    const T *xo = into_first ? w.r : x;
+    T *xn = into_first ? x : w.r;
+    launch_pdl(k_mom_sweep<T, 0>, A.sw.nint, SW_THREADS, 0, st, A, w.n, b, xo, xn, ms.scal, w.scal, ir,
+               ir ? prm.inner_tol : prm.tol, prm.tol, limit, into_first ? 1 : 0, w.partials, w.counter, lc);
+    return 1 + launch_rows(st, A, ms, w, b, xo, xn, into_first ? 1 : 0, 0);
+}
+
+// Every outer row of the result, and BiCGSTAB from it when the sweeps have
+// not converged.
+template <typename T>
+static int launch_end(cudaStream_t st, const OpT<T> &A, MomSweep &ms, KrylovWork<T> &w, const T *b, T *x,
+                      const SolveParams &prm, const IRScal *ir, LoopCtl lc) {
+    launch_pdl(k_mom_rows<T>, (3 * A.sw.nout + 255) / 256, 256, 0, st, A, w.n, b, (const T *)nullptr, x, ms.gcell,
+               (const uint8_t *)ms.gold, 0, 0, A.sw.outer, A.sw.nout, (const MScal *)ms.scal, 1, 1);
+    launch_init_guess(st, A, OP_MOM, w, b, (const T *)x, ir ? prm.inner_tol : prm.tol, 0.0, lc, prm.maxit,
+                      (const MScal *)ms.scal, ir, prm.tol);
+    return 1;
+}
+
+static int sweep_limit(const SolveParams &prm) { return std::min(MS_LIMIT, prm.maxit); }
+
+template <typename T>
+int solve_sweeps(cudaStream_t st, const OpT<T> &A, MomSweep &ms, KrylovWork<T> &w, const T *b, T *x,
+                 const SolveParams &prm, const IRScal *ir, SolveReport &rep) {
+    const LoopCtl none;
+    const int limit = sweep_limit(prm);
+    int k = 0;
+    MScal h;
+    auto running = [&]() {
+        cudaMemcpyAsync(&h, ms.scal, sizeof h, cudaMemcpyDeviceToHost, st);
+        cudaStreamSynchronize(st);
+        return h.state == MS_RUN;
+    };
+    if (!launch_first(st, A, ms, w, b, x, prm, ir, limit, none, &k))
+        k += launch_sweep(st, A, ms, w, b, x, prm, ir, limit, true, none);
+    while (running()) {
+        k += launch_sweep(st, A, ms, w, b, x, prm, ir, limit, false, none);
+        k += launch_sweep(st, A, ms, w, b, x, prm, ir, limit, true, none);
+    }
+    k += launch_end(st, A, ms, w, b, x, prm, ir, none);
+    note_launches(k);
+    if (h.state == MS_A || h.state == MS_B) fetch(st, w);
+    else host_loop<T>(st, A, OP_MOM, w, x, std::max(0, prm.maxit - h.sweeps), nullptr, prm.prof);
+    return report(w, rep);
+}
+
+template <typename T>
+int record_sweeps(cudaStream_t st, const cudaStream_t *aux, const OpT<T> &A, MomSweep &ms, KrylovWork<T> &w,
+                  const T *b, T *x, const SolveParams &prm, const IRScal *ir, int *per_iter, int *idle) {
+    const int limit = sweep_limit(prm);
+    LoopCtl sweeps, rest;
+    if (new_loop(st, sweeps) != 0 || new_loop(st, rest) != 0) return -1;
+    int k = 0, body = 0;
+    if (!launch_first(st, A, ms, w, b, x, prm, ir, limit, sweeps, &k))
+        k += launch_sweep(st, A, ms, w, b, x, prm, ir, limit, true, sweeps);
+    if (begin_while(st, sweeps, aux[0]) != 0) return -1;
+    body += launch_sweep(aux[0], A, ms, w, b, x, prm, ir, limit, false, sweeps);
+    body += launch_sweep(aux[0], A, ms, w, b, x, prm, ir, limit, true, sweeps);
+    if (end_while(aux[0]) != 0) return -1;
+    k += launch_end(st, A, ms, w, b, x, prm, ir, rest);
+    int it = 0;
+    if (record_loop<T>(st, aux[0], A, OP_MOM, w, x, prm.maxit, nullptr, rest, &it) != 0) return -1;
+    cudaMemcpyAsync(w.scal_h, w.scal, sizeof(KScal) * w.nc, cudaMemcpyDeviceToHost, st);
+    note_launches(k + body);
+    *per_iter = (body + 1) / 2;
+    *idle = it + body - *per_iter;
+    return 0;
+}
+
+template int solve_sweeps<double>(cudaStream_t, const OpT<double> &, MomSweep &, KrylovWork<double> &, const double *,
+                                  double *, const SolveParams &, const IRScal *, SolveReport &);
+template int solve_sweeps<float>(cudaStream_t, const OpT<float> &, MomSweep &, KrylovWork<float> &, const float *,
+                                 float *, const SolveParams &, const IRScal *, SolveReport &);
+template int record_sweeps<double>(cudaStream_t, const cudaStream_t *, const OpT<double> &, MomSweep &,
+                                   KrylovWork<double> &, const double *, double *, const SolveParams &,
+                                   const IRScal *, int *, int *);
+template int record_sweeps<float>(cudaStream_t, const cudaStream_t *, const OpT<float> &, MomSweep &,
+                                  KrylovWork<float> &, const float *, float *, const SolveParams &, const IRScal *,
+                                  int *, int *);
 
 // ================================================== flexible GMRES (FP64) ==
 // One restart cycle: V[0] = r / beta; for j = 0, 1, ...: z_j = M V[j]

@@ -22,6 +22,7 @@
 #include "geo3d.h"
 #include "kernels.h"
 #include "krylov.h"
+#include "momsweep.h"
 #include "fastpoisson.h"
 #include "multigrid.h"
 #include "ncfile.h"
@@ -116,6 +117,7 @@ struct ibm3d_device {
     // BiCGSTAB (mixed path), each with its multigrid preconditioner.
     KrylovWork<double> kmom, kpres;
     IRWork irmom, irpres;
+    MomSweep msweep;              // momentum by Jacobi sweeps (msweep.use) instead of BiCGSTAB
     GMG<double> *mg = nullptr;
     GMG<float> *mg32 = nullptr;
     // Fast-diagonalisation preconditioners, null where the multigrid serves
@@ -319,6 +321,7 @@ void release_device(ibm3d_device *d) {
     d->pc64.release();
     d->gm.release();
     d->kmom.release();
+    d->msweep.release();
     d->kpres.release();
     d->kpres_df.release();
     dfree(d->pp_df);
@@ -840,9 +843,10 @@ bool build_ops(IBMSolver *sv) {
     return cuda_check(sv, cudaStreamSynchronize(d->s), "operator tables");
 }
 
-// Fast-diagonalisation preconditioners (fastpoisson.h): in FP32 for every
-// case its axes allow, in FP64 without a body.
-bool build_fast_poisson(IBMSolver *sv) {
+// Tables of the momentum sweeps (momsweep.h), and the fast-diagonalisation
+// preconditioners (fastpoisson.h): in FP32 for every case its axes allow,
+// in FP64 without a body.
+bool build_sweeps_and_poisson(IBMSolver *sv) {
     ibm3d_device *d = sv->dev;
     const Grid &g = d->g;
     const int Ns[3] = {sv->Nx, sv->Ny, sv->Nz};
@@ -869,6 +873,14 @@ bool build_fast_poisson(IBMSolver *sv) {
         cudaMemcpyAsync(h.gidx.data(), d->g_gidx, sizeof(int) * 8 * ng, cudaMemcpyDeviceToHost, d->s);
         cudaMemcpyAsync(h.gwself.data(), d->g_gwself, sizeof(double) * ng, cudaMemcpyDeviceToHost, d->s);
         if (!cuda_check(sv, cudaStreamSynchronize(d->s), "preconditioner tables")) return false;
+    }
+    std::vector<double> ks[3];
+    for (int a = 0; a < 3; a++)
+        for (int q = 0; q < Ns[a]; q++) ks[a].push_back(h.km[a][q] + h.kp[a][q]);
+    const double *const kp[3] = {ks[0].data(), ks[1].data(), ks[2].data()};
+    if (d->msweep.setup(d->s, g, kp, h.flag.data(), d->gargs.cell, h.gcell.data(), h.gidx.data(), ng) != 0) {
+        set_status(sv, IBM3D_ECUDA, "momentum sweep tables failed");
+        return false;
     }
     auto make = [&](auto *&fp, auto &A) {
         fp = new std::remove_reference_t<decltype(*fp)>();
@@ -1260,6 +1272,27 @@ void check_pres(IBMSolver *sv, int rc) {
     else if (rc == 2) set_status(sv, IBM3D_EBREAKDOWN, "breakdown in the pressure solve");
 }
 
+// Momentum by Jacobi sweeps: the FP32 increment of the FP32-stage step, or
+// u* in FP64 (from u^n in the mixed modes).
+bool mom_sweeps(const ibm3d_device *d) { return d->msweep.use; }
+
+// ||b|| and ||c|| of the increment system, for report_inc.
+void fetch_increment_norms(ibm3d_device *d) {
+    cudaMemcpyAsync(d->irmom.scal_h, d->irmom.scal, sizeof(IRScal) * 3, cudaMemcpyDeviceToHost, d->s);
+}
+
+int momentum_sweeps(IBMSolver *sv, const SolveParams &pm) {
+    ibm3d_device *d = sv->dev;
+    if (!step32(d))
+        return solve_sweeps<double>(d->s, d->A64, d->msweep, d->kmom, d->b, d->ustar, pm, nullptr,
+                                    d->rep_mom = SolveReport());
+    solve_sweeps<float>(d->s, d->A32, d->msweep, d->irmom.inner, d->irmom.b32, d->irmom.e32, pm, d->irmom.scal,
+                        d->rep_mom);
+    fetch_increment_norms(d);
+    cudaStreamSynchronize(d->s);
+    return report_inc(d->irmom, sv->tol, d->rep_mom);
+}
+
 // One fractional step, host-sequenced (used while stage profiling is on).
 void one_step(IBMSolver *sv) {
     ibm3d_device *d = sv->dev;
@@ -1268,7 +1301,8 @@ void one_step(IBMSolver *sv) {
     const SolveParams pm = mom_params(sv);
     int t = pf.begin("mom_solve");
     momentum_guess(sv, pm);
-    int rc = step32(d)  ? solve_inc(d->s, d->A32, OP_MOM, d->irmom, pm, d->rep_mom)
+    int rc = mom_sweeps(d) ? momentum_sweeps(sv, pm)
+             : step32(d)  ? solve_inc(d->s, d->A32, OP_MOM, d->irmom, pm, d->rep_mom)
              : mom_ir(d) ? solve_ir(d->s, d->A64, d->A32, OP_MOM, d->irmom, d->b, d->ustar, pm, nullptr, d->rep_mom)
                          : bicgstab<double>(d->s, d->A64, OP_MOM, d->kmom, d->b, d->ustar, pm, nullptr, d->rep_mom);
     pf.end(t);
@@ -1332,7 +1366,13 @@ bool record_step_into(IBMSolver *sv, StepGraph &G) {
         SolveParams pm = mom_params(sv);
         pm.prof = nullptr;
         momentum_guess(sv, pm);
-        if (step32(d))
+        if (mom_sweeps(d)) {
+            ok = (step32(d) ? record_sweeps<float>(d->s, d->aux, d->A32, d->msweep, d->irmom.inner, d->irmom.b32,
+                                                   d->irmom.e32, pm, d->irmom.scal, &mi, &mo)
+                            : record_sweeps<double>(d->s, d->aux, d->A64, d->msweep, d->kmom, d->b, d->ustar, pm,
+                                                    nullptr, &mi, &mo)) == 0;
+            if (step32(d)) fetch_increment_norms(d);
+        } else if (step32(d))
             ok = record_inc(d->s, d->aux, d->A32, OP_MOM, d->irmom, pm, &mf, &mi) == 0;
         else if (mom_ir(d))
             ok = record_ir(d->s, d->aux, d->A64, d->A32, OP_MOM, d->irmom, d->b, d->ustar, pm, nullptr, &mf, &mo,
@@ -1421,10 +1461,11 @@ void finish_step(IBMSolver *sv, const StepGraph &G) {
     int rc;
     if (step32(d)) {
         rc = report_inc(d->irmom, sv->tol, d->rep_mom);
-    } else if (mom_ir(d)) {
+    } else if (mom_ir(d) && !mom_sweeps(d)) {
         rc = report(d->irmom, d->rep_mom);
         launches += (long long)d->rep_mom.outer * G.mom_outer;
     } else {
+        d->rep_mom = SolveReport();
         rc = report(d->kmom, d->rep_mom);
     }
     launches += (long long)std::max({d->rep_mom.iters[0], d->rep_mom.iters[1], d->rep_mom.iters[2]}) * G.mom_iter;
@@ -1813,7 +1854,7 @@ void IBMSolver_assemble(IBMSolver *s) {
     }
     d->mg->set_prof(&d->prof);
     d->mg32->set_prof(&d->prof);
-    if (!build_fast_poisson(s)) return;
+    if (!build_sweeps_and_poisson(s)) return;
     if (d->pc64.allocate(g.ncell, pres_pc32(d)) != 0) {
         set_status(s, IBM3D_ECUDA, "preconditioner workspace allocation failed");
         return;
