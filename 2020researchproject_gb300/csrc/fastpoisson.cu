@@ -1,6 +1,8 @@
 // Fast-diagonalisation preconditioner of the pressure rows (fastpoisson.h).
 #include <algorithm>
+#include <array>
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -31,129 +33,177 @@ __device__ __forceinline__ T fp_outer(const BCRow<T> &F, T ro) {
 }
 
 // ---------------------------------------------------------------- gather --
-// The padded residual as the compact source coeffsum r of the separable
-// system: 0 on solid rows and the pinned row, scaled on ghost rows, with
-// the outer rows' residuals folded into the rows beside them.  Padding
-// columns (k >= nz) are 0.  Bound by its bytes (8 read, 4 written per cell
-// from double-float residuals).  Grid (ld / 32, ny / 8, nx / 4).
+// The source of one interior cell: coeffsum r, 0 on solid rows and the
+// pinned row, scaled on ghost rows, the residuals of the outer rows beside
+// it folded in.
+template <typename T, typename S>
+__device__ __forceinline__ T fp_source(const OpT<T> &c, const S *__restrict__ r, T v, const long long P, const int i,
+                                       const int j, const int k, const uint8_t fl, const T *__restrict__ gscale) {
+    const Grid &g = c.g;
+    v *= c.ks[0][i + 2] + c.ks[1][j + 2] + c.ks[2][k + 2];
+    if (fl == GHOST) v *= gscale[c.gid[P]];
+    else if (fl != FLUID) v = 0;
+    if (i == 0 || i == g.nx - 1 || j == 0 || j == g.ny - 1 || k == 0 || k == g.nz - 1) {
+        if (fl == FLUID) {
+            if (i == 0) v += c.km[0][2] * fp_outer(c.bc[F_W], fp_value<T, S>(r[P - g.sx]));
+            if (i == g.nx - 1) v += c.kp[0][i + 2] * fp_outer(c.bc[F_E], fp_value<T, S>(r[P + g.sx]));
+            if (j == 0) v += c.km[1][2] * fp_outer(c.bc[F_S], fp_value<T, S>(r[P - g.sy]));
+            if (j == g.ny - 1) v += c.kp[1][j + 2] * fp_outer(c.bc[F_N], fp_value<T, S>(r[P + g.sy]));
+            if (k == 0) v += c.km[2][2] * fp_outer(c.bc[F_D], fp_value<T, S>(r[P - 1]));
+            if (k == g.nz - 1) v += c.kp[2][k + 2] * fp_outer(c.bc[F_U], fp_value<T, S>(r[P + 1]));
+        }
+        if (c.p_singular && P == c.pinned) v = 0;
+    }
+    return v;
+}
+
+// The padded residual as the compact source of the separable system.  On a
+// mirror-symmetric z axis (z.fold) a thread takes the cells k and nz-1-k and
+// writes their sum to column k and their difference to column off + k, the
+// inputs of the even and the odd modes.  Columns that hold no value are 0.
+// Bound by its bytes (8 read, 4 written per cell from double-float
+// residuals); every plane's loads are issued before any is used (128^2
+// planes of 192: 24 -> 20 us, cold).  Grid (off / 32, ny / 8, nx / 4).
 constexpr int FP_GPLANES = 4;
 
 template <typename T, typename S>
 __global__ void __launch_bounds__(256)
-k_fp_gather(const OpT<T> c, const S *__restrict__ r, T *__restrict__ f, const int ld, const int body,
+k_fp_gather(const OpT<T> c, const S *__restrict__ r, T *__restrict__ f, const FpModes z, const int ld, const int body,
             const T *__restrict__ gscale, const int *gate) {
     FP_GATE(gate);
     const Grid &g = c.g;
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
-    if (k >= ld || j >= g.ny) return;
-    const bool in = k < g.nz;
-    const int kk = min(k, g.nz - 1);
-    const T ksyz = c.ks[1][j + 2] + c.ks[2][kk + 2];
-    const bool edge = j == 0 || j == g.ny - 1 || kk == 0 || kk == g.nz - 1;
+    const int q = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+    if (q >= z.off || j >= g.ny) return;
+    const int i0 = blockIdx.z * FP_GPLANES;
+    const int k1 = min(q, g.nz - 1), k2 = z.fold ? max(g.nz - 1 - q, 0) : k1;
+    S a[FP_GPLANES], b[FP_GPLANES];
+    uint8_t fa[FP_GPLANES], fb[FP_GPLANES];
 #pragma unroll
     for (int p = 0; p < FP_GPLANES; p++) {
-        const int i = blockIdx.z * FP_GPLANES + p;
-        if (i >= g.nx) break;
-        const long long P = cidx(g, i, j, kk);
-        T v = (c.ks[0][i + 2] + ksyz) * fp_value<T, S>(r[P]);
+        const long long P = cidx(g, min(i0 + p, g.nx - 1), j, 0);
+        a[p] = r[P + k1];
+        if (z.fold) b[p] = r[P + k2];
+        fa[p] = fb[p] = FLUID;
         if (body) {
-            const uint8_t fl = c.flag[P];
-            if (fl == GHOST) v *= gscale[c.gid[P]];
-            else if (fl != FLUID) v = 0;
+            fa[p] = c.flag[P + k1];
+            if (z.fold) fb[p] = c.flag[P + k2];
         }
-        if (edge || i == 0 || i == g.nx - 1) {
-            if (!body || c.flag[P] == FLUID) {
-                if (i == 0) v += c.km[0][2] * fp_outer(c.bc[F_W], fp_value<T, S>(r[P - g.sx]));
-                if (i == g.nx - 1) v += c.kp[0][i + 2] * fp_outer(c.bc[F_E], fp_value<T, S>(r[P + g.sx]));
-                if (j == 0) v += c.km[1][2] * fp_outer(c.bc[F_S], fp_value<T, S>(r[P - g.sy]));
-                if (j == g.ny - 1) v += c.kp[1][j + 2] * fp_outer(c.bc[F_N], fp_value<T, S>(r[P + g.sy]));
-                if (kk == 0) v += c.km[2][2] * fp_outer(c.bc[F_D], fp_value<T, S>(r[P - 1]));
-                if (kk == g.nz - 1) v += c.kp[2][kk + 2] * fp_outer(c.bc[F_U], fp_value<T, S>(r[P + 1]));
-            }
-            if (c.p_singular && P == c.pinned) v = 0;
+    }
+#pragma unroll
+    for (int p = 0; p < FP_GPLANES; p++) {
+        const int i = i0 + p;
+        if (i >= g.nx) break;
+        const long long P = cidx(g, i, j, 0);
+        T *row = f + ((long long)i * g.ny + j) * ld;
+        T v = fp_source<T, S>(c, r, fp_value<T, S>(a[p]), P + k1, i, j, k1, fa[p], gscale);
+        if (!z.fold) {
+            row[q] = q < g.nz ? v : (T)0;
+            continue;
         }
-        f[((long long)i * g.ny + j) * ld + k] = in ? v : (T)0;
+        T d = 0;
+        if (q < z.no) {
+            const T w = fp_source<T, S>(c, r, fp_value<T, S>(b[p]), P + k2, i, j, k2, fb[p], gscale);
+            d = v - w;
+            v += w;
+        }
+        row[q] = q < z.ne ? v : (T)0;
+        if (z.off + q < ld) row[z.off + q] = d;
     }
 }
 
 // ------------------------------------------------------------ transforms --
-// C = A B for row-major operands in tiles of TM x TM, 64 threads with an
-// R x R register tile each (as 2 x 2 sub-tiles, so that shared-memory reads
-// are conflict-free 16-byte ones or broadcasts), the k loop in steps of 16
-// through two shared-memory buffers with the next step's loads in flight.
-// TA = false: A(m, k) with k contiguous (the data, when the contiguous axis
-// is transformed); TA = true: A given as its transpose, (k, m) with m
-// contiguous (the axis matrix, applied to another axis).  A and C or B and
-// C advance by their batch strides.  out (with SCATTER): row m is the grid
-// line (i, j), written to the padded array, shifted so that the pinned cell
-// takes its residual's value.  Bound by the FP32 (FP64) multiply-add pipe.
-template <typename T>
-struct FpTile;
-template <>
-struct FpTile<float> {
-    static constexpr int TM = 64, R = 8, V = 4;
-};
-template <>
-struct FpTile<double> {
-    static constexpr int TM = 32, R = 4, V = 2;
+// Dense transforms as tiled products C = A B, 64 threads with register
+// tiles of R x R made of 2 x 2 sub-tiles (shared-memory reads are
+// conflict-free vectors or broadcasts), k in steps of 16 through two
+// shared-memory buffers with the next step's loads in flight.  Bound by the
+// FP32 (FP64) multiply-add pipe.
+//
+// On a mirror-symmetric axis the modes are even or odd, so a transform
+// splits into two of half the size, half the multiplications: forward, from
+// the sums and differences of mirrored cells (k_fp_gemm: formed by the
+// gather along z, while loading along x and y); backward, both parities'
+// parts E and O of the first half's cells at once, x_i = E + O and
+// x_(n-1-i) = E - O (k_fp_back).
+//
+// Sphere 192x128x128 FP32, cold: forward z 26 -> 16, forward y 25 -> 21,
+// backward y 25 -> 25, backward z 27 -> 22 us (half the products; the loads
+// of both halves and the register tiles' shared-memory reads bound them
+// now); cavity 64^3 FP64, an application: 0.36 -> 0.23 ms.
+//
+// Tiles: TM = 64 (R = 8) in FP32, 32 (R = 4) in FP64 and on FP32 grids whose
+// 64-tiles would leave SMs without a block (run).
+template <typename T, int TM>
+struct FpTile {
+    static constexpr int R = TM / 8, R2 = R / 2, V = 16 / (int)sizeof(T);
+    static constexpr int VR = R2 < V ? R2 : V;   // elements per shared-memory read
 };
 constexpr int FP_TK = 16;
 
+template <typename T, int N>
+struct alignas(sizeof(T) * N) FpVec {
+    T v[N];
+};
+
+// Operands per parity (blockIdx.z & 1 when nb = 2); batch strides over the
+// remaining part of blockIdx.z.
 template <typename T>
 struct FpGemm {
-    const T *a, *b;
-    T *c;
-    int M, N, K;
-    int lda, ldb, ldc;
-    long long sa, sb, sc;   // batch strides
+    const T *a[2], *b[2];
+    T *c[2];
+    int M[2], N[2], K[2];
+    int lda[2], ldb[2], ldc;
+    long long sb, sc;
+    int nb;
+    int fold;   // > 0: row k of B is B(k) + sign B(fold - 1 - k), sign by parity
 };
 
-template <typename T, typename S>
-struct FpScatter {
-    Grid g;
-    FastDiv dny;
-    const S *r;             // residual (pinned shift)
-    const T *brow;          // row 0 of the backward transform's result basis: V(0, .)
-    long long pinned;
-    int singular;
-};
-
-template <typename T, bool TA, bool SCATTER, typename S>
+// TA = false: A(m, k) with k contiguous (the data, when the contiguous axis
+// is transformed); TA = true: A given as its transpose, (k, m) with m
+// contiguous (the axis matrix, applied to another axis).
+template <typename T, int TM, bool TA>
 __global__ void __launch_bounds__(64)
-k_fp_gemm(const FpGemm<T> p, const FpScatter<T, S> sc, const int *gate) {
+k_fp_gemm(const FpGemm<T> p, const int *gate) {
     FP_GATE(gate);
-    constexpr int TM = FpTile<T>::TM, R = FpTile<T>::R, V = FpTile<T>::V, H = TM / 2, R2 = R / 2;
+    using Tile = FpTile<T, TM>;
+    constexpr int R = Tile::R, R2 = Tile::R2, V = Tile::V, VR = Tile::VR, H = TM / 2;
     constexpr int PITCH = TA ? TM : TM + V;
     constexpr int NQ = TM * FP_TK / V / 64;   // vector loads per thread and operand
-    struct alignas(16) Vec {
-        T v[V];
-    };
+    using Vec = FpVec<T, V>;
+    using Rd = FpVec<T, VR>;
     __shared__ alignas(16) T As[2][FP_TK][PITCH];
     __shared__ alignas(16) T Bs[2][FP_TK][TM];
-    const T *A = p.a + blockIdx.z * p.sa, *B = p.b + blockIdx.z * p.sb;
+    const int par = p.nb == 2 ? blockIdx.z & 1 : 0, batch = p.nb == 2 ? blockIdx.z >> 1 : blockIdx.z;
+    const T *A = par ? p.a[1] : p.a[0], *B = (par ? p.b[1] : p.b[0]) + batch * p.sb;
+    const int M = par ? p.M[1] : p.M[0], N = par ? p.N[1] : p.N[0], K = par ? p.K[1] : p.K[0];
+    const int lda = par ? p.lda[1] : p.lda[0], ldb = par ? p.ldb[1] : p.ldb[0];
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TM;
+    if (m0 >= M || n0 >= N) return;
     const int t = threadIdx.x, tx = t & 7, ty = t >> 3;
     Vec ra[NQ], rb[NQ];
     auto load = [&](int k0) {
 #pragma unroll
         for (int q = 0; q < NQ; q++) {
             const int e = t + 64 * q;
-            {
-                constexpr int PER = TM / V;
-                const int k = k0 + e / PER, n = n0 + (e % PER) * V;
-                if (k < p.K && n < p.N) rb[q] = *reinterpret_cast<const Vec *>(B + (long long)k * p.ldb + n);
-                else rb[q] = Vec{};
-                if (TA) {
-                    const int m = m0 + (e % PER) * V;
-                    if (k < p.K && m < p.lda) ra[q] = *reinterpret_cast<const Vec *>(A + (long long)k * p.lda + m);
-                    else ra[q] = Vec{};
+            constexpr int PER = TM / V;
+            const int k = k0 + e / PER, n = n0 + (e % PER) * V;
+            rb[q] = Vec{};
+            if (k < K && n < N) {
+                rb[q] = *reinterpret_cast<const Vec *>(B + (long long)k * ldb + n);
+                const int km = p.fold - 1 - k;
+                if (TA && p.fold && km != k) {
+                    const Vec m = *reinterpret_cast<const Vec *>(B + (long long)km * ldb + n);
+#pragma unroll
+                    for (int l = 0; l < V; l++) rb[q].v[l] = par ? rb[q].v[l] - m.v[l] : rb[q].v[l] + m.v[l];
                 }
             }
-            if (!TA) {
-                constexpr int PER = FP_TK / V;
-                const int m = m0 + e / PER, k = k0 + (e % PER) * V;
-                if (m < p.M && k < p.lda) ra[q] = *reinterpret_cast<const Vec *>(A + (long long)m * p.lda + k);
-                else ra[q] = Vec{};
+            ra[q] = Vec{};
+            if (TA) {
+                const int m = m0 + (e % PER) * V;
+                if (k < K && m < lda) ra[q] = *reinterpret_cast<const Vec *>(A + (long long)k * lda + m);
+            } else {
+                constexpr int PK = FP_TK / V;
+                const int m = m0 + e / PK, ka = k0 + (e % PK) * V;
+                if (m < M && ka < K) ra[q] = *reinterpret_cast<const Vec *>(A + (long long)m * lda + ka);
             }
         }
     };
@@ -161,12 +211,11 @@ k_fp_gemm(const FpGemm<T> p, const FpScatter<T, S> sc, const int *gate) {
 #pragma unroll
         for (int q = 0; q < NQ; q++) {
             const int e = t + 64 * q;
-            constexpr int PER = TM / V;
+            constexpr int PER = TM / V, PK = FP_TK / V;
             *reinterpret_cast<Vec *>(&Bs[buf][e / PER][(e % PER) * V]) = rb[q];
             if (TA) {
                 *reinterpret_cast<Vec *>(&As[buf][e / PER][(e % PER) * V]) = ra[q];
             } else {
-                constexpr int PK = FP_TK / V;
 #pragma unroll
                 for (int l = 0; l < V; l++) As[buf][(e % PK) * V + l][e / PK] = ra[q].v[l];
             }
@@ -177,25 +226,12 @@ k_fp_gemm(const FpGemm<T> p, const FpScatter<T, S> sc, const int *gate) {
     for (int x = 0; x < R; x++)
 #pragma unroll
         for (int y = 0; y < R; y++) acc[x][y] = 0;
-    T shift = 0;
-    if (SCATTER && sc.singular) {
-        // z(0,0,0) of the unshifted solution: one line's product, by every
-        // block for itself.
-        __shared__ T red[2];
-        T s = 0;
-        for (int q = t; q < p.K; q += 64) s += A[q] * sc.brow[(long long)q * p.ldb];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((t & 31) == 0) red[t >> 5] = s;
-        __syncthreads();
-        shift = fp_value<T, S>(sc.r[sc.pinned]) - (red[0] + red[1]);
-    }
     load(0);
     store(0);
     __syncthreads();
     int buf = 0;
-    for (int k0 = 0; k0 < p.K; k0 += FP_TK) {
-        const bool more = k0 + FP_TK < p.K;
+    for (int k0 = 0; k0 < K; k0 += FP_TK) {
+        const bool more = k0 + FP_TK < K;
         if (more) load(k0 + FP_TK);
 #pragma unroll
         for (int k = 0; k < FP_TK; k++) {
@@ -203,9 +239,9 @@ k_fp_gemm(const FpGemm<T> p, const FpScatter<T, S> sc, const int *gate) {
 #pragma unroll
             for (int h = 0; h < 2; h++) {
 #pragma unroll
-                for (int l = 0; l < R2; l += V) {
-                    *reinterpret_cast<Vec *>(&av[h * R2 + l]) = *reinterpret_cast<const Vec *>(&As[buf][k][h * H + ty * R2 + l]);
-                    *reinterpret_cast<Vec *>(&bv[h * R2 + l]) = *reinterpret_cast<const Vec *>(&Bs[buf][k][h * H + tx * R2 + l]);
+                for (int l = 0; l < R2; l += VR) {
+                    *reinterpret_cast<Rd *>(&av[h * R2 + l]) = *reinterpret_cast<const Rd *>(&As[buf][k][h * H + ty * R2 + l]);
+                    *reinterpret_cast<Rd *>(&bv[h * R2 + l]) = *reinterpret_cast<const Rd *>(&Bs[buf][k][h * H + tx * R2 + l]);
                 }
             }
 #pragma unroll
@@ -219,38 +255,214 @@ k_fp_gemm(const FpGemm<T> p, const FpScatter<T, S> sc, const int *gate) {
             buf ^= 1;
         }
     }
+    T *C = (par ? p.c[1] : p.c[0]) + batch * p.sc;
 #pragma unroll
     for (int x = 0; x < R; x++) {
         const int m = m0 + (x / R2) * H + ty * R2 + x % R2;
-        if (m >= p.M) continue;
-        if (SCATTER) {
-            const int i = (int)fdiv(sc.dny, (uint32_t)m), j = m - i * sc.g.ny;
-            T *row = p.c + cidx(sc.g, i, j, 0);
-            const bool pair = ((sc.g.sy | sc.g.sx) & 1) == 0;
+        if (m >= M) continue;
+        T *row = C + (long long)m * p.ldc;
 #pragma unroll
-            for (int y = 0; y < R; y += 2) {
-                const int n = n0 + (y / R2) * H + tx * R2 + y % R2;
-                struct alignas(2 * sizeof(T)) Two {
-                    T v[2];
-                };
-                if (pair && n + 1 < sc.g.nz) {
-                    *reinterpret_cast<Two *>(row + n) = Two{{acc[x][y] + shift, acc[x][y + 1] + shift}};
+        for (int y = 0; y < R; y += VR) {
+            const int n = n0 + (y / R2) * H + tx * R2 + y % R2;
+            if (n < N) {
+                Rd o;
+#pragma unroll
+                for (int l = 0; l < VR; l++) o.v[l] = acc[x][y + l];
+                *reinterpret_cast<Rd *>(row + n) = o;
+            }
+        }
+    }
+}
+
+// Where the last backward transform (along z) writes: the padded array,
+// grid line (i, j) per row, shifted so that the pinned cell takes its
+// residual's value.
+template <typename T, typename S>
+struct FpScatter {
+    Grid g;
+    const S *r;             // residual (pinned shift)
+    const T *v0;            // z(0, 0, 0) of line (0, 0) in terms of its modes
+    long long pinned;
+    int singular, ld;
+};
+
+template <typename T, typename S>
+__device__ __forceinline__ T fp_shift(const FpScatter<T, S> &sc, const T *__restrict__ line) {
+    if (!sc.singular) return 0;
+    // z(0,0,0) of the unshifted solution: one line's product, by every
+    // block for itself.
+    __shared__ T red[2];
+    const int t = threadIdx.x;
+    T s = 0;
+    for (int q = t; q < sc.ld; q += 64) s += line[q] * sc.v0[q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((t & 31) == 0) red[t >> 5] = s;
+    __syncthreads();
+    return fp_value<T, S>(sc.r[sc.pinned]) - (red[0] + red[1]);
+}
+
+// Backward transform of an axis, one product for both parities: E = Ae Be
+// and O = Ao Bo over the first half's cells.  ROWS (the contiguous axis): A
+// is the data, row m its modes (even, then odd from column off), B the axis
+// matrices (mode, cell); the result goes to the padded array.  Otherwise A
+// holds the axis matrices (mode, cell), B the data's mode rows (even, then
+// odd from row ne), and C receives rows i and n - 1 - i.  An axis without
+// the symmetry passes fold = 0: E alone over all its cells.
+template <typename T>
+struct FpBack {
+    const T *a[2], *b[2];
+    T *c;
+    int M, N;               // rows and columns of E
+    int K[2];
+    int lda[2], ldb[2], ldc;
+    long long sb, sc;       // batch strides (blockIdx.z)
+    int fold, n;            // fold: both parities; n: cells of the axis
+};
+
+template <typename T, int TM, bool ROWS, bool FOLD, typename S>
+__global__ void __launch_bounds__(64)
+k_fp_back(const FpBack<T> p, const FpScatter<T, S> sc, const int *gate) {
+    FP_GATE(gate);
+    using Tile = FpTile<T, TM>;
+    constexpr int R = Tile::R, V = Tile::V, VR = Tile::VR;
+    constexpr int NP = FOLD ? 2 : 1;
+    // The side that is halved by the two parities sharing the tile.
+    constexpr int MA = FOLD && !ROWS ? TM / 2 : TM, NB = FOLD && ROWS ? TM / 2 : TM;
+    constexpr int RA = MA / 8, RB = NB / 8;              // register tile per parity
+    constexpr int GA = RA == R ? 2 : 1, GB = RB == R ? 2 : 1;   // sub-tile groups
+    constexpr int PITCH = ROWS ? MA + V : MA;
+    constexpr int QA = MA * FP_TK / V / 64, QB = NB * FP_TK / V / 64;
+    static_assert(QA >= 1 && QB >= 1, "tile too small for 64 threads");
+    using Vec = FpVec<T, V>;
+    using Rd = FpVec<T, VR>;
+    __shared__ alignas(16) T As[2][NP][FP_TK][PITCH];
+    __shared__ alignas(16) T Bs[2][NP][FP_TK][NB];
+    const int m0 = blockIdx.y * MA, n0 = blockIdx.x * NB;
+    const int t = threadIdx.x, tx = t & 7, ty = t >> 3;
+    Vec ra[NP][QA], rb[NP][QB];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int h = 0; h < NP; h++) {
+            const T *A = p.a[h], *B = p.b[h] + blockIdx.z * p.sb;
+#pragma unroll
+            for (int q = 0; q < QB; q++) {
+                const int e = t + 64 * q, k = k0 + e / (NB / V), n = n0 + (e % (NB / V)) * V;
+                rb[h][q] = Vec{};
+                if (k < p.K[h] && n < p.ldb[h]) rb[h][q] = *reinterpret_cast<const Vec *>(B + (long long)k * p.ldb[h] + n);
+            }
+#pragma unroll
+            for (int q = 0; q < QA; q++) {
+                const int e = t + 64 * q;
+                ra[h][q] = Vec{};
+                if (ROWS) {
+                    const int m = m0 + e / (FP_TK / V), k = k0 + (e % (FP_TK / V)) * V;
+                    if (m < p.M && k < p.K[h]) ra[h][q] = *reinterpret_cast<const Vec *>(A + (long long)m * p.lda[h] + k);
                 } else {
-                    if (n < sc.g.nz) row[n] = acc[x][y] + shift;
-                    if (n + 1 < sc.g.nz) row[n + 1] = acc[x][y + 1] + shift;
+                    const int k = k0 + e / (MA / V), m = m0 + (e % (MA / V)) * V;
+                    if (k < p.K[h] && m < p.lda[h]) ra[h][q] = *reinterpret_cast<const Vec *>(A + (long long)k * p.lda[h] + m);
                 }
             }
-        } else {
-            T *row = p.c + blockIdx.z * p.sc + (long long)m * p.ldc;
+        }
+    };
+    auto store = [&](int buf) {
 #pragma unroll
-            for (int y = 0; y < R; y += V) {
-                const int n = n0 + (y / R2) * H + tx * R2 + y % R2;
-                if (n < p.N) {
-                    Vec o;
+        for (int h = 0; h < NP; h++) {
 #pragma unroll
-                    for (int l = 0; l < V; l++) o.v[l] = acc[x][y + l];
-                    *reinterpret_cast<Vec *>(row + n) = o;
+            for (int q = 0; q < QB; q++) {
+                const int e = t + 64 * q;
+                *reinterpret_cast<Vec *>(&Bs[buf][h][e / (NB / V)][(e % (NB / V)) * V]) = rb[h][q];
+            }
+#pragma unroll
+            for (int q = 0; q < QA; q++) {
+                const int e = t + 64 * q;
+                if (ROWS) {
+#pragma unroll
+                    for (int l = 0; l < V; l++)
+                        As[buf][h][(e % (FP_TK / V)) * V + l][e / (FP_TK / V)] = ra[h][q].v[l];
+                } else {
+                    *reinterpret_cast<Vec *>(&As[buf][h][e / (MA / V)][(e % (MA / V)) * V]) = ra[h][q];
                 }
+            }
+        }
+    };
+    T acc[NP][RA][RB];
+#pragma unroll
+    for (int h = 0; h < NP; h++)
+#pragma unroll
+        for (int x = 0; x < RA; x++)
+#pragma unroll
+            for (int y = 0; y < RB; y++) acc[h][x][y] = 0;
+    T shift = 0;
+    if constexpr (ROWS) shift = fp_shift(sc, p.a[0]);
+    load(0);
+    store(0);
+    __syncthreads();
+    int buf = 0;
+    const int K = p.K[0];   // the even part is never the shorter one
+    for (int k0 = 0; k0 < K; k0 += FP_TK) {
+        const bool more = k0 + FP_TK < K;
+        if (more) load(k0 + FP_TK);
+#pragma unroll
+        for (int k = 0; k < FP_TK; k++) {
+#pragma unroll
+            for (int h = 0; h < NP; h++) {
+                T av[RA], bv[RB];
+#pragma unroll
+                for (int gq = 0; gq < GA; gq++)
+#pragma unroll
+                    for (int l = 0; l < RA / GA; l += VR)
+                        *reinterpret_cast<Rd *>(&av[gq * (RA / GA) + l]) =
+                            *reinterpret_cast<const Rd *>(&As[buf][h][k][gq * (MA / 2) + ty * (RA / GA) + l]);
+#pragma unroll
+                for (int gq = 0; gq < GB; gq++)
+#pragma unroll
+                    for (int l = 0; l < RB / GB; l += VR)
+                        *reinterpret_cast<Rd *>(&bv[gq * (RB / GB) + l]) =
+                            *reinterpret_cast<const Rd *>(&Bs[buf][h][k][gq * (NB / 2) + tx * (RB / GB) + l]);
+#pragma unroll
+                for (int x = 0; x < RA; x++)
+#pragma unroll
+                    for (int y = 0; y < RB; y++) acc[h][x][y] += av[x] * bv[y];
+            }
+        }
+        if (more) {
+            store(buf ^ 1);
+            __syncthreads();
+            buf ^= 1;
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < RA; x++) {
+        const int m = m0 + (x / (RA / GA)) * (MA / 2) + ty * (RA / GA) + x % (RA / GA);
+        if (m >= p.M) continue;
+        if constexpr (ROWS) {
+            const int i = (int)fdiv(sc.g.dny, (uint32_t)m), j = m - i * sc.g.ny;
+            T *row = p.c + cidx(sc.g, i, j, 0);
+#pragma unroll
+            for (int y = 0; y < RB; y++) {
+                const int n = n0 + (y / (RB / GB)) * (NB / 2) + tx * (RB / GB) + y % (RB / GB);
+                if (n >= p.N) continue;
+                const T e = acc[0][x][y] + shift, o = FOLD ? acc[NP - 1][x][y] : (T)0;
+                row[n] = e + o;
+                if (FOLD && p.n - 1 - n != n) row[p.n - 1 - n] = e - o;
+            }
+        } else {
+            T *C = p.c + blockIdx.z * p.sc;
+            T *row = C + (long long)m * p.ldc, *mir = C + (long long)(p.n - 1 - m) * p.ldc;
+#pragma unroll
+            for (int y = 0; y < RB; y += VR) {
+                const int n = n0 + (y / (RB / GB)) * (NB / 2) + tx * (RB / GB) + y % (RB / GB);
+                if (n >= p.N) continue;
+                Rd e, o;
+#pragma unroll
+                for (int l = 0; l < VR; l++) {
+                    const T E = acc[0][x][y + l], O = FOLD ? acc[NP - 1][x][y + l] : (T)0;
+                    e.v[l] = E + O;
+                    o.v[l] = E - O;
+                }
+                *reinterpret_cast<Rd *>(row + n) = e;
+                if (FOLD && p.n - 1 - m != m) *reinterpret_cast<Rd *>(mir + n) = o;
             }
         }
     }
@@ -381,16 +593,16 @@ k_fp_diag(const T *__restrict__ iv, const int ny, const int ld, const FpPin<T> p
 template <typename T>
 __global__ void k_fp_pivots(const double *__restrict__ diag, const double *__restrict__ km,
                             const double *__restrict__ kp, const double *__restrict__ l1, const double *__restrict__ l2,
-                            T *iv, const int n, const long long st, const long long outer, const int n1, const int n2,
-                            const int ld, const int z1, const int z2) {
+                            T *iv, const int n, const long long st, const long long outer, const int ld, const int z1,
+                            const int z2) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x, o = blockIdx.y;
     if (c >= ld) return;
     const long long base = o * outer + c;
-    if (c >= n2) {
+    const double lam = l1[o] + l2[c];
+    if (!(lam == lam)) {   // no mode in this column (NaN)
         for (int i = 0; i < n; i++) iv[base + i * st] = 0;
         return;
     }
-    const double lam = l1[o] + l2[c];
     double u = 0;
     for (int i = 0; i < n; i++) {
         double p = diag[i] + lam;
@@ -402,27 +614,35 @@ __global__ void k_fp_pivots(const double *__restrict__ diag, const double *__res
 
 template <typename T>
 __global__ void k_fp_sums(const double *__restrict__ l0, const double *__restrict__ l1, const double *__restrict__ l2,
-                          T *iv, const int ny, const int nz, const int ld, const int z0, const int z1, const int z2) {
+                          T *iv, const int ny, const int ld, const int z0, const int z1, const int z2) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
     if (c >= ld) return;
+    const double lam = l0[i] + l1[j] + l2[c];
     const bool zero = i == z0 && j == z1 && c == z2;
-    iv[((long long)i * ny + j) * ld + c] = c >= nz || zero ? (T)0 : (T)(1.0 / (l0[i] + l1[j] + l2[c]));
+    iv[((long long)i * ny + j) * ld + c] = !(lam == lam) || zero ? (T)0 : (T)(1.0 / lam);
 }
 
 // ------------------------------------------------------- outer rows, body --
 // Outer rows solved for the outer values, each through its chain of
-// partners down to an interior cell (as the multigrid's outer pass), and
-// the identity rows of solid cells.
+// partners down to an interior cell (as the multigrid's outer pass), the
+// identity rows of solid cells, and the swept values of the cells near the
+// body (cell[q] takes val[q]).  The three lists touch different cells; a
+// body whose swept cells are partners of outer rows gets its outer rows in
+// a launch of their own.
 template <typename T, typename S>
 __global__ void __launch_bounds__(256)
 k_fp_edges(const OpT<T> c, const S *__restrict__ r, T *z, const int *__restrict__ outer, const int nout,
-           const int *__restrict__ solid, const int nsolid, const int *gate) {
+           const int *__restrict__ solid, const int nsolid, const int *__restrict__ cell, const T *__restrict__ val,
+           const int ncell, const int *gate) {
     FP_GATE(gate);
-    const int t = blockIdx.x * 256 + threadIdx.x;
+    int t = blockIdx.x * 256 + threadIdx.x;
     if (t >= nout) {
-        if (t - nout < nsolid) {
-            const int P = solid[t - nout];
+        t -= nout;
+        if (t < nsolid) {
+            const int P = solid[t];
             z[P] = fp_value<T, S>(r[P]);
+        } else if (t - nsolid < ncell) {
+            z[cell[t - nsolid]] = val[t - nsolid];
         }
         return;
     }
@@ -457,56 +677,71 @@ k_fp_edges(const OpT<T> c, const S *__restrict__ r, T *z, const int *__restrict_
     z[outer[t]] = v;
 }
 
-// Gauss-Seidel sweeps over the cells near the body (red fluid cells, black
-// ones, then the ghost rows Jacobi-style through tmp), all in one launch of
-// one thread-block cluster whose barrier separates the passes: the lists
-// hold some thousands of cells, so a pass is one latency, and a launch per
-// pass would cost more than the pass.  Values cross the cluster's blocks
-// through L2 (ld/st.cg).
-constexpr int FP_CLUSTER = 8, FP_CT = 1024;
-
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
+// Sweeps over the cells near the body: an overlapping Schwarz step.  The
+// cells (fluid ones within FP_LAYERS of a ghost, and the ghosts) are cut
+// into patches of neighbouring cells; a block takes one patch with
+// FP_OVERLAP more layers of them, loads values and rows into shared memory
+// (couplings to cells outside go into the right-hand side), runs its sweeps
+// there (red, black, then the ghost rows Jacobi-style) and returns the
+// values of its own cells, which k_fp_edges writes to z.  A pass is one
+// block barrier, so the sweeps cost less than loading the patch.  (Sweeps
+// over all the cells at once with a barrier per pass, across the blocks of
+// a cluster or as launches, spend 3-4 us per pass on the L2 round trip.)
+// Bound by latency: one load of the rows, FP_SWEEPS x 4 block barriers.
+constexpr int FP_PT = 256;       // threads of a patch block
+constexpr int FP_PMAX = 1536;    // cells of a patch, overlap included
 
 template <typename T, typename S>
-__global__ void __cluster_dims__(FP_CLUSTER, 1, 1) __launch_bounds__(FP_CT)
-k_fp_near(const OpT<T> c, const S *__restrict__ r, T *z, const int *__restrict__ near, const int nred,
-          const int nblack, const int *__restrict__ gcell, const int ng, const T *__restrict__ gidiv, T *tmp,
-          const int sweeps, const int *gate) {
+__global__ void __launch_bounds__(FP_PT)
+k_fp_patch(const FpPatches<T> p, const S *__restrict__ r, const T *__restrict__ z, T *__restrict__ out,
+           const int sweeps, const int *gate) {
     FP_GATE(gate);
-    const int t0 = blockIdx.x * FP_CT + threadIdx.x;
-    constexpr int NT = FP_CLUSTER * FP_CT;
-    const long long sx = c.g.sx, sy = c.g.sy;
-    for (int s = 0; s < sweeps; s++) {
-        for (int col = 0; col < 2; col++) {
-            const int lo = col ? nred : 0, hi = col ? nred + nblack : nred;
-            for (int q = lo + t0; q < hi; q += NT) {
-                const int P = near[q];
-                int i, j, k;
-                cijk_fast(c.g, c.fdx, c.fdy, P, i, j, k);
-                const T zw = __ldcg(z + P - sx), ze = __ldcg(z + P + sx), zs = __ldcg(z + P - sy),
-                        zn = __ldcg(z + P + sy), zd = __ldcg(z + P - 1), zu = __ldcg(z + P + 1);
-                const T nb = sum6(c.km[0][i + 2], zw, c.kp[0][i + 2], ze, c.km[1][j + 2], zs, c.kp[1][j + 2], zn,
-                                  c.km[2][k + 2], zd, c.kp[2][k + 2], zu);
-                __stcg(z + P, fp_value<T, S>(r[P]) + c.dinv[P] * nb);
-            }
-            cluster_barrier();
-        }
-        for (int g = t0; g < ng; g += NT) {
-            const int P = gcell[g];
-            T sum = 0;
+    __shared__ T v[FP_PMAX], f[FP_PMAX];
+    const int b = blockIdx.x, s0 = p.start[b], nr = p.count[3 * b], nb = p.count[3 * b + 1], ng = p.count[3 * b + 2];
+    const int n = nr + nb + ng;
+    for (int q = threadIdx.x; q < n; q += FP_PT) {
+        const int P = p.P[s0 + q];
+        v[q] = z[P];
+        T t = p.rw[s0 + q] * fp_value<T, S>(r[P]);
 #pragma unroll
-            for (int e = 0; e < 8; e++) {
-                const int q = c.gidx[8 * g + e];
-                if (q >= 0) sum += c.gw[8 * g + e] * __ldcg(z + q);
-            }
-            const T zp = __ldcg(z + P);
-            tmp[g] = zp + (fp_value<T, S>(r[P]) + sum - ((T)1 - c.gwself[g]) * zp) * gidiv[g];
+        for (int e = 0; e < 8; e++) {
+            const int m = p.ref[(size_t)e * p.nloc + s0 + q];
+            if (m < 0) t += p.w[(size_t)e * p.nloc + s0 + q] * z[~m];
         }
-        cluster_barrier();
-        for (int g = t0; g < ng; g += NT) __stcg(z + gcell[g], tmp[g]);   // this thread's own tmp entries
-        cluster_barrier();
+        f[q] = t;
+    }
+    __syncthreads();
+    // Rows of this thread's cells: couplings inside the patch.
+    auto row = [&](int q, int ne) {
+        T t = f[q];
+        for (int e = 0; e < ne; e++) {
+            const int m = p.ref[(size_t)e * p.nloc + s0 + q];
+            if (m >= 0 && m != FP_NONE) t += p.w[(size_t)e * p.nloc + s0 + q] * v[m];
+        }
+        return t;
+    };
+    for (int s = 0; s < sweeps; s++) {
+        for (int q = threadIdx.x; q < nr; q += FP_PT) v[q] = row(q, 6);
+        __syncthreads();
+        for (int q = nr + threadIdx.x; q < nr + nb; q += FP_PT) v[q] = row(q, 6);
+        __syncthreads();
+        T g[(FP_PMAX + FP_PT - 1) / FP_PT];
+#pragma unroll
+        for (int u = 0; u < (FP_PMAX + FP_PT - 1) / FP_PT; u++) {
+            const int q = nr + nb + u * FP_PT + threadIdx.x;
+            if (q < n) g[u] = row(q, 8) + p.self[s0 + q] * v[q];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < (FP_PMAX + FP_PT - 1) / FP_PT; u++) {
+            const int q = nr + nb + u * FP_PT + threadIdx.x;
+            if (q < n) v[q] = g[u];
+        }
+        __syncthreads();
+    }
+    for (int q = threadIdx.x; q < n; q += FP_PT) {
+        const int m = p.slot[s0 + q];
+        if (m >= 0) out[m] = v[q];
     }
 }
 
@@ -622,6 +857,195 @@ FastPoisson<T>::~FastPoisson() {
     for (void *p : allocs_) cudaFree(p);
 }
 
+// The cells near the body, their rows and the patches (k_fp_patch).
+template <typename T>
+template <typename Put>
+bool FastPoisson<T>::build_patches(const OpT<T> &A, const FastPoissonGeom &h, const std::vector<double> &gw, Put put) {
+    const Grid &g = A.g;
+    const int n[3] = {g.nx, g.ny, g.nz};
+    const long long st[3] = {g.sx, g.sy, 1};
+    std::vector<int> id(g.ncell, -1);   // near cell number of a padded index
+    std::vector<int> cells = h.gcell, cur = h.gcell;
+    for (size_t q = 0; q < cells.size(); q++) id[cells[q]] = (int)q;
+    const int ng = nghost_;
+    for (int layer = 0; layer < FP_LAYERS; layer++) {
+        std::vector<int> next;
+        auto add = [&](long long Q) {
+            int i, j, k;
+            cijk(g, Q, i, j, k);
+            if (i < 0 || i >= n[0] || j < 0 || j >= n[1] || k < 0 || k >= n[2] || id[Q] >= 0 || h.flag[Q] != FLUID) return;
+            if (A.p_singular && Q == A.pinned) return;
+            id[Q] = (int)cells.size();
+            cells.push_back((int)Q);
+            next.push_back((int)Q);
+        };
+        if (layer == 0)
+            for (int q : h.gidx)
+                if (q >= 0) add(q);
+        for (int P : cur)
+            for (int a = 0; a < 3; a++) {
+                add(P - st[a]);
+                add(P + st[a]);
+            }
+        cur = next;
+    }
+    const int nc = (int)cells.size();
+    // Rows: couplings (padded index, weight), weight of the old value and of
+    // the residual.  Ghost rows are relaxed as the multigrid relaxes them.
+    std::vector<int> to((size_t)nc * 8, -1);
+    std::vector<double> w((size_t)nc * 8, 0.0), self(nc, 0.0), rw(nc, 1.0);
+    std::vector<int> ijk((size_t)nc * 3);
+    for (int q = 0; q < nc; q++) {
+        int *x = &ijk[3 * (size_t)q];
+        cijk(g, cells[q], x[0], x[1], x[2]);
+        for (int a = 0; a < 3; a++) near_outer_ = near_outer_ || x[a] < 2 || x[a] >= n[a] - 2;
+        if (q < ng) {
+            double off = 0;
+            for (int e = 0; e < 8; e++) {
+                const int P = h.gidx[8 * (size_t)q + e];
+                if (P >= 0 && h.flag[P] == GHOST) off += std::fabs(gw[8 * (size_t)q + e]);
+            }
+            const double dg = 1.0 - h.gwself[q], dv = 1.0 / std::max({dg, 2.0 * off, 1e-3});
+            for (int e = 0; e < 8; e++) {
+                to[8 * (size_t)q + e] = h.gidx[8 * (size_t)q + e];
+                w[8 * (size_t)q + e] = dv * gw[8 * (size_t)q + e];
+            }
+            self[q] = 1.0 - dg * dv;
+            rw[q] = dv;
+        } else {
+            double sum = 0;
+            for (int a = 0; a < 3; a++) sum += h.km[a][x[a]] + h.kp[a][x[a]];
+            for (int a = 0; a < 3; a++) {
+                to[8 * (size_t)q + 2 * a] = (int)(cells[q] - st[a]);
+                to[8 * (size_t)q + 2 * a + 1] = (int)(cells[q] + st[a]);
+                w[8 * (size_t)q + 2 * a] = h.km[a][x[a]] / sum;
+                w[8 * (size_t)q + 2 * a + 1] = h.kp[a][x[a]] / sum;
+            }
+        }
+    }
+    // Patches: cubes of the grid, halved until each fits with its overlap.
+    std::vector<std::vector<int>> todo;
+    {
+        std::vector<std::pair<std::array<int, 3>, int>> key(nc);
+        for (int q = 0; q < nc; q++)
+            key[q] = {{ijk[3 * (size_t)q] / FP_CUBE, ijk[3 * (size_t)q + 1] / FP_CUBE, ijk[3 * (size_t)q + 2] / FP_CUBE}, q};
+        std::sort(key.begin(), key.end());
+        for (int q = 0; q < nc; q++) {
+            if (q == 0 || key[q].first != key[q - 1].first) todo.emplace_back();
+            todo.back().push_back(key[q].second);
+        }
+    }
+    std::vector<int> start, count, P, slot, mark(nc, -1);
+    std::vector<int> loc_cell;
+    std::vector<int> order;   // near cells in output order
+    std::vector<int> pos(nc);
+    int stamp = 0;
+    for (size_t t = 0; t < todo.size(); t++) {
+        std::vector<int> own = todo[t], all = own;
+        stamp++;
+        std::vector<int> front = own;
+        for (int q : own) mark[q] = stamp;
+        for (int o = 0; o < FP_OVERLAP; o++) {
+            std::vector<int> next;
+            auto grow = [&](long long Q) {
+                const int m = Q >= 0 && Q < g.ncell ? id[Q] : -1;
+                if (m < 0 || mark[m] == stamp) return;
+                mark[m] = stamp;
+                next.push_back(m);
+            };
+            for (int q : front) {
+                for (int e = 0; e < 8; e++)
+                    if (to[8 * (size_t)q + e] >= 0) grow(to[8 * (size_t)q + e]);
+                for (int a = 0; a < 3; a++) {
+                    grow(cells[q] - st[a]);
+                    grow(cells[q] + st[a]);
+                }
+            }
+            all.insert(all.end(), next.begin(), next.end());
+            front = next;
+        }
+        if ((int)all.size() > FP_PMAX) {   // split the cube along its longest side
+            if (own.size() < 2) return false;
+            int best = 0, lo = 0, hi = -1;
+            for (int a = 0; a < 3; a++) {
+                int l = ijk[3 * (size_t)own[0] + a], u = l;
+                for (int q : own) {
+                    l = std::min(l, ijk[3 * (size_t)q + a]);
+                    u = std::max(u, ijk[3 * (size_t)q + a]);
+                }
+                if (u - l > hi - lo) {
+                    best = a;
+                    lo = l;
+                    hi = u;
+                }
+            }
+            const int mid = (lo + hi + 1) / 2;
+            std::vector<int> a0, a1;
+            for (int q : own) (ijk[3 * (size_t)q + best] < mid ? a0 : a1).push_back(q);
+            todo.push_back(a0);
+            todo.push_back(a1);
+            continue;
+        }
+        // Local order: red, black, ghost; by padded index within each.
+        auto kind = [&](int q) {
+            return q < ng ? 2 : (ijk[3 * (size_t)q] + ijk[3 * (size_t)q + 1] + ijk[3 * (size_t)q + 2]) & 1;
+        };
+        std::vector<int> list(all);
+        std::sort(list.begin(), list.end(), [&](int x, int y) {
+            const int kx = kind(x), ky = kind(y);
+            return kx != ky ? kx < ky : cells[x] < cells[y];
+        });
+        int c3[3] = {0, 0, 0};
+        start.push_back((int)loc_cell.size());
+        std::vector<int> sorted_own(own);
+        std::sort(sorted_own.begin(), sorted_own.end());
+        for (int q : list) {
+            c3[kind(q)]++;
+            loc_cell.push_back(q);
+            const bool mine = std::binary_search(sorted_own.begin(), sorted_own.end(), q);
+            slot.push_back(mine ? (int)order.size() : -1);
+            if (mine) order.push_back(q);
+            P.push_back(cells[q]);
+        }
+        count.insert(count.end(), c3, c3 + 3);
+    }
+    npatch_ = (int)start.size();
+    nnear_ = nc;
+    const int nloc = (int)loc_cell.size();
+    std::vector<int> ref(8 * (size_t)nloc, FP_NONE);
+    std::vector<T> lw(8 * (size_t)nloc, (T)0), ls(nloc), lr(nloc);
+    for (int b = 0; b < npatch_; b++) {
+        const int s0 = start[b], s1 = b + 1 < npatch_ ? start[b + 1] : nloc;
+        for (int l = s0; l < s1; l++) pos[loc_cell[l]] = l - s0, mark[loc_cell[l]] = ~b;
+        for (int l = s0; l < s1; l++) {
+            const int q = loc_cell[l];
+            ls[l] = (T)self[q];
+            lr[l] = (T)rw[q];
+            for (int e = 0; e < 8; e++) {
+                const int Q = to[8 * (size_t)q + e];
+                if (Q < 0) continue;
+                const int m = id[Q];
+                ref[(size_t)e * nloc + l] = m >= 0 && mark[m] == ~b ? pos[m] : ~Q;
+                lw[(size_t)e * nloc + l] = (T)w[8 * (size_t)q + e];
+            }
+        }
+    }
+    std::vector<int> out_cell(nc);
+    for (int q = 0; q < nc; q++) out_cell[q] = cells[order[q]];
+    patch_.start = (const int *)put(start.data(), sizeof(int) * start.size());
+    patch_.count = (const int *)put(count.data(), sizeof(int) * count.size());
+    patch_.P = (const int *)put(P.data(), sizeof(int) * P.size());
+    patch_.slot = (const int *)put(slot.data(), sizeof(int) * slot.size());
+    patch_.ref = (const int *)put(ref.data(), sizeof(int) * ref.size());
+    patch_.w = (const T *)put(lw.data(), sizeof(T) * lw.size());
+    patch_.self = (const T *)put(ls.data(), sizeof(T) * ls.size());
+    patch_.rw = (const T *)put(lr.data(), sizeof(T) * lr.size());
+    patch_.nloc = nloc;
+    near_cell_ = (const int *)put(out_cell.data(), sizeof(int) * nc);
+    near_val_ = (T *)put(nullptr, sizeof(T) * nc);
+    return near_val_ != nullptr;
+}
+
 template <typename T>
 int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &A, const FastPoissonGeom &h) {
     const Grid &g = A.g;
@@ -636,9 +1060,7 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
     for (int a = 0; a < 3; a++)
         if (n[a] < 3 || (a != tri_ && n[a] > FP_MAX_DENSE)) return 1;
     A_ = A;
-    ld_ = (n[2] + 3) & ~3;
     nghost_ = (int)h.gcell.size();
-    gcell_ = nullptr;
     bool ok = true;
     auto put = [&](const void *src, size_t bytes) -> void * {
         void *p = nullptr;
@@ -652,11 +1074,11 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
         return p;
     };
     std::vector<double> lam[3], diag;
-    std::vector<T> row0[3];
+    std::vector<T> row0[3], v0;
     for (int a = 0; a < 3 && ok; a++) {
         const int N = n[a];
         const std::vector<double> &km = h.km[a], &kp = h.kp[a], &d = h.d[a];
-        std::vector<double> dg(N);
+        std::vector<double> dg(N), e(N, 0.0);
         for (int i = 0; i < N; i++) dg[i] = km[i] + kp[i];
         if (!per[a]) {
             const BCRow<double> &L = A64.bc[lo[a]], &U = A64.bc[hi[a]];
@@ -667,42 +1089,81 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
             diag = dg;
             continue;
         }
-        std::vector<double> w = dg, e(N, 0.0), q;
         for (int i = 0; i + 1 < N; i++) e[i] = -std::sqrt(kp[i] * km[i + 1]);
-        bool good;
-        if (per[a]) {
-            std::vector<double> m((size_t)N * N, 0.0);
-            for (int i = 0; i < N; i++) {
-                m[(size_t)i * N + i] = dg[i];
-                if (i + 1 < N) m[(size_t)i * N + i + 1] = m[(size_t)(i + 1) * N + i] = e[i];
+        const double wrap = per[a] ? -std::sqrt(km[0] * kp[N - 1]) : 0.0;   // couples cells 0 and N - 1
+        // Mirror symmetry, up to the rounding of the face coordinates.
+        auto near_ = [](double x, double y) { return std::fabs(x - y) <= 1e-11 * (std::fabs(x) + std::fabs(y)); };
+        bool sym = true;
+        for (int i = 0; i < N; i++) sym = sym && near_(d[i], d[N - 1 - i]) && near_(dg[i], dg[N - 1 - i]);
+        for (int i = 0; i + 1 < N; i++) sym = sym && near_(e[i], e[N - 2 - i]);
+        FpModes &m = modes_[a];
+        m.fold = sym;
+        m.no = sym ? N / 2 : 0;
+        m.ne = N - m.no;
+        // Columns of the odd modes start on a vector boundary along z.
+        m.off = a == 2 ? (m.ne + 3) & ~3 : m.ne;
+        m.ld = a == 2 ? m.off + ((m.no + 3) & ~3) : N;
+        lam[a].assign(m.ld, __builtin_nan(""));
+        row0[a].assign(m.ld, (T)0);
+        if (a == 2) v0.assign(m.ld, (T)0);
+        double best = INFINITY;
+        for (int odd = 0; odd < (sym ? 2 : 1); odd++) {
+            const int H = odd ? m.no : m.ne;   // size of this parity's problem
+            std::vector<double> w(H), eh(H, 0.0), q;
+            bool good;
+            if (!sym && per[a]) {
+                std::vector<double> f((size_t)N * N, 0.0);
+                for (int i = 0; i < N; i++) {
+                    f[(size_t)i * N + i] = dg[i];
+                    if (i + 1 < N) f[(size_t)i * N + i + 1] = f[(size_t)(i + 1) * N + i] = e[i];
+                }
+                f[N - 1] = f[(size_t)(N - 1) * N] = wrap;
+                good = dense_eigen(N, f, w, q);
+            } else {
+                // On vectors even (odd) about the middle: the first half's
+                // rows, the couplings to the mirrored half folded in.
+                for (int i = 0; i < H; i++) {
+                    w[i] = sym ? (dg[i] + dg[N - 1 - i]) / 2 : dg[i];
+                    if (i + 1 < H) eh[i] = sym ? (e[i] + e[N - 2 - i]) / 2 : e[i];
+                }
+                if (sym) {
+                    const double sg = odd ? -1.0 : 1.0;
+                    w[0] += sg * wrap;
+                    if (N % 2 == 0) w[H - 1] += sg * e[N / 2 - 1];
+                    else if (!odd) eh[H - 2] *= std::sqrt(2.0);
+                }
+                q.assign((size_t)H * H, 0.0);
+                for (int i = 0; i < H; i++) q[(size_t)i * H + i] = 1;
+                good = tridiag_eigen(H, w, eh, q);
             }
-            m[N - 1] = m[(size_t)(N - 1) * N] = -std::sqrt(km[0] * kp[N - 1]);
-            good = dense_eigen(N, m, w, q);
-        } else {
-            q.assign((size_t)N * N, 0.0);
-            for (int i = 0; i < N; i++) q[(size_t)i * N + i] = 1;
-            good = tridiag_eigen(N, w, e, q);
+            if (!good) return 1;
+            const int ld = (H + 3) & ~3, base = odd ? m.off : 0;
+            m.ldm[odd] = ld;
+            std::vector<T> f((size_t)H * ld, (T)0), b((size_t)H * ld, (T)0);
+            for (int k = 0; k < H; k++) {
+                lam[a][base + k] = w[k];
+                if (std::fabs(w[k]) < best) {
+                    best = std::fabs(w[k]);
+                    zero_[a] = base + k;
+                }
+                for (int i = 0; i < H; i++) {
+                    const bool pair = sym && i < N / 2;
+                    const double sd = std::sqrt(sym ? (d[i] + d[N - 1 - i]) / 2 : d[i]);
+                    const double v = q[(size_t)k * H + i] * (pair ? std::sqrt(0.5) : 1.0);
+                    f[(size_t)i * ld + k] = (T)(v * sd);
+                    b[(size_t)k * ld + i] = (T)(v / sd);
+                }
+                row0[a][base + k] = f[k];
+                if (a == 2) v0[base + k] = b[(size_t)k * ld];
+            }
+            fwd_[a][odd] = (T *)put(f.data(), sizeof(T) * f.size());
+            bwd_[a][odd] = (T *)put(b.data(), sizeof(T) * b.size());
         }
-        if (!good) return 1;
-        int z = 0;
-        for (int i = 1; i < N; i++)
-            if (std::fabs(w[i]) < std::fabs(w[z])) z = i;
-        zero_[a] = z;
-        if (A.p_singular) w[z] = 0.0;   // the constants
-        lam[a] = w;
-        const int ld = (N + 3) & ~3;
-        ldm_[a] = ld;
-        std::vector<T> f((size_t)N * ld, (T)0), b((size_t)N * ld, (T)0);
-        for (int m = 0; m < N; m++)
-            for (int i = 0; i < N; i++) {
-                const double sd = std::sqrt(d[i]), v = q[(size_t)m * N + i];
-                f[(size_t)i * ld + m] = (T)(v * sd);
-                b[(size_t)m * ld + i] = (T)(v / sd);
-            }
-        row0[a].assign(f.begin(), f.begin() + ld);
-        fwd_[a] = (T *)put(f.data(), sizeof(T) * f.size());
-        bwd_[a] = (T *)put(b.data(), sizeof(T) * b.size());
+        if (A.p_singular) lam[a][zero_[a]] = 0.0;   // the constants
+        row0_[a] = (T *)put(row0[a].data(), sizeof(T) * row0[a].size());
     }
+    ld_ = modes_[2].ld;
+    v0_ = (T *)put(v0.data(), sizeof(T) * v0.size());
     const size_t cells = (size_t)n[0] * n[1] * ld_;
     for (T *&f : F_) f = (T *)put(nullptr, sizeof(T) * cells);
     inv_ = (T *)put(nullptr, sizeof(T) * cells);
@@ -727,22 +1188,19 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
         const long long st = tri_ == 0 ? (long long)n[1] * ld_ : ld_, outer = tri_ == 0 ? ld_ : (long long)n[1] * ld_;
         const bool sing = A.p_singular != 0;
         k_fp_pivots<T><<<dim3((ld_ + 127) / 128, n[o]), 128, 0, s>>>(dk[0], dk[1], dk[2], dl[o], dl[2], inv_, N, st, outer,
-                                                                      n[o], n[2], ld_, sing ? zero_[o] : -1,
-                                                                      sing ? zero_[2] : -1);
+                                                                      ld_, sing ? zero_[o] : -1, sing ? zero_[2] : -1);
     } else {
         // f0: the x transform's constant-mode value of cell 0, then row 0.
-        std::vector<T> w(1 + ldm_[0]);
+        std::vector<T> w(1 + row0[0].size());
         w[0] = row0[0][zero_[0]];
         std::copy(row0[0].begin(), row0[0].end(), w.begin() + 1);
         dtri_ = (T *)put(w.data(), sizeof(T) * w.size());
         if (!ok) return -1;
         const bool sing = A.p_singular != 0;
-        k_fp_sums<T><<<dim3((ld_ + 127) / 128, n[1], n[0]), 128, 0, s>>>(dl[0], dl[1], dl[2], inv_, n[1], n[2], ld_,
+        k_fp_sums<T><<<dim3((ld_ + 127) / 128, n[1], n[0]), 128, 0, s>>>(dl[0], dl[1], dl[2], inv_, n[1], ld_,
                                                                          sing ? zero_[0] : -1, zero_[1], zero_[2]);
     }
-    // Solid cells, and the cells near the body.
     std::vector<int> solid;
-    const long long st[3] = {g.sx, g.sy, 1};
     for (int i = 0; i < n[0]; i++)
         for (int j = 0; j < n[1]; j++) {
             const long long P0 = cidx(g, i, j, 0);
@@ -752,105 +1210,116 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
     nsolid_ = (int)solid.size();
     solid_ = (int *)put(solid.data(), sizeof(int) * solid.size());
     if (nghost_ > 0) {
-        std::vector<uint8_t> mark(g.ncell, 0);
-        std::vector<int> cur = h.gcell, all;
-        for (int P : cur) mark[P] = 1;
-        auto add = [&](long long Q, std::vector<int> &to) {
-            int i, j, k;
-            cijk(g, Q, i, j, k);
-            if (i < 0 || i >= n[0] || j < 0 || j >= n[1] || k < 0 || k >= n[2] || mark[Q] || h.flag[Q] != FLUID) return;
-            if (A.p_singular && Q == A.pinned) return;
-            mark[Q] = 1;
-            to.push_back((int)Q);
-        };
-        for (int layer = 0; layer < 3; layer++) {
-            std::vector<int> next;
-            if (layer == 0)
-                for (int q : h.gidx)
-                    if (q >= 0) add(q, next);
-            for (int P : cur)
-                for (int a = 0; a < 3; a++) {
-                    add(P - st[a], next);
-                    add(P + st[a], next);
-                }
-            all.insert(all.end(), next.begin(), next.end());
-            cur = next;
-        }
-        std::sort(all.begin(), all.end());
-        std::vector<int> red, black;
-        for (int P : all) {
-            int i, j, k;
-            cijk(g, P, i, j, k);
-            ((i + j + k) & 1 ? black : red).push_back(P);
-            near_outer_ = near_outer_ || i < 2 || i >= n[0] - 2 || j < 2 || j >= n[1] - 2 || k < 2 || k >= n[2] - 2;
-        }
-        nred_ = (int)red.size();
-        nblack_ = (int)black.size();
-        red.insert(red.end(), black.begin(), black.end());
-        near_ = (int *)put(red.data(), sizeof(int) * red.size());
-        gcell_ = (const int *)put(h.gcell.data(), sizeof(int) * nghost_);
-        // Divisors of the ghost rows' relaxation (as the multigrid's) and
-        // the scale of their sources.
         std::vector<double> gw(8 * (size_t)nghost_);
         cudaMemcpyAsync(gw.data(), A64.gw, sizeof(double) * gw.size(), cudaMemcpyDeviceToHost, s);
         if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
-        std::vector<T> sc(nghost_), dv(nghost_);
-        for (int q = 0; q < nghost_; q++) {
-            double off = 0;
-            for (int e = 0; e < 8; e++) {
-                const int P = h.gidx[8 * (size_t)q + e];
-                if (P >= 0 && h.flag[P] == GHOST) off += std::fabs(gw[8 * (size_t)q + e]);
-            }
-            const double dgl = 1.0 - h.gwself[q];
-            sc[q] = (T)(1.0 / std::max(dgl, 1e-3));
-            dv[q] = (T)(1.0 / std::max({dgl, 2.0 * off, 1e-3}));
-        }
+        std::vector<T> sc(nghost_);
+        for (int q = 0; q < nghost_; q++) sc[q] = (T)(1.0 / std::max(1.0 - h.gwself[q], 1e-3));
         gscale_ = (T *)put(sc.data(), sizeof(T) * nghost_);
-        gidiv_ = (T *)put(dv.data(), sizeof(T) * nghost_);
-        gtmp_ = (T *)put(nullptr, sizeof(T) * nghost_);
+        if (!build_patches(A, h, gw, put)) return -1;
     }
     if (!ok) return -1;
     return cudaStreamSynchronize(s) == cudaSuccess ? 0 : -1;
 }
 
 // ------------------------------------------------------------ application --
-// The contiguous axis: rows of `a` times the axis matrix.
+// Forward transform of an axis, from F_[0] to F_[1] or back.
 template <typename T>
-void FastPoisson<T>::gemm_rows(cudaStream_t s, const T *a, int axis, bool forward, T *c, const int *gate) {
-    constexpr int TM = FpTile<T>::TM;
+template <int TM>
+void FastPoisson<T>::forward(cudaStream_t s, int axis, const T *in, T *out, const int *gate) {
     const Grid &g = A_.g;
-    FpGemm<T> p{a, forward ? fwd_[axis] : bwd_[axis], c, g.nx * g.ny, ld_, g.nz, ld_, ldm_[axis], ld_, 0, 0, 0};
-    launch_pdl(k_fp_gemm<T, false, false, T>, dim3((p.N + TM - 1) / TM, (p.M + TM - 1) / TM), 64, 0, s, p,
-               FpScatter<T, T>{}, gate);
+    const FpModes &m = modes_[axis];
+    const int np = m.fold ? 2 : 1, H[2] = {m.ne, m.no};
+    const long long plane = (long long)g.ny * ld_;
+    FpGemm<T> p{};
+    p.nb = np;
+    unsigned gx = 0, gy = 0, batch = 1;
+    for (int h = 0; h < np; h++) {
+        p.K[h] = H[h];
+        if (axis == 2) {   // rows of the data times the axis matrix
+            p.a[h] = in + h * m.off;
+            p.b[h] = fwd_[2][h];
+            p.c[h] = out + h * m.off;
+            p.M[h] = g.nx * g.ny;
+            p.N[h] = p.ldb[h] = m.ldm[h];
+            p.lda[h] = ld_;
+        } else {           // the axis matrix times the lines of the data
+            p.a[h] = fwd_[axis][h];
+            p.b[h] = in;
+            p.c[h] = out + (long long)h * m.off * (axis == 0 ? plane : ld_);
+            p.M[h] = H[h];
+            p.N[h] = p.ldb[h] = axis == 0 ? (int)plane : ld_;
+            p.lda[h] = m.ldm[h];
+        }
+        gx = std::max(gx, (unsigned)((p.N[h] + TM - 1) / TM));
+        gy = std::max(gy, (unsigned)((p.M[h] + TM - 1) / TM));
+    }
+    p.ldc = axis == 0 ? (int)plane : ld_;
+    if (axis == 1) {
+        p.sb = p.sc = plane;
+        batch = g.nx;
+    }
+    p.fold = m.fold && axis != 2 ? (axis == 0 ? g.nx : g.ny) : 0;
+    const dim3 grd(gx, gy, batch * np);
+    if (axis == 2) launch_pdl(k_fp_gemm<T, TM, false>, grd, 64, 0, s, p, gate);
+    else launch_pdl(k_fp_gemm<T, TM, true>, grd, 64, 0, s, p, gate);
 }
 
-// x or y: the axis matrix times the lines of `b`.
+// Backward transform along x or y.
 template <typename T>
-void FastPoisson<T>::gemm_cols(cudaStream_t s, const T *b, int axis, bool forward, T *c, const int *gate) {
-    constexpr int TM = FpTile<T>::TM;
+template <int TM>
+void FastPoisson<T>::backward(cudaStream_t s, int axis, const T *in, T *out, const int *gate) {
     const Grid &g = A_.g;
-    const T *w = forward ? fwd_[axis] : bwd_[axis];
+    const FpModes &m = modes_[axis];
     const long long plane = (long long)g.ny * ld_;
-    FpGemm<T> p;
-    if (axis == 0) p = FpGemm<T>{w, b, c, g.nx, (int)plane, g.nx, ldm_[0], (int)plane, (int)plane, 0, 0, 0};
-    else p = FpGemm<T>{w, b, c, g.ny, ld_, g.ny, ldm_[1], ld_, ld_, 0, plane, plane};
-    launch_pdl(k_fp_gemm<T, true, false, T>, dim3((p.N + TM - 1) / TM, (p.M + TM - 1) / TM, axis == 0 ? 1 : g.nx), 64,
-               0, s, p, FpScatter<T, T>{}, gate);
+    FpBack<T> p{};
+    p.c = out;
+    p.M = m.ne;
+    p.N = p.ldc = axis == 0 ? (int)plane : ld_;
+    for (int h = 0; h < 2; h++) {
+        p.a[h] = bwd_[axis][h];
+        p.b[h] = in + (long long)h * m.off * p.ldc;
+        p.K[h] = h ? m.no : m.ne;
+        p.lda[h] = m.ldm[h];
+        p.ldb[h] = p.ldc;
+    }
+    if (axis == 1) p.sb = p.sc = plane;
+    p.fold = m.fold;
+    p.n = axis == 0 ? g.nx : g.ny;
+    const int MA = m.fold ? TM / 2 : TM;
+    const dim3 grd((p.N + TM - 1) / TM, (p.M + MA - 1) / MA, axis == 1 ? g.nx : 1);
+    if (m.fold) launch_pdl(k_fp_back<T, TM, false, true, T>, grd, 64, 0, s, p, FpScatter<T, T>{}, gate);
+    else launch_pdl(k_fp_back<T, TM, false, false, T>, grd, 64, 0, s, p, FpScatter<T, T>{}, gate);
 }
 
 template <typename T>
 template <typename S>
 void FastPoisson<T>::run(cudaStream_t s, const S *r, T *z, const int *gate) {
-    constexpr int TM = FpTile<T>::TM;
+    // FP64, and FP32 grids with fewer 64 x 64 tiles than SMs (times two:
+    // below that a 32-tile grid's shorter blocks win), take 32 x 32 tiles.
+    if constexpr (sizeof(T) == 8) {
+        run_tiled<32, S>(s, r, z, gate);
+    } else {
+        const Grid &g = A_.g;
+        const long long tiles = (long long)((g.nx * g.ny + 63) / 64) * ((ld_ + 63) / 64);
+        if (tiles < 2 * 152) run_tiled<32, S>(s, r, z, gate);
+        else run_tiled<64, S>(s, r, z, gate);
+    }
+}
+
+template <typename T>
+template <int TM, typename S>
+void FastPoisson<T>::run_tiled(cudaStream_t s, const S *r, T *z, const int *gate) {
     const Grid &g = A_.g;
+    const FpModes &mz = modes_[2];
     int k = 0;
     const int body = nghost_ > 0 || nsolid_ > 0;
-    launch_pdl(k_fp_gather<T, S>, dim3((ld_ + 31) / 32, (g.ny + 7) / 8, (g.nx + FP_GPLANES - 1) / FP_GPLANES),
-               dim3(32, 8), 0, s, A_, r, F_[0], ld_, body, (const T *)gscale_, gate);
+    launch_pdl(k_fp_gather<T, S>, dim3((mz.off + 31) / 32, (g.ny + 7) / 8, (g.nx + FP_GPLANES - 1) / FP_GPLANES),
+               dim3(32, 8), 0, s, A_, r, F_[0], mz, ld_, body, (const T *)gscale_, gate);
     T *x = F_[0], *y = F_[1];
-    auto turn = [&](int axis, bool forward) {
-        if (axis == 2) gemm_rows(s, x, axis, forward, y, gate);
-        else gemm_cols(s, x, axis, forward, y, gate);
+    auto turn = [&](int axis, bool fwd) {
+        if (fwd) forward<TM>(s, axis, x, y, gate);
+        else backward<TM>(s, axis, x, y, gate);
         std::swap(x, y);
         k++;
     };
@@ -859,50 +1328,71 @@ void FastPoisson<T>::run(cudaStream_t s, const S *r, T *z, const int *gate) {
     if (tri_ != 0) turn(0, true);
     FpPin<T> pin{};
     pin.singular = A_.p_singular;
+    pin.f2 = row0_[2];
+    pin.z2 = zero_[2];
     const long long plane = (long long)g.ny * ld_;
     if (tri_ >= 0) {
         const int o = tri_ == 0 ? 1 : 0, n = tri_ == 0 ? g.nx : g.ny;
         const long long st = tri_ == 0 ? plane : ld_, outer = tri_ == 0 ? ld_ : plane;
         pin.w = dtri_;
         pin.zero = zero_[o] * outer + zero_[2];
-        pin.f1 = fwd_[o];
-        pin.f2 = fwd_[2];
+        pin.f1 = row0_[o];
         pin.z1 = zero_[o];
-        pin.z2 = zero_[2];
         launch_pdl(n <= 16 * FP_SEG ? k_fp_tri<T, 512> : k_fp_tri<T, 1024>,
-                   dim3((ld_ + 31) / 32, o == 1 ? g.ny : g.nx), dim3(32, (n + FP_SEG - 1) / FP_SEG), 0, s, (const T *)inv_, A_.km[tri_] + 2, A_.kp[tri_] + 2, n, st, outer, ld_, pin, (const T *)x, y, gate);
+                   dim3((ld_ + 31) / 32, o == 1 ? g.ny : g.nx), dim3(32, (n + FP_SEG - 1) / FP_SEG), 0, s, (const T *)inv_,
+                   A_.km[tri_] + 2, A_.kp[tri_] + 2, n, st, outer, ld_, pin, (const T *)x, y, gate);
     } else {
         pin.w = nullptr;
         pin.zero = zero_[0] * plane + (long long)zero_[1] * ld_ + zero_[2];
-        pin.f1 = fwd_[1];
-        pin.f2 = fwd_[2];
+        pin.f1 = row0_[1];
         pin.z1 = zero_[1];
-        pin.z2 = zero_[2];
         launch_pdl(k_fp_diag<T>, dim3((ld_ + 31) / 32, (g.ny + 7) / 8, g.nx), dim3(32, 8), 0, s, (const T *)inv_,
                    g.ny, ld_, pin, (const T *)dtri_, (const T *)x, y, gate);
     }
     std::swap(x, y);
     if (tri_ != 0) turn(0, false);
     if (tri_ != 1) turn(1, false);
-    FpScatter<T, S> sc{g, g.dny, r, bwd_[2], A_.pinned, A_.p_singular};
-    FpGemm<T> p{x, bwd_[2], z, g.nx * g.ny, ld_, g.nz, ld_, ldm_[2], 0, 0, 0, 0};
-    launch_pdl(k_fp_gemm<T, false, true, S>, dim3((p.N + TM - 1) / TM, (p.M + TM - 1) / TM), 64, 0, s, p, sc, gate);
+    // Along z, into the padded array.
+    FpScatter<T, S> sc{g, r, v0_, A_.pinned, A_.p_singular, ld_};
+    FpBack<T> p{};
+    p.c = z;
+    p.M = g.nx * g.ny;
+    p.N = mz.ne;
+    for (int h = 0; h < 2; h++) {
+        p.a[h] = x + h * mz.off;
+        p.b[h] = bwd_[2][h];
+        p.K[h] = h ? mz.no : mz.ne;
+        p.lda[h] = ld_;
+        p.ldb[h] = mz.ldm[h];
+    }
+    p.fold = mz.fold;
+    p.n = g.nz;
+    const int NB = mz.fold ? TM / 2 : TM;
+    const dim3 grd((p.N + NB - 1) / NB, (p.M + TM - 1) / TM);
+    if (mz.fold) launch_pdl(k_fp_back<T, TM, true, true, S>, grd, 64, 0, s, p, sc, gate);
+    else launch_pdl(k_fp_back<T, TM, true, false, S>, grd, 64, 0, s, p, sc, gate);
     const int nout = A_.sw.nout;
-    auto edges = [&](int solids) {
-        launch_pdl(k_fp_edges<T, S>, (nout + solids + 255) / 256, 256, 0, s, A_, r, z, A_.sw.outer, nout,
-                   (const int *)solid_, solids, gate);
+    auto edges = [&](int outer, int solids, int swept) {
+        launch_pdl(k_fp_edges<T, S>, (outer + solids + swept + 255) / 256, 256, 0, s, A_, r, z, A_.sw.outer, outer,
+                   (const int *)solid_, solids, near_cell_, (const T *)near_val_, swept, gate);
         k++;
     };
-    edges(nsolid_);
     k += 3;
     if (nghost_ > 0) {
-        launch_pdl(k_fp_near<T, S>, FP_CLUSTER, FP_CT, 0, s, A_, r, z, (const int *)near_, nred_, nblack_, gcell_,
-                   nghost_, (const T *)gidiv_, gtmp_, 2, gate);
+        if (near_outer_) edges(nout, nsolid_, 0);   // the sweeps read outer values
+        launch_pdl(k_fp_patch<T, S>, npatch_, FP_PT, 0, s, patch_, r, (const T *)z, near_val_, FP_SWEEPS, gate);
         k++;
-        if (near_outer_) edges(0);
+        if (near_outer_) edges(0, 0, nnear_);
     }
+    if (near_outer_ || nghost_ == 0) edges(nout, nsolid_, 0);
+    else edges(nout, nsolid_, nnear_);
     note_launches(k);
     launches_ = k;
+}
+
+template <typename T>
+void FastPoisson<T>::apply(cudaStream_t s, const T *r, T *z, const int *gate) {
+    run(s, r, z, gate);
 }
 
 template <typename T>

@@ -16,7 +16,7 @@
 // With a body the same solve ignores it (solid rows get no source, a ghost
 // row the source of a fluid row over its diagonal 1 - w_self): the result
 // is exact away from the body, and a few Gauss-Seidel sweeps over the cells
-// within three cells of a ghost repair the rows near it.
+// near it, in overlapping patches, repair the rows there.
 //
 // The pinned row p'(0,0,0) of problems without a pressure boundary value is
 // kept exactly: its fluid row's source is chosen so that the singular
@@ -51,40 +51,81 @@ struct FastPoissonGeom {
 constexpr int FP_MAX_DENSE = 512, FP_MAX_TRI = 512;
 constexpr int FP_SEG = 16;   // rows of the tridiagonal axis per thread
 
+// Modes of a transformed axis.  fold: the axis is mirror-symmetric, its
+// modes split into ne even and no odd ones; otherwise all n are in the
+// first part.  The second part starts at off (along z: a column on a vector
+// boundary, and rows hold ld entries).
+struct FpModes {
+    int fold, ne, no, off, ld;
+    int ldm[2];   // row lengths of the two parts' matrices
+};
+
+// The cells near the body, cut into patches (k_fp_patch).  Pressure
+// iterations per step with 2, 3, 5, 8 and 16 sweeps: sphere 192x128x128 3.7,
+// 3.5, 3.35, 3.35, 3.15; boxes 95x61x47 6.2, 6.0, 5.35, 4.75, 4.4; the
+// twelve-case ensemble 5.75, 5.0, 4.5, 3.9, 3.8, at 1 us of an application
+// per 3 sweeps: 8 is the fastest step everywhere.  Thinner or thicker layers
+// and overlaps are within 3 %.
+constexpr int FP_LAYERS = 3;     // fluid layers around the ghosts
+constexpr int FP_OVERLAP = 3;    // layers a patch takes beyond its own cells
+constexpr int FP_SWEEPS = 8;     // sweeps of a patch
+constexpr int FP_CUBE = 8;       // side of the cubes the cells are cut by
+template <typename T>
+struct FpPatches {
+    const int *start;      // [patch]: its first local cell in the arrays below
+    const int *count;      // [3 patch]: red, black and ghost cells
+    const int *P;          // padded index
+    const int *slot;       // position of the value in `out` (-1: another patch's cell)
+    const int *ref;        // [8][nloc]: local cell of a coupling, ~padded index outside the patch, or FP_NONE
+    const T *w;            // [8][nloc]: weights
+    const T *self;         // weight of the old value (ghost rows; 0 for fluid ones)
+    const T *rw;           // weight of the residual
+    int nloc;
+};
+constexpr int FP_NONE = 0x7fffffff;
+
 template <typename T>
 class FastPoisson : public Preconditioner<T> {
   public:
     ~FastPoisson() override;
     // 0: ready; 1: not for this case (the multigrid serves it); -1: error.
     int setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &A, const FastPoissonGeom &h);
-    void apply(cudaStream_t s, const T *r, T *z, const int *gate) override { run(s, r, z, gate); }
+    void apply(cudaStream_t s, const T *r, T *z, const int *gate) override;
     bool apply_from64(cudaStream_t s, const double *r, T *z, const int *gate) override;
     bool apply_from_df(cudaStream_t s, const dfloat *r, T *z, const int *gate) override;
     int launches() const override { return launches_; }
 
   private:
     OpT<T> A_{};
-    int ld_ = 0;                   // nz rounded up to 4: row length of the compact arrays
+    int ld_ = 0;                   // row length of the compact arrays
     int tri_ = 0;                  // tridiagonal axis: 0, 1, or -1
+    FpModes modes_[3] = {};
     T *F_[2] = {nullptr, nullptr};
-    T *fwd_[3] = {}, *bwd_[3] = {};
-    int ldm_[3] = {0, 0, 0};
+    T *fwd_[3][2] = {}, *bwd_[3][2] = {};   // per parity: (cell, mode) and (mode, cell)
+    T *row0_[3] = {};              // value of cell 0 in every mode
+    T *v0_ = nullptr;              // z: weight of every mode in cell 0
     T *inv_ = nullptr;             // inverse pivots (or eigenvalue sums), compact layout
     T *dtri_ = nullptr;            // widths of the tridiagonal axis
-    int zero_[3] = {0, 0, 0};      // index of each axis's constant mode
+    int zero_[3] = {0, 0, 0};      // each axis's constant mode
     T *gscale_ = nullptr;          // per ghost id: 1 / max(1 - w_self, 1e-3)
-    T *gidiv_ = nullptr, *gtmp_ = nullptr;
-    int *near_ = nullptr;          // red, black and ghost cells near the body
-    int nred_ = 0, nblack_ = 0, nghost_ = 0, nsolid_ = 0;
-    const int *gcell_ = nullptr;
+    FpPatches<T> patch_{};
+    const int *near_cell_ = nullptr;   // cells near the body, and their swept values
+    T *near_val_ = nullptr;
+    int npatch_ = 0, nnear_ = 0, nghost_ = 0, nsolid_ = 0;
     int *solid_ = nullptr;
     bool near_outer_ = false;
     int launches_ = 0;
     std::vector<void *> allocs_;
+    template <typename Put>
+    bool build_patches(const OpT<T> &A, const FastPoissonGeom &h, const std::vector<double> &gw, Put put);
     template <typename S>
     void run(cudaStream_t s, const S *r, T *z, const int *gate);
-    void gemm_rows(cudaStream_t s, const T *a, int axis, bool forward, T *c, const int *gate);
-    void gemm_cols(cudaStream_t s, const T *b, int axis, bool forward, T *c, const int *gate);
+    template <int TM, typename S>
+    void run_tiled(cudaStream_t s, const S *r, T *z, const int *gate);
+    template <int TM>
+    void forward(cudaStream_t s, int axis, const T *in, T *out, const int *gate);
+    template <int TM>
+    void backward(cudaStream_t s, int axis, const T *in, T *out, const int *gate);
 };
 
 }  // namespace ibm
