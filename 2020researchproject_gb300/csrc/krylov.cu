@@ -1427,7 +1427,7 @@ __device__ __forceinline__ double ms_rcp(double d) { return f2d_int(__frcp_rn(d2
 // three, x's planes stay in registers.  FP32: bound by its bytes (36 per
 // cell); FP64: by the FP64 pipe (28 operations per cell).
 template <typename T, int MODE>
-__global__ void __launch_bounds__(SW_THREADS)
+__global__ void __launch_bounds__(SW_THREADS, sizeof(T) == 4 ? 3 : 2)
 k_mom_sweep(const OpT<T> A, const long long n, const T *__restrict__ b, const T *__restrict__ xo, T *__restrict__ xn,
             MScal *ms, KScal *sc, const IRScal *__restrict__ ir, const double tol, const double outer_tol,
             const int limit, const int into_first, double *partials, unsigned int *counter, const LoopCtl lc) {
@@ -1453,22 +1453,53 @@ k_mom_sweep(const OpT<T> A, const long long n, const T *__restrict__ b, const T 
                     xc[l] = xo[l * n + P];
                 }
             }
+            // The loads of a plane; in FP32 the next plane's are in flight
+            // while a plane is computed (sphere 192x128x128: 73 -> 52 us; three
+            // blocks per SM: 10 % faster there than two).
+            struct Plane {
+                T e[3], s[3], n[3], d[3], u[3], b[3];
+                uint8_t fl;
+            };
+            auto fetch = [&](long long Q) {
+                Plane L;
+                L.fl = A.flag[Q];
+#pragma unroll
+                for (int l = 0; l < 3; l++) {
+                    const long long o = l * n + Q;
+                    L.b[l] = b[o];
+                    if (MODE != 1) {
+                        L.e[l] = xo[o + sx];
+                        L.s[l] = xo[o - sy];
+                        L.n[l] = xo[o + sy];
+                        L.d[l] = xo[o - 1];
+                        L.u[l] = xo[o + 1];
+                    }
+                }
+                return L;
+            };
+            constexpr bool AHEAD = sizeof(T) == 4;
+            Plane cur;
+            if (AHEAD) cur = fetch(P);
             for (int i = i0; i < i1; i++, P += sx) {
-                const uint8_t fl = A.flag[P];
+                Plane nxt;
+                if (AHEAD) {
+                    if (i + 1 < i1) nxt = fetch(P + sx);
+                } else {
+                    cur = fetch(P);
+                }
+                const uint8_t fl = cur.fl;
                 const T D = d0 + A.ks[0][i + 2], W = ms_rcp(D);
                 const T kmx = A.km[0][i + 2], kpx = A.kp[0][i + 2];
                 T y[3], r[3];
 #pragma unroll
                 for (int l = 0; l < 3; l++) {
-                    const long long o = l * n + P;
-                    const T bv = b[o];
+                    const T bv = cur.b[l];
                     if (MODE == 1) {
                         r[l] = bv;
                         y[l] = fl == FLUID ? W * bv : bv;
                     } else {
-                        const T xe = xo[o + sx];
-                        const T nb = sum6(kmx, xw[l], kpx, xe, q.kmy, xo[o - sy], q.kpy, xo[o + sy], q.kmz, xo[o - 1],
-                                          q.kpz, xo[o + 1]);
+                        const T nb = sum6(kmx, xw[l], kpx, cur.e[l], q.kmy, cur.s[l], q.kpy, cur.n[l], q.kmz, cur.d[l],
+                                          q.kpz, cur.u[l]);
                         r[l] = bv + (nb - D * xc[l]);
                         y[l] = xc[l] + W * r[l];
                         if (fl != FLUID) {
@@ -1486,7 +1517,7 @@ k_mom_sweep(const OpT<T> A, const long long n, const T *__restrict__ b, const T 
                             r[l] = bv - (((T)1 + A.gwself[g]) * xc[l] + sum);
                         }
                         xw[l] = xc[l];
-                        xc[l] = xe;
+                        xc[l] = cur.e[l];
                         if (MODE == 2) mac(a[3 + l], bv, bv);
                     }
                     mac(a[l], r[l], r[l]);
@@ -1495,6 +1526,7 @@ k_mom_sweep(const OpT<T> A, const long long n, const T *__restrict__ b, const T 
 #pragma unroll
                     for (int l = 0; l < 3; l++) xn[l * n + P] = y[l];
                 }
+                if (AHEAD) cur = nxt;
             }
         }
     } else {

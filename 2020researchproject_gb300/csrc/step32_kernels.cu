@@ -38,7 +38,6 @@ namespace {
 
 constexpr int K32_THREADS = 256;
 constexpr int K32_BLOCKS = 1216;  // 8 per SM on 152 SMs; grid-stride
-// Tiles of the marching kernels: 32 (k) x 8 (j) columns, UN_PLANES planes of i.
 constexpr int UN_TK = 32, UN_TJ = 8, UN_PLANES = 8;
 
 // An FP64 field value in FP32; NaN (solid cells) becomes 0, the value the
@@ -68,140 +67,217 @@ __device__ __forceinline__ float outer_row_u(const OpT<float> &c, int comp, cons
 
 }  // namespace
 
+// Tiles of the marching kernels: 32 (k) x 8 (j) columns over up to UN_PLANES
+// planes of i, fewer on grids that would leave SMs without a block (a
+// 32^3 grid in 8-plane tiles is 16 blocks, each a serial chain of 8 planes:
+// the projection took 46 us, U* 43 us; in 1-plane tiles 11 and 18 us).
+struct Tiles {
+    int tk, tj, planes, nb;
+    explicit Tiles(const Grid &g) {
+        tk = (g.nz + UN_TK - 1) / UN_TK;
+        tj = (g.ny + UN_TJ - 1) / UN_TJ;
+        planes = UN_PLANES;
+        auto blocks = [&]() { return (long long)tk * tj * ((g.nx + planes - 1) / planes); };
+        while (planes > 1 && blocks() < 2 * 152) planes /= 2;
+        nb = (int)blocks();
+    }
+};
+
 // ------------------------------------------------------------------------
 // calc_N + momentum right-hand side (src/ibm3d_fracstep.c:117-170,
 // 237-352) in FP32, written as the increment system's right-hand side c
 // (3 components, w.b32 layout l*n + P) and N (FP32).  The last block
 // stores ||b||^2 and ||c||^2 per component in the increment solve's
 // scalars (out[l].bnorm2, .rnorm2).
+//
+// Blocks [0, nb) take tiles of interior columns and march over planes of i;
+// the others take the outer rows.  Each FP64 value of u and p is loaded and
+// converted once per tile: a plane's values sit in shared memory with a halo
+// of one cell (y and z neighbours), the planes before and after in
+// registers, and the next plane's loads are in flight while a plane is
+// computed.  (One thread per padded cell loading its neighbours converted
+// 25 values per cell behind two load latencies: sphere 192x128x128 232 ->
+// 148 us, against 47 us of HBM time.)
 // ------------------------------------------------------------------------
 __global__ void __launch_bounds__(K32_THREADS)
 k_conv_rhs32(const Grid g, const AxisF ax, const AxisF ay, const AxisF az, const OpT<float> A, const BCSet bc,
              const uint8_t *__restrict__ flag, const Conv32Args a, const float dt, const float f1, const float f2,
-             const float f3, const int les, double *partials, unsigned int *counter, IRScal *out) {
+             const float f3, const int les, const Tiles tl, const int *__restrict__ outer, const int nout,
+             double *partials, unsigned int *counter, IRScal *out) {
     __shared__ double smem[32 * 6];
+    __shared__ float sp[2][4][UN_TJ + 2][UN_TK + 2];   // u1, u2, u3, p of a plane, with halo
     float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // ||b||^2 (3), ||c||^2 (3)
     const long long n = g.ncell;
     const float NaNf = __int_as_float(0x7fc00000);
-    const int lane = threadIdx.x & 31;
-    // Block-uniform loop: the lanes of a warp hold consecutive padded cells,
-    // so the k neighbours (P -/+ 1) of the values every lane converts for
-    // its own cell come by shuffle; lanes 0 and 31 load theirs.
-    for (long long base = blockIdx.x * (long long)blockDim.x; base < n; base += (long long)gridDim.x * blockDim.x) {
-        const long long P = base + threadIdx.x;
-        const bool act = P < n;
-        float own[5] = {0.f, 0.f, 0.f, 0.f, 0.f};   // u1, u2, u3, p, W (low z face)
-        if (act) {
-            own[0] = ld32(a.u[0], P);
-            own[1] = ld32(a.u[1], P);
-            own[2] = ld32(a.u[2], P);
-            own[3] = ldp32(a.p, P);
-            own[4] = ldp32(a.U[2], P);
-        }
-        float dn[4], up[5];
-#pragma unroll
-        for (int q = 0; q < 4; q++) dn[q] = __shfl_up_sync(0xffffffffu, own[q], 1);
-#pragma unroll
-        for (int q = 0; q < 5; q++) up[q] = __shfl_down_sync(0xffffffffu, own[q], 1);
-        if (!act) continue;
-        int i, j, k;
-        cijk_g(g, P, i, j, k);
-        int layer;
-        const int f = owner_face(g, i, j, k, layer);
-        float bv[3], cv[3];
-        if (f >= 0) {
+    if ((int)blockIdx.x >= tl.nb) {
+        const int t = (blockIdx.x - tl.nb) * K32_THREADS + threadIdx.x;
+        if (t < nout) {
             // Outer rows: the velocity BC value (VELOCITY faces) or 0.
+            const long long P = outer[t];
+            int i, j, k;
+            cijk_g(g, P, i, j, k);
+            int layer;
+            const int f = owner_face(g, i, j, k, layer);
             const BCFace &F = bc.f[f];
             const bool vel = F.type == BCT_VELOCITY;
             const double *sv = F.scur ? F.scur + face_line(g, f, i, j, k) : nullptr;
 #pragma unroll
             for (int l = 0; l < 3; l++) {
-                bv[l] = vel ? d2f_int(sv ? sv[l * F.nt] : F.val[l]) : 0.0f;
-                cv[l] = bv[l] - outer_row_u(A, l, a.u[l], P, i, j, k, f, layer);
-            }
-        } else if (flag[P] != FLUID) {
-            // Ghost rows (1 + w_self) x_g + sum w x = 0, solid rows x = 0.
-#pragma unroll
-            for (int l = 0; l < 3; l++) {
-                a.N[l][P] = NaNf;
-                bv[l] = 0.0f;
-                cv[l] = 0.0f;
-            }
-            if (flag[P] == GHOST) {
-                const int q = A.gid[P];
-                const float ws = A.gwself[q];
-#pragma unroll
-                for (int l = 0; l < 3; l++) {
-                    float sum = 0.0f;
-#pragma unroll
-                    for (int e = 0; e < 8; e++) {
-                        const int m = A.gidx[8 * q + e];
-                        if (m >= 0) sum += A.gw[8 * q + e] * ld32(a.u[l], m);
-                    }
-                    cv[l] = -((1.0f + ws) * ld32(a.u[l], P) + sum);
-                }
-            }
-        } else {
-            const long long sx = g.sx, sy = g.sy;
-            const int I = i + 2, J = j + 2, K = k + 2;
-            // A fluid cell is interior, so P -/+ 1 are cells of the grid:
-            // the warp's edge lanes load them here.
-            if (lane == 0) {
-                for (int q = 0; q < 3; q++) dn[q] = ld32(a.u[q], P - 1);
-                dn[3] = ldp32(a.p, P - 1);
-            }
-            if (lane == 31) {
-                for (int q = 0; q < 3; q++) up[q] = ld32(a.u[q], P + 1);
-                up[3] = ldp32(a.p, P + 1);
-                up[4] = ldp32(a.U[2], P + 1);
-            }
-            const float wmx0 = ax.wm[I], wpx0 = ax.wp[I], wmx1 = ax.wm[I + 1], wpx1 = ax.wp[I + 1];
-            const float wmy0 = ay.wm[J], wpy0 = ay.wp[J], wmy1 = ay.wm[J + 1], wpy1 = ay.wp[J + 1];
-            const float wmz0 = az.wm[K], wpz0 = az.wp[K], wmz1 = az.wm[K + 1], wpz1 = az.wp[K + 1];
-            const float Uw = ldp32(a.U[0], P), Ue = ldp32(a.U[0], P + sx);
-            const float Vs = ldp32(a.U[1], P), Vn = ldp32(a.U[1], P + sy);
-            const float Wd = own[4], Wu = up[4];
-            const float rdx = ax.rd[I], rdy = ay.rd[J], rdz = az.rd[K];
-            const float kW = ax.km[I], kE = ax.kp[I], kS = ay.km[J], kN = ay.kp[J], kD = az.km[K], kU = az.kp[K];
-            const float gx = ax.rdcc[I], gy = ay.rdcc[J], gz = az.rdcc[K];
-            const float ff[3] = {f1, f2, f3};
-#pragma unroll
-            for (int l = 0; l < 3; l++) {
-                const double *u = a.u[l];
-                const float uc = own[l];
-                const float uW = ld32(u, P - sx), uE = ld32(u, P + sx), uS = ld32(u, P - sy), uN = ld32(u, P + sy);
-                const float uD = dn[l], uU = up[l];
-                const float fw = uW * wmx0 + uc * wpx0, fe = uc * wmx1 + uE * wpx1;
-                const float fs = uS * wmy0 + uc * wpy0, fn = uc * wmy1 + uN * wpy1;
-                const float fd = uD * wmz0 + uc * wpz0, fu = uc * wmz1 + uU * wpz1;
-                const float Nl = (Ue * fe - Uw * fw) * rdx + (Vn * fn - Vs * fs) * rdy + (Wu * fu - Wd * fd) * rdz;
-                a.N[l][P] = Nl;
-                float dp;
-                if (l == 0) dp = (ldp32(a.p, P + sx) - ldp32(a.p, P - sx)) * gx;
-                else if (l == 1) dp = (ldp32(a.p, P + sy) - ldp32(a.p, P - sy)) * gy;
-                else dp = (up[3] - dn[3]) * gz;
-                float divtau = 0.0f;
-                if (les) {
-                    const int t1 = l == 0 ? 0 : l == 1 ? 1 : 2;
-                    const int t2 = l == 0 ? 1 : l == 1 ? 3 : 4;
-                    const int t3 = l == 0 ? 2 : l == 1 ? 4 : 5;
-                    divtau = (ldp32(a.tau[t1], P + sx) - ldp32(a.tau[t1], P - sx)) * gx +
-                             (ldp32(a.tau[t2], P + sy) - ldp32(a.tau[t2], P - sy)) * gy +
-                             (ldp32(a.tau[t3], P + 1) - ldp32(a.tau[t3], P - 1)) * gz;
-                }
-                const float fl = a.force ? ldp32(a.force, l * n + P) : ff[l];
-                const float lap = kW * (uW - uc) + kE * (uE - uc) + kS * (uS - uc) + kN * (uN - uc) +
-                                  kD * (uD - uc) + kU * (uU - uc);
-                const float rest = -dt / 2 * (3 * Nl - a.Np[l][P]) - dt * dp + dt * fl - dt * divtau;
-                bv[l] = uc + lap + rest;
-                cv[l] = 2 * lap + rest;
+                const float bv = vel ? d2f_int(sv ? sv[l * F.nt] : F.val[l]) : 0.0f;
+                const float cv = bv - outer_row_u(A, l, a.u[l], P, i, j, k, f, layer);
+                a.c[l * n + P] = cv;
+                acc[l] += bv * bv;
+                acc[3 + l] += cv * cv;
             }
         }
+    } else {
+        int b = blockIdx.x;
+        const int bk = b % tl.tk;
+        b /= tl.tk;
+        const int bj = b % tl.tj, bi = b / tl.tj;
+        const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
+        const int k = bk * UN_TK + tx, j = bj * UN_TJ + ty;
+        const int i0 = bi * tl.planes, i1 = min(i0 + tl.planes, g.nx);
+        const bool live = j < g.ny && k < g.nz;
+        const long long sx = g.sx, sy = g.sy;
+        // This thread's column (clamped into the padded box) and its halo
+        // cell: 2 x 32 cells above and below, 2 x 8 left and right.
+        const int jc = min(j, g.ny + 1), kc = min(k, g.nz + 1);
+        const bool halo = t < 2 * UN_TK + 2 * UN_TJ;
+        const int hy = t < UN_TK ? 0 : t < 2 * UN_TK ? UN_TJ + 1 : 1 + (t - 2 * UN_TK) % UN_TJ;
+        const int hx = t < 2 * UN_TK ? 1 + (t & 31) : t < 2 * UN_TK + UN_TJ ? 0 : UN_TK + 1;
+        const int hj = min(bj * UN_TJ + hy - 1, g.ny + 1), hk = min(bk * UN_TK + hx - 1, g.nz + 1);
+        long long P = cidx(g, i0, jc, kc), H = cidx(g, i0, hj, hk);
+        const double *fld[4] = {a.u[0], a.u[1], a.u[2], a.p};
+        const int J = jc + 2, K = kc + 2;
+        const float wmy0 = ay.wm[J], wpy0 = ay.wp[J], wmy1 = ay.wm[min(J + 1, g.ny + 3)], wpy1 = ay.wp[min(J + 1, g.ny + 3)];
+        const float wmz0 = az.wm[K], wpz0 = az.wp[K], wmz1 = az.wm[min(K + 1, g.nz + 3)], wpz1 = az.wp[min(K + 1, g.nz + 3)];
+        const float rdy = ay.rd[J], rdz = az.rd[K], gy = ay.rdcc[J], gz = az.rdcc[K];
+        const float kS = ay.km[J], kN = ay.kp[J], kD = az.km[K], kU = az.kp[K];
+        const float ff[3] = {f1, f2, f3};
+        float vw[4], vc[4];
+        double nx[4], nh[4], Uen;   // the next plane: own, halo, high x face
 #pragma unroll
-        for (int l = 0; l < 3; l++) {
-            a.c[l * n + P] = cv[l];
-            acc[l] += bv[l] * bv[l];
-            acc[3 + l] += cv[l] * cv[l];
+        for (int q = 0; q < 4; q++) {
+            vw[q] = d2f_int(fld[q][P - sx]);
+            vc[q] = d2f_int(fld[q][P]);
+            const float hv = halo ? d2f_int(fld[q][H]) : 0.0f;
+            if (q < 3) {
+                vw[q] = vw[q] == vw[q] ? vw[q] : 0.0f;
+                vc[q] = vc[q] == vc[q] ? vc[q] : 0.0f;
+            }
+            sp[0][q][ty + 1][tx + 1] = vc[q];
+            if (halo) sp[0][q][hy][hx] = q < 3 && hv != hv ? 0.0f : hv;
+        }
+        float Uw = ldp32(a.U[0], P);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            nx[q] = fld[q][P + sx];
+            nh[q] = halo ? fld[q][H + sx] : 0.0;
+        }
+        Uen = a.U[0][P + sx];
+        int buf = 0;
+        for (int i = i0; i < i1; i++, P += sx, H += sx) {
+            const int I = i + 2;
+            // Everything else this plane needs, and then the next plane's
+            // loads, before the arithmetic.
+            const uint8_t fl = flag[P];
+            const double Vs64 = a.U[1][P], Vn64 = a.U[1][P + (live ? sy : 0)], Wd64 = a.U[2][P],
+                         Wu64 = a.U[2][P + (live ? 1 : 0)];
+            float np[3];
+#pragma unroll
+            for (int l = 0; l < 3; l++) np[l] = a.Np[l][P];
+            float ve[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                ve[q] = d2f_int(nx[q]);
+                if (q < 3) ve[q] = ve[q] == ve[q] ? ve[q] : 0.0f;
+                sp[buf ^ 1][q][ty + 1][tx + 1] = ve[q];
+                if (halo) {
+                    const float hv = d2f_int(nh[q]);
+                    sp[buf ^ 1][q][hy][hx] = q < 3 && hv != hv ? 0.0f : hv;
+                }
+            }
+            const float Ue = d2f_int(Uen);
+            if (i + 1 < i1) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    nx[q] = fld[q][P + 2 * sx];
+                    if (halo) nh[q] = fld[q][H + 2 * sx];
+                }
+                Uen = a.U[0][P + 2 * sx];
+            }
+            __syncthreads();   // plane i complete (its stores precede the last barrier), i + 1 being written
+            if (live) {
+                float bv[3], cv[3];
+                if (fl != FLUID) {
+                    // Ghost rows (1 + w_self) x_g + sum w x = 0, solid rows x = 0.
+                    const int q = fl == GHOST ? A.gid[P] : 0;
+#pragma unroll
+                    for (int l = 0; l < 3; l++) {
+                        a.N[l][P] = NaNf;
+                        bv[l] = 0.0f;
+                        cv[l] = 0.0f;
+                        if (fl == GHOST) {
+                            float sum = 0.0f;
+#pragma unroll
+                            for (int e = 0; e < 8; e++) {
+                                const int m = A.gidx[8 * q + e];
+                                if (m >= 0) sum += A.gw[8 * q + e] * ld32(a.u[l], m);
+                            }
+                            cv[l] = -((1.0f + A.gwself[q]) * vc[l] + sum);
+                        }
+                    }
+                } else {
+                    const float wmx0 = ax.wm[I], wpx0 = ax.wp[I], wmx1 = ax.wm[I + 1], wpx1 = ax.wp[I + 1];
+                    const float rdx = ax.rd[I], kW = ax.km[I], kE = ax.kp[I], gx = ax.rdcc[I];
+                    const float Vs = d2f_int(Vs64), Vn = d2f_int(Vn64), Wd = d2f_int(Wd64), Wu = d2f_int(Wu64);
+#pragma unroll
+                    for (int l = 0; l < 3; l++) {
+                        const float uc = vc[l], uW = vw[l], uE = ve[l];
+                        const float uS = sp[buf][l][ty][tx + 1], uN = sp[buf][l][ty + 2][tx + 1];
+                        const float uD = sp[buf][l][ty + 1][tx], uU = sp[buf][l][ty + 1][tx + 2];
+                        const float fw = uW * wmx0 + uc * wpx0, fe = uc * wmx1 + uE * wpx1;
+                        const float fs = uS * wmy0 + uc * wpy0, fn = uc * wmy1 + uN * wpy1;
+                        const float fd = uD * wmz0 + uc * wpz0, fu = uc * wmz1 + uU * wpz1;
+                        const float Nl = (Ue * fe - Uw * fw) * rdx + (Vn * fn - Vs * fs) * rdy + (Wu * fu - Wd * fd) * rdz;
+                        a.N[l][P] = Nl;
+                        float dp;
+                        if (l == 0) dp = (ve[3] - vw[3]) * gx;
+                        else if (l == 1) dp = (sp[buf][3][ty + 2][tx + 1] - sp[buf][3][ty][tx + 1]) * gy;
+                        else dp = (sp[buf][3][ty + 1][tx + 2] - sp[buf][3][ty + 1][tx]) * gz;
+                        float divtau = 0.0f;
+                        if (les) {
+                            const int t1 = l == 0 ? 0 : l == 1 ? 1 : 2;
+                            const int t2 = l == 0 ? 1 : l == 1 ? 3 : 4;
+                            const int t3 = l == 0 ? 2 : l == 1 ? 4 : 5;
+                            divtau = (ldp32(a.tau[t1], P + sx) - ldp32(a.tau[t1], P - sx)) * gx +
+                                     (ldp32(a.tau[t2], P + sy) - ldp32(a.tau[t2], P - sy)) * gy +
+                                     (ldp32(a.tau[t3], P + 1) - ldp32(a.tau[t3], P - 1)) * gz;
+                        }
+                        const float fl_ = a.force ? ldp32(a.force, l * n + P) : ff[l];
+                        const float lap = kW * (uW - uc) + kE * (uE - uc) + kS * (uS - uc) + kN * (uN - uc) +
+                                          kD * (uD - uc) + kU * (uU - uc);
+                        const float rest = -dt / 2 * (3 * Nl - np[l]) - dt * dp + dt * fl_ - dt * divtau;
+                        bv[l] = uc + lap + rest;
+                        cv[l] = 2 * lap + rest;
+                    }
+                }
+#pragma unroll
+                for (int l = 0; l < 3; l++) {
+                    a.c[l * n + P] = cv[l];
+                    acc[l] += bv[l] * bv[l];
+                    acc[3 + l] += cv[l] * cv[l];
+                }
+            }
+            __syncthreads();   // plane i is read before i + 2 overwrites it
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                vw[q] = vc[q];
+                vc[q] = ve[q];
+            }
+            Uw = Ue;
+            buf ^= 1;
         }
     }
     double tot[6];
@@ -228,8 +304,11 @@ k_conv_rhs32(const Grid g, const AxisF ax, const AxisF ay, const AxisF az, const
 void launch_conv_rhs32(cudaStream_t s, const Grid &g, const AxisF axf[3], const OpT<float> &A, const BCSet &bc,
                        const uint8_t *flag, const Conv32Args &a, double dt, const double f[3], int les,
                        double *partials, unsigned int *counter, IRScal *out) {
-    k_conv_rhs32<<<K32_BLOCKS, K32_THREADS, 0, s>>>(g, axf[0], axf[1], axf[2], A, bc, flag, a, (float)dt, (float)f[0],
-                                                    (float)f[1], (float)f[2], les, partials, counter, out);
+    const int no = A.sw.nout, ob = (no + K32_THREADS - 1) / K32_THREADS;
+    const Tiles t(g);
+    k_conv_rhs32<<<t.nb + ob, K32_THREADS, 0, s>>>(g, axf[0], axf[1], axf[2], A, bc, flag, a, (float)dt, (float)f[0],
+                                                   (float)f[1], (float)f[2], les, t, A.sw.outer, no, partials,
+                                                   counter, out);
     note_launches(1);
 }
 
@@ -246,85 +325,118 @@ void launch_conv_rhs32(cudaStream_t s, const Grid &g, const AxisF axf[3], const 
 // ------------------------------------------------------------------------
 namespace {
 
+__device__ __forceinline__ float ustar_of(double u, float e) {
+    const float v = d2f_int(u);
+    return __fadd_rn(v == v ? v : 0.0f, e);
+}
 __device__ __forceinline__ float ustar_at(const double *__restrict__ u, const float *__restrict__ e, long long P) {
-    return __fadd_rn(ld32(u, P), e[P]);
+    return ustar_of(u[P], e[P]);
 }
 
 __device__ __forceinline__ bool fg_pair32(uint8_t a, uint8_t b) {
     return (a == FLUID && b == GHOST) || (a == GHOST && b == FLUID);
 }
 
-// U* on the face between Pm (index ii-1) and Pp (index ii) from u~ (ut)
-// or, across a fluid-ghost pair, from u*.
-__device__ __forceinline__ float face32t(const double *__restrict__ u, const float *__restrict__ e,
-                                         const float *__restrict__ ut, const double *__restrict__ p, const AxisF &a,
-                                         int ii, long long Pm, long long Pp, bool fluid_ghost, float dt) {
-    const float wm = a.wm[ii + 2], wp = a.wp[ii + 2];
-    if (fluid_ghost) return __fadd_rn(__fmul_rn(ustar_at(u, e, Pm), wm), __fmul_rn(ustar_at(u, e, Pp), wp));
-    const float gf = __fmul_rn(__fsub_rn(ldp32(p, Pp), ldp32(p, Pm)), a.rdc[ii + 2]);
-    return __fsub_rn(__fadd_rn(__fmul_rn(ut[Pm], wm), __fmul_rn(ut[Pp], wp)), __fmul_rn(dt, gf));
+// U* on a face between the cells m and p of an axis (weights wm, wp; rdc
+// the reciprocal of their distance): from u~ (utm, utp) and the pressure
+// difference, or, across a fluid-ghost pair, from u*.
+__device__ __forceinline__ float face32t(float wm, float wp, float rdc, float utm, float utp, float pm, float pp, float dt) {
+    const float gf = __fmul_rn(__fsub_rn(pp, pm), rdc);
+    return __fsub_rn(__fadd_rn(__fmul_rn(utm, wm), __fmul_rn(utp, wp)), __fmul_rn(dt, gf));
+}
+__device__ __forceinline__ float face32g(const double *__restrict__ u, const float *__restrict__ e, long long Pm,
+                                         long long Pp, float wm, float wp) {
+    return __fadd_rn(__fmul_rn(ustar_at(u, e, Pm), wm), __fmul_rn(ustar_at(u, e, Pp), wp));
 }
 
 }  // namespace
 
+// Grid (ceil((nz + 2) / 32), ceil((ny + 2) / 8), nx + 2) of 32 x 8 threads,
+// no index division.
 __global__ void __launch_bounds__(256)
 k_utilde32(const Grid g, const AxisF ax, const AxisF ay, const AxisF az, const Ustar32Args a, float *__restrict__ ut,
            const float dt) {
-    const long long nx2 = g.nx + 2, ny2 = g.ny + 2, nz2 = g.nz + 2, n = nx2 * ny2 * nz2;
-    const long long sx = g.sx, sy = g.sy;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-         q += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(q % nz2) - 1;
-        const long long r = q / nz2;
-        const int j = (int)(r % ny2) - 1, i = (int)(r / ny2) - 1;
-        const long long P = cidx(g, i, j, k);
-        const float gx = (ldp32(a.p, P + sx) - ldp32(a.p, P - sx)) * ax.rdcc[i + 2];
-        const float gy = (ldp32(a.p, P + sy) - ldp32(a.p, P - sy)) * ay.rdcc[j + 2];
-        const float gz = (ldp32(a.p, P + 1) - ldp32(a.p, P - 1)) * az.rdcc[k + 2];
-        ut[P] = ustar_at(a.u[0], a.e[0], P) + dt * gx;
-        ut[g.ncell + P] = ustar_at(a.u[1], a.e[1], P) + dt * gy;
-        ut[2 * g.ncell + P] = ustar_at(a.u[2], a.e[2], P) + dt * gz;
-    }
+    const int k = blockIdx.x * 32 + threadIdx.x - 1, j = blockIdx.y * 8 + threadIdx.y - 1, i = (int)blockIdx.z - 1;
+    if (k > g.nz || j > g.ny) return;
+    const long long sx = g.sx, sy = g.sy, P = cidx(g, i, j, k);
+    const double pe = a.p[P + sx], pw = a.p[P - sx], pn = a.p[P + sy], ps = a.p[P - sy], pu = a.p[P + 1], pd = a.p[P - 1];
+    const double u0 = a.u[0][P], u1 = a.u[1][P], u2 = a.u[2][P];
+    const float e0 = a.e[0][P], e1 = a.e[1][P], e2 = a.e[2][P];
+    const float gx = (d2f_int(pe) - d2f_int(pw)) * ax.rdcc[i + 2];
+    const float gy = (d2f_int(pn) - d2f_int(ps)) * ay.rdcc[j + 2];
+    const float gz = (d2f_int(pu) - d2f_int(pd)) * az.rdcc[k + 2];
+    ut[P] = ustar_of(u0, e0) + dt * gx;
+    ut[g.ncell + P] = ustar_of(u1, e1) + dt * gy;
+    ut[2 * g.ncell + P] = ustar_of(u2, e2) + dt * gz;
 }
 
-__global__ void __launch_bounds__(UN_TK * UN_TJ)
+__global__ void __launch_bounds__(UN_TK * UN_TJ, 3)
 k_ustar_faces32(const Grid g, const AxisF ax, const AxisF ay, const AxisF az, const Axis ax64, const Axis ay64,
                 const Axis az64, const BCSet bc, const uint8_t *__restrict__ flag, const Ustar32Args a,
-                const float *__restrict__ ut, const float dt, const double m2re, const int tk, const int tj,
-                const int planes) {
+                const float *__restrict__ ut, const float dt, const double m2re, const Tiles tl) {
     __shared__ float sVs[2][UN_TJ][UN_TK];
     int b = blockIdx.x;
-    const int bk = b % tk;
-    b /= tk;
-    const int bj = b % tj, bi = b / tj;
+    const int bk = b % tl.tk;
+    b /= tl.tk;
+    const int bj = b % tl.tj, bi = b / tl.tj;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int k = bk * UN_TK + tx, j = bj * UN_TJ + ty;
-    const int i0 = bi * planes, i1 = min(i0 + planes, g.nx);
+    const int i0 = bi * tl.planes, i1 = min(i0 + tl.planes, g.nx);
     const bool live = j < g.ny && k < g.nz;
     const bool own_vn = ty == UN_TJ - 1 || j == g.ny - 1;
     const bool own_wu = tx == UN_TK - 1 || k == g.nz - 1;
     const long long sx = g.sx, sy = g.sy, n = g.ncell;
     const float *ut0 = ut, *ut1 = ut + n, *ut2 = ut + 2 * n;
-    long long P = live ? cidx(g, i0, j, k) : 0;
-    uint8_t fc = live ? flag[P] : (uint8_t)SOLID;
-    float Uw = 0.0f;
-    if (live) Uw = face32t(a.u[0], a.e[0], ut0, a.p, ax, i0, P - sx, P, fg_pair32(flag[P - sx], fc), dt);
+    // Threads off the grid follow a column inside it and store nothing.
+    const int jc = min(j, g.ny - 1), kc = min(k, g.nz - 1), J = jc + 2, K = kc + 2;
+    const float wms = ay.wm[J], wps = ay.wp[J], rds = ay.rdc[J], wmn = ay.wm[J + 1], wpn = ay.wp[J + 1], rdn = ay.rdc[J + 1];
+    const float wmd = az.wm[K], wpd = az.wp[K], rdd = az.rdc[K], wmu = az.wm[K + 1], wpu = az.wp[K + 1], rdu = az.rdc[K + 1];
+    long long P = cidx(g, i0, jc, kc);
+    uint8_t fc = flag[P];
+    float pc = d2f_int(a.p[P]), u0c = ut0[P];
+    float Uw;
+    {
+        const int I = i0 + 2;
+        Uw = fg_pair32(flag[P - sx], fc) ? face32g(a.u[0], a.e[0], P - sx, P, ax.wm[I], ax.wp[I])
+                                         : face32t(ax.wm[I], ax.wp[I], ax.rdc[I], ut0[P - sx], u0c, d2f_int(a.p[P - sx]), pc, dt);
+    }
     int buf = 0;
     for (int i = i0; i < i1; i++, P += sx) {
-        float Ue = 0.f, Vs = 0.f, Wd = 0.f, Vn = 0.f, Wu = 0.f;
-        uint8_t fe = SOLID;
-        if (live) {
-            fe = flag[P + sx];
-            Ue = face32t(a.u[0], a.e[0], ut0, a.p, ax, i + 1, P, P + sx, fg_pair32(fc, fe), dt);
-            Vs = face32t(a.u[1], a.e[1], ut1, a.p, ay, j, P - sy, P, fg_pair32(flag[P - sy], fc), dt);
-            Wd = face32t(a.u[2], a.e[2], ut2, a.p, az, k, P - 1, P, fg_pair32(flag[P - 1], fc), dt);
-            if (own_vn) Vn = face32t(a.u[1], a.e[1], ut1, a.p, ay, j + 1, P, P + sy, fg_pair32(fc, flag[P + sy]), dt);
-            if (own_wu) Wu = face32t(a.u[2], a.e[2], ut2, a.p, az, k + 1, P, P + 1, fg_pair32(fc, flag[P + 1]), dt);
+        const int I = i + 2;
+        // Every load of the plane before its arithmetic.
+        const uint8_t fe = flag[P + sx], fs = flag[P - sy], fd = flag[P - 1];
+        const float u0e = ut0[P + sx], u1s = ut1[P - sy], u1c = ut1[P], u2d = ut2[P - 1], u2c = ut2[P];
+        const double pe64 = a.p[P + sx], ps64 = a.p[P - sy], pd64 = a.p[P - 1];
+        const double dinv = a.dinv[P];
+        uint8_t fn = SOLID, fu = SOLID;
+        float u1n = 0.f, u2u = 0.f;
+        double pn64 = 0.0, pu64 = 0.0;
+        if (own_vn) {
+            fn = flag[P + sy];
+            u1n = ut1[P + sy];
+            pn64 = a.p[P + sy];
         }
+        if (own_wu) {
+            fu = flag[P + 1];
+            u2u = ut2[P + 1];
+            pu64 = a.p[P + 1];
+        }
+        const float pe = d2f_int(pe64);
+        float Ue = face32t(ax.wm[I + 1], ax.wp[I + 1], ax.rdc[I + 1], u0c, u0e, pc, pe, dt);
+        float Vs = face32t(wms, wps, rds, u1s, u1c, d2f_int(ps64), pc, dt);
+        float Wd = face32t(wmd, wpd, rdd, u2d, u2c, d2f_int(pd64), pc, dt);
+        float Vn = 0.f, Wu = 0.f;
+        if (own_vn) Vn = face32t(wmn, wpn, rdn, u1c, u1n, pc, d2f_int(pn64), dt);
+        if (own_wu) Wu = face32t(wmu, wpu, rdu, u2c, u2u, pc, d2f_int(pu64), dt);
+        if (fg_pair32(fc, fe)) Ue = face32g(a.u[0], a.e[0], P, P + sx, ax.wm[I + 1], ax.wp[I + 1]);
+        if (fg_pair32(fs, fc)) Vs = face32g(a.u[1], a.e[1], P - sy, P, wms, wps);
+        if (fg_pair32(fd, fc)) Wd = face32g(a.u[2], a.e[2], P - 1, P, wmd, wpd);
+        if (own_vn && fg_pair32(fc, fn)) Vn = face32g(a.u[1], a.e[1], P, P + sy, wmn, wpn);
+        if (own_wu && fg_pair32(fc, fu)) Wu = face32g(a.u[2], a.e[2], P, P + 1, wmu, wpu);
         sVs[buf][ty][tx] = Vs;
         const float wnext = __shfl_down_sync(0xffffffffu, Wd, 1);
         __syncthreads();
-        if (!own_vn) Vn = sVs[buf][ty + 1][tx];
+        if (!own_vn) Vn = sVs[buf][min(ty + 1, UN_TJ - 1)][tx];
         if (!own_wu) Wu = wnext;
         buf ^= 1;
         if (live) {
@@ -338,14 +450,15 @@ k_ustar_faces32(const Grid g, const AxisF ax, const AxisF ay, const AxisF az, co
             if (k == g.nz - 1) a.Us[2][P + 1] = Wu64;
             double rhs = 0.0;
             if (fc == FLUID && !(bc.p_singular && i == 0 && j == 0 && k == 0)) {
-                const double div = (Ue64 - Uw64) * ax64.rd[i + 2] + (Vn64 - Vs64) * ay64.rd[j + 2] +
-                                   (Wu64 - Wd64) * az64.rd[k + 2];
-                rhs = div * m2re * a.dinv[P];   // -div / (2 Re coeffsum)
+                const double div = (Ue64 - Uw64) * ax64.rd[I] + (Vn64 - Vs64) * ay64.rd[J] + (Wu64 - Wd64) * az64.rd[K];
+                rhs = div * m2re * dinv;   // -div / (2 Re coeffsum)
             }
             a.b[P] = rhs;
         }
         Uw = Ue;
         fc = fe;
+        pc = pe;
+        u0c = u0e;
     }
 }
 
@@ -372,13 +485,11 @@ k_prhs_outer(const Grid g, const BCSet bc, const int *__restrict__ outer, const 
 void launch_ustar_prhs32_tiled(cudaStream_t s, const Grid &g, const AxisF axf[3], const Axis ax64[3],
                                const BCSet &bc, const uint8_t *flag, const Ustar32Args &a, float *ut, double dt,
                                double Re, const int *outer, int nout) {
-    const long long nt = (long long)(g.nx + 2) * (g.ny + 2) * (g.nz + 2);
-    k_utilde32<<<(unsigned)std::min<long long>((nt + 255) / 256, 8 * K32_BLOCKS), 256, 0, s>>>(
-        g, axf[0], axf[1], axf[2], a, ut, (float)dt);
-    const int tk = (g.nz + UN_TK - 1) / UN_TK, tj = (g.ny + UN_TJ - 1) / UN_TJ, planes = UN_PLANES;
-    const int nb = tk * tj * ((g.nx + planes - 1) / planes);
-    k_ustar_faces32<<<nb, dim3(UN_TK, UN_TJ), 0, s>>>(g, axf[0], axf[1], axf[2], ax64[0], ax64[1], ax64[2], bc, flag, a,
-                                                      ut, (float)dt, -1.0 / (2.0 * Re), tk, tj, planes);
+    k_utilde32<<<dim3((g.nz + 33) / 32, (g.ny + 9) / 8, g.nx + 2), dim3(32, 8), 0, s>>>(g, axf[0], axf[1], axf[2], a, ut,
+                                                                                       (float)dt);
+    const Tiles t(g);
+    k_ustar_faces32<<<t.nb, dim3(UN_TK, UN_TJ), 0, s>>>(g, axf[0], axf[1], axf[2], ax64[0], ax64[1], ax64[2], bc, flag, a,
+                                                        ut, (float)dt, -1.0 / (2.0 * Re), t);
     if (nout > 0) k_prhs_outer<<<(nout + 255) / 256, 256, 0, s>>>(g, bc, outer, nout, a.b);
     note_launches(nout > 0 ? 3 : 2);
 }
@@ -391,27 +502,28 @@ void launch_ustar_prhs32_tiled(cudaStream_t s, const Grid &g, const AxisF axf[3]
 // y face of the thread at j+1 (shared memory, one barrier per plane); the
 // high z face is the low z face of the next lane (warp shuffle).  Tile-edge
 // threads compute their high faces themselves.  Per fluid cell that is 3
-// face updates on the FP64 pipe instead of 6.  F32: the increment form of
+// face updates on the FP64 pipe instead of 6; the maximum runs on the
+// integer pipe and a plane's loads go out together (sphere 192x128x128 218
+// -> 160 us; its 16 FP64 operations per cell take 96 us).  F32: the increment form of
 // the FP32-stage step (the cell velocity takes the FP32 increment
 // e - dt G_c p'); otherwise the FP64 step.
 // ------------------------------------------------------------------------
 template <bool F32>
-__global__ void __launch_bounds__(UN_TK * UN_TJ)
+__global__ void __launch_bounds__(UN_TK * UN_TJ, 3)
 k_update_next_tiled(const Grid g, const Axis ax, const Axis ay, const Axis az, const DtAxis dx, const DtAxis dy,
                     const DtAxis dz, const AxisF axf, const AxisF ayf, const AxisF azf, const BCSet bc,
                     const uint8_t *__restrict__ flag, const NextArgs a64, const Next32Args a32, const double dt,
-                    const int tk, const int tj, const int planes, double *partials, unsigned int *counter,
-                    double *maxdiv_out) {
-    __shared__ double smem[32];
+                    const Tiles tl, double *partials, unsigned int *counter, double *maxdiv_out) {
+    __shared__ long long smem[32];
     __shared__ double sVs[2][UN_TJ][UN_TK];
     const double NaN = __longlong_as_double(0x7ff8000000000000LL);
     int b = blockIdx.x;
-    const int bk = b % tk;
-    b /= tk;
-    const int bj = b % tj, bi = b / tj;
+    const int bk = b % tl.tk;
+    b /= tl.tk;
+    const int bj = b % tl.tj, bi = b / tl.tj;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int k = bk * UN_TK + tx, j = bj * UN_TJ + ty;
-    const int i0 = bi * planes, i1 = min(i0 + planes, g.nx);
+    const int i0 = bi * tl.planes, i1 = min(i0 + tl.planes, g.nx);
     const bool live = j < g.ny && k < g.nz;
     const bool own_vn = ty == UN_TJ - 1 || j == g.ny - 1;
     const bool own_wu = tx == UN_TK - 1 || k == g.nz - 1;
@@ -421,33 +533,46 @@ k_update_next_tiled(const Grid g, const Axis ax, const Axis ay, const Axis az, c
     const double *pp = F32 ? a32.pp : a64.pp, *p = F32 ? a32.p : a64.p;
     double *const *Un = F32 ? a32.Un : a64.Un;
     double *const *un = F32 ? a32.un : a64.un;
+    const double *const *uo = F32 ? a32.u : a64.us;   // u^n, or u*
     double *pn = F32 ? a32.pn : a64.pn;
-    const int J = j + 2, K = k + 2;
-    double mdiv = 0.0;
-    long long P = live ? cidx(g, i0, j, k) : 0;
-    uint8_t fc = live ? flag[P] : (uint8_t)SOLID;
-    double ppc = live ? pp[P] : 0.0;
-    double Uw = NaN;
-    if (live && flag[P - sx] != SOLID && fc != SOLID) Uw = Us0[P] - dx.dtrdc[i0 + 2] * (ppc - pp[P - sx]);
+    // Threads off the grid follow a column inside it and store nothing.
+    const int jc = min(j, g.ny - 1), kc = min(k, g.nz - 1), J = jc + 2, K = kc + 2;
+    const double dys = dy.dtrdc[J], dyn = dy.dtrdc[J + 1], dzd = dz.dtrdc[K], dzu = dz.dtrdc[K + 1];
+    const double rdy = ay.rd[J], rdz = az.rd[K];
+    long long mdiv = 0;   // max|div U| as the bits of a double >= 0 (ordered as integers; NaN largest)
+    long long P = cidx(g, i0, jc, kc);
+    uint8_t fc = flag[P];
+    double ppc = pp[P], ppw = pp[P - sx];
+    double Uw = flag[P - sx] != SOLID && fc != SOLID ? Us0[P] - dx.dtrdc[i0 + 2] * (ppc - ppw) : NaN;
     int buf = 0;
     for (int i = i0; i < i1; i++, P += sx) {
         const int I = i + 2;
-        double Ue = NaN, Vs = NaN, Wd = NaN, Vn = NaN, Wu = NaN;
-        uint8_t fe = SOLID;
-        double ppe = 0.0;
-        if (live) {
-            fe = flag[P + sx];
-            ppe = pp[P + sx];
-            if (fc != SOLID && fe != SOLID) Ue = Us0[P + sx] - dx.dtrdc[I + 1] * (ppe - ppc);
-            if (fc != SOLID && flag[P - sy] != SOLID) Vs = Us1[P] - dy.dtrdc[J] * (ppc - pp[P - sy]);
-            if (fc != SOLID && flag[P - 1] != SOLID) Wd = Us2[P] - dz.dtrdc[K] * (ppc - pp[P - 1]);
-            if (own_vn && fc != SOLID && flag[P + sy] != SOLID) Vn = Us1[P + sy] - dy.dtrdc[J + 1] * (pp[P + sy] - ppc);
-            if (own_wu && fc != SOLID && flag[P + 1] != SOLID) Wu = Us2[P + 1] - dz.dtrdc[K + 1] * (pp[P + 1] - ppc);
+        // Every load of the plane before its arithmetic (behind the flags'
+        // tests they cost three latencies per plane).
+        const uint8_t fe = flag[P + sx], fs = flag[P - sy], fd = flag[P - 1], fn = flag[P + sy], fu = flag[P + 1];
+        const double ppe = pp[P + sx], pps = pp[P - sy], ppn = pp[P + sy], ppd = pp[P - 1], ppu = pp[P + 1];
+        const double ue = Us0[P + sx], vs = Us1[P], wd = Us2[P], pc = p[P];
+        const double o0 = uo[0][P], o1 = uo[1][P], o2 = uo[2][P];
+        float e0 = 0.f, e1 = 0.f, e2 = 0.f;
+        if (F32) {
+            e0 = a32.e[0][P];
+            e1 = a32.e[1][P];
+            e2 = a32.e[2][P];
         }
+        double vn = 0.0, wu = 0.0;
+        if (own_vn) vn = Us1[P + sy];
+        if (own_wu) wu = Us2[P + 1];
+        const bool in = fc != SOLID;
+        const double Ue = in && fe != SOLID ? ue - dx.dtrdc[I + 1] * (ppe - ppc) : NaN;
+        const double Vs = in && fs != SOLID ? vs - dys * (ppc - pps) : NaN;
+        const double Wd = in && fd != SOLID ? wd - dzd * (ppc - ppd) : NaN;
+        double Vn = NaN, Wu = NaN;
+        if (own_vn && in && fn != SOLID) Vn = vn - dyn * (ppn - ppc);
+        if (own_wu && in && fu != SOLID) Wu = wu - dzu * (ppu - ppc);
         sVs[buf][ty][tx] = Vs;
         const double wnext = __shfl_down_sync(0xffffffffu, Wd, 1);
         __syncthreads();
-        if (!own_vn) Vn = sVs[buf][ty + 1][tx];
+        if (!own_vn) Vn = sVs[buf][min(ty + 1, UN_TJ - 1)][tx];
         if (!own_wu) Wu = wnext;
         buf ^= 1;
         if (live) {
@@ -457,25 +582,24 @@ k_update_next_tiled(const Grid g, const Axis ax, const Axis ay, const Axis az, c
             if (i == g.nx - 1) Un[0][P + sx] = Ue;
             if (j == g.ny - 1) Un[1][P + sy] = Vn;
             if (k == g.nz - 1) Un[2][P + 1] = Wu;
-            pn[P] = (fc == FLUID || fc == GHOST) ? p[P] + ppc : NaN;
+            pn[P] = (fc == FLUID || fc == GHOST) ? pc + ppc : NaN;
             if (fc == FLUID) {
-                const double ppw = pp[P - sx], pps = pp[P - sy], ppn = pp[P + sy], ppd = pp[P - 1], ppu = pp[P + 1];
                 if (F32) {
                     const float gx = (d2f_int(ppe) - d2f_int(ppw)) * axf.rdcc[I];
                     const float gy = (d2f_int(ppn) - d2f_int(pps)) * ayf.rdcc[J];
                     const float gz = (d2f_int(ppu) - d2f_int(ppd)) * azf.rdcc[K];
                     const float dtf = (float)dt;
-                    un[0][P] = a32.u[0][P] + f2d_int(a32.e[0][P] - dtf * gx);
-                    un[1][P] = a32.u[1][P] + f2d_int(a32.e[1][P] - dtf * gy);
-                    un[2][P] = a32.u[2][P] + f2d_int(a32.e[2][P] - dtf * gz);
+                    un[0][P] = o0 + f2d_int(e0 - dtf * gx);
+                    un[1][P] = o1 + f2d_int(e1 - dtf * gy);
+                    un[2][P] = o2 + f2d_int(e2 - dtf * gz);
                 } else {
-                    un[0][P] = a64.us[0][P] - dx.dtrdcc[I] * (ppe - ppw);
-                    un[1][P] = a64.us[1][P] - dy.dtrdcc[J] * (ppn - pps);
-                    un[2][P] = a64.us[2][P] - dz.dtrdcc[K] * (ppu - ppd);
+                    un[0][P] = o0 - dx.dtrdcc[I] * (ppe - ppw);
+                    un[1][P] = o1 - dy.dtrdcc[J] * (ppn - pps);
+                    un[2][P] = o2 - dz.dtrdcc[K] * (ppu - ppd);
                 }
                 if (!(bc.p_singular && i == 0 && j == 0 && k == 0)) {
-                    const double div = (Ue - Uw) * ax.rd[I] + (Vn - Vs) * ay.rd[J] + (Wu - Wd) * az.rd[K];
-                    mdiv = nanmax(mdiv, fabs(div));
+                    const double div = (Ue - Uw) * ax.rd[I] + (Vn - Vs) * rdy + (Wu - Wd) * rdz;
+                    mdiv = max(mdiv, __double_as_longlong(div) & 0x7fffffffffffffffLL);
                 }
             } else if (fc == SOLID) {
                 un[0][P] = un[1][P] = un[2][P] = NaN;
@@ -483,38 +607,37 @@ k_update_next_tiled(const Grid g, const Axis ax, const Axis ay, const Axis az, c
         }
         Uw = Ue;
         fc = fe;
+        ppw = ppc;
         ppc = ppe;
     }
     // Maximum over the block, then over the blocks (the last block to
-    // finish reduces every block's value in a fixed order).
+    // finish reduces every block's value).  Integer maxima of the bits keep
+    // the FP64 pipe free and NaN largest.
     const int t = ty * UN_TK + tx, lane = t & 31, warp = t >> 5;
-    double x = mdiv;
+    auto block_max = [&](long long x) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x = nanmax(x, __shfl_down_sync(0xffffffffu, x, o));
-    if (lane == 0) smem[warp] = x;
-    __syncthreads();
+        for (int o = 16; o > 0; o >>= 1) x = max(x, __shfl_down_sync(0xffffffffu, x, o));
+        __syncthreads();
+        if (lane == 0) smem[warp] = x;
+        __syncthreads();
+        for (int w = 0; w < (UN_TK * UN_TJ) / 32; w++) x = max(x, smem[w]);
+        return x;   // of the whole block in thread 0
+    };
+    long long m = block_max(mdiv);
     __shared__ bool last;
     if (t == 0) {
-        double m = 0.0;
-        for (int w = 0; w < (UN_TK * UN_TJ) / 32; w++) m = nanmax(m, smem[w]);
-        partials[blockIdx.x] = m;
+        partials[blockIdx.x] = __longlong_as_double(m);
         __threadfence();
         last = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
-    double m = 0.0;
-    for (int q = t; q < (int)gridDim.x; q += UN_TK * UN_TJ) m = nanmax(m, __ldcg(partials + q));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = nanmax(m, __shfl_down_sync(0xffffffffu, m, o));
-    __syncthreads();
-    if (lane == 0) smem[warp] = m;
-    __syncthreads();
+    m = 0;
+    for (int q = t; q < (int)gridDim.x; q += UN_TK * UN_TJ) m = max(m, __double_as_longlong(__ldcg(partials + q)));
+    m = block_max(m);
     if (t == 0) {
-        double r = 0.0;
-        for (int w = 0; w < (UN_TK * UN_TJ) / 32; w++) r = nanmax(r, smem[w]);
-        *maxdiv_out = r;
+        *maxdiv_out = __longlong_as_double(m);
         *counter = 0;
     }
 }
@@ -523,21 +646,16 @@ void launch_update_next_tiled(cudaStream_t s, const Grid &g, const Axis ax64[3],
                               const AxisF axf[3], const BCSet &bc, const uint8_t *flag, const NextArgs *a64,
                               const Next32Args *a32, double dt, double *partials, unsigned int *counter,
                               double *maxdiv_out) {
-    const int tk = (g.nz + UN_TK - 1) / UN_TK, tj = (g.ny + UN_TJ - 1) / UN_TJ;
-    // UN_PLANES planes per tile, more on grids whose tiles would outnumber
-    // the reduction's partials (8 x 4096).
-    int planes = UN_PLANES;
-    while ((long long)tk * tj * ((g.nx + planes - 1) / planes) > 8 * 4096) planes *= 2;
-    const int nb = tk * tj * ((g.nx + planes - 1) / planes);
+    const Tiles t(g);
     const dim3 blk(UN_TK, UN_TJ);
     if (a32)
-        k_update_next_tiled<true><<<nb, blk, 0, s>>>(g, ax64[0], ax64[1], ax64[2], dta[0], dta[1], dta[2], axf[0],
-                                                    axf[1], axf[2], bc, flag, NextArgs{}, *a32, dt, tk, tj, planes,
-                                                    partials, counter, maxdiv_out);
+        k_update_next_tiled<true><<<t.nb, blk, 0, s>>>(g, ax64[0], ax64[1], ax64[2], dta[0], dta[1], dta[2], axf[0],
+                                                      axf[1], axf[2], bc, flag, NextArgs{}, *a32, dt, t, partials,
+                                                      counter, maxdiv_out);
     else
-        k_update_next_tiled<false><<<nb, blk, 0, s>>>(g, ax64[0], ax64[1], ax64[2], dta[0], dta[1], dta[2], axf[0],
-                                                     axf[1], axf[2], bc, flag, *a64, Next32Args{}, dt, tk, tj,
-                                                     planes, partials, counter, maxdiv_out);
+        k_update_next_tiled<false><<<t.nb, blk, 0, s>>>(g, ax64[0], ax64[1], ax64[2], dta[0], dta[1], dta[2], axf[0],
+                                                       axf[1], axf[2], bc, flag, *a64, Next32Args{}, dt, t, partials,
+                                                       counter, maxdiv_out);
     note_launches(1);
 }
 
