@@ -130,8 +130,7 @@ k_fp_gather(const OpT<T> c, const S *__restrict__ r, T *__restrict__ f, const Fp
 // of both halves and the register tiles' shared-memory reads bound them
 // now); cavity 64^3 FP64, an application: 0.36 -> 0.23 ms.
 //
-// Tiles: TM = 64 (R = 8) in FP32, 32 (R = 4) in FP64 and on FP32 grids whose
-// 64-tiles would leave SMs without a block (run).
+// Tiles: TM = 64 (R = 8) or 32 in FP32, 32 (R = 4) or 16 in FP64 (run).
 template <typename T, int TM>
 struct FpTile {
     static constexpr int R = TM / 8, R2 = R / 2, V = 16 / (int)sizeof(T);
@@ -699,24 +698,29 @@ k_fp_patch(const FpPatches<T> p, const S *__restrict__ r, const T *__restrict__ 
     __shared__ T v[FP_PMAX], f[FP_PMAX];
     const int b = blockIdx.x, s0 = p.start[b], nr = p.count[3 * b], nb = p.count[3 * b + 1], ng = p.count[3 * b + 2];
     const int n = nr + nb + ng;
+    auto cell = [&](int q) {
+        const int c = p.loc[s0 + q];
+        return c < 0 ? ~c : c;
+    };
     for (int q = threadIdx.x; q < n; q += FP_PT) {
-        const int P = p.P[s0 + q];
+        const int c = cell(q), P = p.P[c];
         v[q] = z[P];
-        T t = p.rw[s0 + q] * fp_value<T, S>(r[P]);
+        T t = p.rw[c] * fp_value<T, S>(r[P]);
 #pragma unroll
         for (int e = 0; e < 8; e++) {
-            const int m = p.ref[(size_t)e * p.nloc + s0 + q];
-            if (m < 0) t += p.w[(size_t)e * p.nloc + s0 + q] * z[~m];
+            const int Q = p.to[e * p.ncell + c];
+            if (Q >= 0 && p.ref[(size_t)e * p.nloc + s0 + q] < 0) t += p.w[e * p.ncell + c] * z[Q];
         }
         f[q] = t;
     }
     __syncthreads();
     // Rows of this thread's cells: couplings inside the patch.
     auto row = [&](int q, int ne) {
+        const int c = cell(q);
         T t = f[q];
         for (int e = 0; e < ne; e++) {
             const int m = p.ref[(size_t)e * p.nloc + s0 + q];
-            if (m >= 0 && m != FP_NONE) t += p.w[(size_t)e * p.nloc + s0 + q] * v[m];
+            if (m >= 0) t += p.w[e * p.ncell + c] * v[m];
         }
         return t;
     };
@@ -729,7 +733,7 @@ k_fp_patch(const FpPatches<T> p, const S *__restrict__ r, const T *__restrict__ 
 #pragma unroll
         for (int u = 0; u < (FP_PMAX + FP_PT - 1) / FP_PT; u++) {
             const int q = nr + nb + u * FP_PT + threadIdx.x;
-            if (q < n) g[u] = row(q, 8) + p.self[s0 + q] * v[q];
+            if (q < n) g[u] = row(q, 8) + p.self[cell(q)] * v[q];
         }
         __syncthreads();
 #pragma unroll
@@ -740,8 +744,8 @@ k_fp_patch(const FpPatches<T> p, const S *__restrict__ r, const T *__restrict__ 
         __syncthreads();
     }
     for (int q = threadIdx.x; q < n; q += FP_PT) {
-        const int m = p.slot[s0 + q];
-        if (m >= 0) out[m] = v[q];
+        const int c = p.loc[s0 + q];
+        if (c >= 0) out[c] = v[q];
     }
 }
 
@@ -857,48 +861,74 @@ FastPoisson<T>::~FastPoisson() {
     for (void *p : allocs_) cudaFree(p);
 }
 
-// The cells near the body, their rows and the patches (k_fp_patch).
-template <typename T>
-template <typename Put>
-bool FastPoisson<T>::build_patches(const OpT<T> &A, const FastPoissonGeom &h, const std::vector<double> &gw, Put put) {
+// The cells near the body, their rows and the patches (k_fp_patch), cut by
+// cubes of side `cube`; false when a patch cannot be made small enough.
+static bool build_patches(const OpT<double> &A, const FastPoissonGeom &h, const std::vector<double> &gw, int cube,
+                          FpPatchTables &t_) {
     const Grid &g = A.g;
     const int n[3] = {g.nx, g.ny, g.nz};
     const long long st[3] = {g.sx, g.sy, 1};
     std::vector<int> id(g.ncell, -1);   // near cell number of a padded index
-    std::vector<int> cells = h.gcell, cur = h.gcell;
-    for (size_t q = 0; q < cells.size(); q++) id[cells[q]] = (int)q;
-    const int ng = nghost_;
+    std::vector<int> cells, ijk;
+    const int ng = (int)h.gcell.size();
+    cells.reserve(32 * (size_t)ng);
+    ijk.reserve(96 * (size_t)ng);
+    auto push = [&](long long Q, int i, int j, int k) {
+        id[Q] = (int)cells.size();
+        cells.push_back((int)Q);
+        ijk.push_back(i);
+        ijk.push_back(j);
+        ijk.push_back(k);
+    };
+    auto add = [&](long long Q, int i, int j, int k) {
+        if (i < 0 || i >= n[0] || j < 0 || j >= n[1] || k < 0 || k >= n[2] || id[Q] >= 0 || h.flag[Q] != FLUID) return;
+        if (!(A.p_singular && Q == A.pinned)) push(Q, i, j, k);
+    };
+    auto split = [&](int Q, int &i, int &j, int &k) {
+        const uint32_t I = (uint32_t)Q / (uint32_t)g.sx, r = (uint32_t)Q - I * (uint32_t)g.sx, J = r / (uint32_t)g.sy;
+        i = (int)I - 2;
+        j = (int)J - 2;
+        k = (int)(r - J * (uint32_t)g.sy) - 2;
+    };
+    int i, j, k;
+    for (int Q : h.gcell) {
+        split(Q, i, j, k);
+        push(Q, i, j, k);
+    }
+    size_t first = 0;   // the last layer's cells
     for (int layer = 0; layer < FP_LAYERS; layer++) {
-        std::vector<int> next;
-        auto add = [&](long long Q) {
-            int i, j, k;
-            cijk(g, Q, i, j, k);
-            if (i < 0 || i >= n[0] || j < 0 || j >= n[1] || k < 0 || k >= n[2] || id[Q] >= 0 || h.flag[Q] != FLUID) return;
-            if (A.p_singular && Q == A.pinned) return;
-            id[Q] = (int)cells.size();
-            cells.push_back((int)Q);
-            next.push_back((int)Q);
-        };
+        const size_t last = cells.size();
         if (layer == 0)
-            for (int q : h.gidx)
-                if (q >= 0) add(q);
-        for (int P : cur)
-            for (int a = 0; a < 3; a++) {
-                add(P - st[a]);
-                add(P + st[a]);
-            }
-        cur = next;
+            for (int Q : h.gidx)
+                if (Q >= 0 && id[Q] < 0) {
+                    split(Q, i, j, k);
+                    add(Q, i, j, k);
+                }
+        for (size_t q = first; q < last; q++) {
+            const long long Q = cells[q];
+            i = ijk[3 * q];
+            j = ijk[3 * q + 1];
+            k = ijk[3 * q + 2];
+            add(Q - st[0], i - 1, j, k);
+            add(Q + st[0], i + 1, j, k);
+            add(Q - st[1], i, j - 1, k);
+            add(Q + st[1], i, j + 1, k);
+            add(Q - st[2], i, j, k - 1);
+            add(Q + st[2], i, j, k + 1);
+        }
+        first = last;
     }
     const int nc = (int)cells.size();
     // Rows: couplings (padded index, weight), weight of the old value and of
     // the residual.  Ghost rows are relaxed as the multigrid relaxes them.
-    std::vector<int> to((size_t)nc * 8, -1);
-    std::vector<double> w((size_t)nc * 8, 0.0), self(nc, 0.0), rw(nc, 1.0);
-    std::vector<int> ijk((size_t)nc * 3);
+    t_.to.assign((size_t)nc * 8, -1);
+    t_.w.assign((size_t)nc * 8, 0.0);
+    t_.self.assign(nc, 0.0);
+    t_.rw.assign(nc, 1.0);
+    std::vector<int> &to = t_.to;   // [8][nc]
     for (int q = 0; q < nc; q++) {
-        int *x = &ijk[3 * (size_t)q];
-        cijk(g, cells[q], x[0], x[1], x[2]);
-        for (int a = 0; a < 3; a++) near_outer_ = near_outer_ || x[a] < 2 || x[a] >= n[a] - 2;
+        const int *x = &ijk[3 * (size_t)q];
+        for (int a = 0; a < 3; a++) t_.near_outer = t_.near_outer || x[a] < 2 || x[a] >= n[a] - 2;
         if (q < ng) {
             double off = 0;
             for (int e = 0; e < 8; e++) {
@@ -907,62 +937,68 @@ bool FastPoisson<T>::build_patches(const OpT<T> &A, const FastPoissonGeom &h, co
             }
             const double dg = 1.0 - h.gwself[q], dv = 1.0 / std::max({dg, 2.0 * off, 1e-3});
             for (int e = 0; e < 8; e++) {
-                to[8 * (size_t)q + e] = h.gidx[8 * (size_t)q + e];
-                w[8 * (size_t)q + e] = dv * gw[8 * (size_t)q + e];
+                to[(size_t)e * nc + q] = h.gidx[8 * (size_t)q + e];
+                t_.w[(size_t)e * nc + q] = dv * gw[8 * (size_t)q + e];
             }
-            self[q] = 1.0 - dg * dv;
-            rw[q] = dv;
+            t_.self[q] = 1.0 - dg * dv;
+            t_.rw[q] = dv;
         } else {
             double sum = 0;
             for (int a = 0; a < 3; a++) sum += h.km[a][x[a]] + h.kp[a][x[a]];
             for (int a = 0; a < 3; a++) {
-                to[8 * (size_t)q + 2 * a] = (int)(cells[q] - st[a]);
-                to[8 * (size_t)q + 2 * a + 1] = (int)(cells[q] + st[a]);
-                w[8 * (size_t)q + 2 * a] = h.km[a][x[a]] / sum;
-                w[8 * (size_t)q + 2 * a + 1] = h.kp[a][x[a]] / sum;
+                to[(size_t)(2 * a) * nc + q] = (int)(cells[q] - st[a]);
+                to[(size_t)(2 * a + 1) * nc + q] = (int)(cells[q] + st[a]);
+                t_.w[(size_t)(2 * a) * nc + q] = h.km[a][x[a]] / sum;
+                t_.w[(size_t)(2 * a + 1) * nc + q] = h.kp[a][x[a]] / sum;
             }
         }
     }
+    // The cells each row couples to, by number (-1: not near the body).
+    std::vector<int> nbr((size_t)nc * 8);
+    for (int q = 0; q < nc; q++)
+        for (int e = 0; e < 8; e++) {
+            const int Q = to[(size_t)e * nc + q];
+            nbr[8 * (size_t)q + e] = Q >= 0 ? id[Q] : -1;
+        }
     // Patches: cubes of the grid, halved until each fits with its overlap.
     std::vector<std::vector<int>> todo;
     {
-        std::vector<std::pair<std::array<int, 3>, int>> key(nc);
-        for (int q = 0; q < nc; q++)
-            key[q] = {{ijk[3 * (size_t)q] / FP_CUBE, ijk[3 * (size_t)q + 1] / FP_CUBE, ijk[3 * (size_t)q + 2] / FP_CUBE}, q};
-        std::sort(key.begin(), key.end());
+        const int cy = (n[1] + cube - 1) / cube, cz = (n[2] + cube - 1) / cube;
+        std::vector<int> at((size_t)((n[0] + cube - 1) / cube) * cy * cz, -1);
         for (int q = 0; q < nc; q++) {
-            if (q == 0 || key[q].first != key[q - 1].first) todo.emplace_back();
-            todo.back().push_back(key[q].second);
+            const int *x = &ijk[3 * (size_t)q];
+            int &b = at[((size_t)(x[0] / cube) * cy + x[1] / cube) * cz + x[2] / cube];
+            if (b < 0) {
+                b = (int)todo.size();
+                todo.emplace_back();
+            }
+            todo[b].push_back(q);
         }
     }
-    std::vector<int> start, count, P, slot, mark(nc, -1);
-    std::vector<int> loc_cell;
-    std::vector<int> order;   // near cells in output order
-    std::vector<int> pos(nc);
-    int stamp = 0;
+    std::vector<int> mark(nc, -1), all, list[3], pos(nc);
+    std::vector<int16_t> refs;   // [local][8] of every patch
     for (size_t t = 0; t < todo.size(); t++) {
-        std::vector<int> own = todo[t], all = own;
-        stamp++;
-        std::vector<int> front = own;
+        const std::vector<int> own = todo[t];
+        const int stamp = (int)t;
+        all = own;
         for (int q : own) mark[q] = stamp;
+        size_t from = 0;
         for (int o = 0; o < FP_OVERLAP; o++) {
-            std::vector<int> next;
-            auto grow = [&](long long Q) {
-                const int m = Q >= 0 && Q < g.ncell ? id[Q] : -1;
-                if (m < 0 || mark[m] == stamp) return;
-                mark[m] = stamp;
-                next.push_back(m);
-            };
-            for (int q : front) {
-                for (int e = 0; e < 8; e++)
-                    if (to[8 * (size_t)q + e] >= 0) grow(to[8 * (size_t)q + e]);
-                for (int a = 0; a < 3; a++) {
-                    grow(cells[q] - st[a]);
-                    grow(cells[q] + st[a]);
+            const size_t upto = all.size();
+            for (size_t l = from; l < upto; l++) {
+                const int q = all[l];
+                auto grow = [&](int m) {
+                    if (m < 0 || mark[m] == stamp) return;
+                    mark[m] = stamp;
+                    all.push_back(m);
+                };
+                for (int e = 0; e < 8; e++) grow(nbr[8 * (size_t)q + e]);
+                for (int a = 0; q < ng && a < 3; a++) {
+                    grow(id[cells[q] - st[a]]);
+                    grow(id[cells[q] + st[a]]);
                 }
             }
-            all.insert(all.end(), next.begin(), next.end());
-            front = next;
+            from = upto;
         }
         if ((int)all.size() > FP_PMAX) {   // split the cube along its longest side
             if (own.size() < 2) return false;
@@ -986,68 +1022,42 @@ bool FastPoisson<T>::build_patches(const OpT<T> &A, const FastPoissonGeom &h, co
             todo.push_back(a1);
             continue;
         }
-        // Local order: red, black, ghost; by padded index within each.
-        auto kind = [&](int q) {
-            return q < ng ? 2 : (ijk[3 * (size_t)q] + ijk[3 * (size_t)q + 1] + ijk[3 * (size_t)q + 2]) & 1;
-        };
-        std::vector<int> list(all);
-        std::sort(list.begin(), list.end(), [&](int x, int y) {
-            const int kx = kind(x), ky = kind(y);
-            return kx != ky ? kx < ky : cells[x] < cells[y];
-        });
-        int c3[3] = {0, 0, 0};
-        start.push_back((int)loc_cell.size());
-        std::vector<int> sorted_own(own);
-        std::sort(sorted_own.begin(), sorted_own.end());
-        for (int q : list) {
-            c3[kind(q)]++;
-            loc_cell.push_back(q);
-            const bool mine = std::binary_search(sorted_own.begin(), sorted_own.end(), q);
-            slot.push_back(mine ? (int)order.size() : -1);
-            if (mine) order.push_back(q);
-            P.push_back(cells[q]);
+        // Local order: red, black, ghost; the patch's own cells are the
+        // first own.size() of `all`.
+        for (auto &l : list) l.clear();
+        for (size_t l = 0; l < all.size(); l++) {
+            const int q = all[l], *x = &ijk[3 * (size_t)q];
+            list[q < ng ? 2 : (x[0] + x[1] + x[2]) & 1].push_back(l < own.size() ? q : ~q);
         }
-        count.insert(count.end(), c3, c3 + 3);
-    }
-    npatch_ = (int)start.size();
-    nnear_ = nc;
-    const int nloc = (int)loc_cell.size();
-    std::vector<int> ref(8 * (size_t)nloc, FP_NONE);
-    std::vector<T> lw(8 * (size_t)nloc, (T)0), ls(nloc), lr(nloc);
-    for (int b = 0; b < npatch_; b++) {
-        const int s0 = start[b], s1 = b + 1 < npatch_ ? start[b + 1] : nloc;
-        for (int l = s0; l < s1; l++) pos[loc_cell[l]] = l - s0, mark[loc_cell[l]] = ~b;
-        for (int l = s0; l < s1; l++) {
-            const int q = loc_cell[l];
-            ls[l] = (T)self[q];
-            lr[l] = (T)rw[q];
-            for (int e = 0; e < 8; e++) {
-                const int Q = to[8 * (size_t)q + e];
-                if (Q < 0) continue;
-                const int m = id[Q];
-                ref[(size_t)e * nloc + l] = m >= 0 && mark[m] == ~b ? pos[m] : ~Q;
-                lw[(size_t)e * nloc + l] = (T)w[8 * (size_t)q + e];
+        t_.start.push_back((int)t_.loc.size());
+        int k_ = 0;
+        for (const auto &l : list) {
+            t_.count.push_back((int)l.size());
+            for (int u : l) {
+                t_.loc.push_back(u);
+                pos[u < 0 ? ~u : u] = k_++;
             }
         }
+        for (const auto &l : list)
+            for (int u : l) {
+                const int q = u < 0 ? ~u : u;
+                for (int e = 0; e < 8; e++) {
+                    const int m = nbr[8 * (size_t)q + e];
+                    refs.push_back(m >= 0 && mark[m] == stamp ? (int16_t)pos[m] : (int16_t)-1);
+                }
+            }
     }
-    std::vector<int> out_cell(nc);
-    for (int q = 0; q < nc; q++) out_cell[q] = cells[order[q]];
-    patch_.start = (const int *)put(start.data(), sizeof(int) * start.size());
-    patch_.count = (const int *)put(count.data(), sizeof(int) * count.size());
-    patch_.P = (const int *)put(P.data(), sizeof(int) * P.size());
-    patch_.slot = (const int *)put(slot.data(), sizeof(int) * slot.size());
-    patch_.ref = (const int *)put(ref.data(), sizeof(int) * ref.size());
-    patch_.w = (const T *)put(lw.data(), sizeof(T) * lw.size());
-    patch_.self = (const T *)put(ls.data(), sizeof(T) * ls.size());
-    patch_.rw = (const T *)put(lr.data(), sizeof(T) * lr.size());
-    patch_.nloc = nloc;
-    near_cell_ = (const int *)put(out_cell.data(), sizeof(int) * nc);
-    near_val_ = (T *)put(nullptr, sizeof(T) * nc);
-    return near_val_ != nullptr;
+    const size_t nloc = t_.loc.size();
+    t_.ref.resize(8 * nloc);
+    for (size_t l = 0; l < nloc; l++)
+        for (int e = 0; e < 8; e++) t_.ref[e * nloc + l] = refs[8 * l + e];
+    t_.P = cells;
+    return true;
 }
 
 template <typename T>
-int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &A, const FastPoissonGeom &h) {
+int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &A, const FastPoissonGeom &h,
+                          double max_ops) {
     const Grid &g = A.g;
     const int n[3] = {g.nx, g.ny, g.nz};
     const int lo[3] = {F_W, F_S, F_D}, hi[3] = {F_E, F_N, F_U};
@@ -1062,15 +1072,24 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
     A_ = A;
     nghost_ = (int)h.gcell.size();
     bool ok = true;
+    // Device arrays from chunks (an allocation each would be most of the
+    // set-up of a small case).  A copy from pageable memory has read its
+    // source when the call returns.
+    char *chunk = nullptr;
+    size_t left = 0;
     auto put = [&](const void *src, size_t bytes) -> void * {
-        void *p = nullptr;
-        if (!ok || cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
-            ok = false;
-            return nullptr;
+        const size_t need = (bytes + 255) & ~(size_t)255;
+        if (ok && need > left) {
+            const size_t size = std::max(need, (size_t)1 << 20);
+            ok = cudaMalloc((void **)&chunk, size) == cudaSuccess;
+            if (ok) allocs_.push_back(chunk);
+            left = size;
         }
-        allocs_.push_back(p);
-        if (src) ok = cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-                      cudaStreamSynchronize(s) == cudaSuccess;
+        if (!ok) return nullptr;
+        void *p = chunk;
+        chunk += need;
+        left -= need;
+        if (src && bytes) ok = cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess;
         return p;
     };
     std::vector<double> lam[3], diag;
@@ -1162,6 +1181,10 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
         if (A.p_singular) lam[a][zero_[a]] = 0.0;   // the constants
         row0_[a] = (T *)put(row0[a].data(), sizeof(T) * row0[a].size());
     }
+    double ops = 0;
+    for (int a = 0; a < 3; a++)
+        if (a != tri_) ops += 4.0 * n[0] * n[1] * n[2] * modes_[a].ne;
+    if (ops > max_ops) return 1;
     ld_ = modes_[2].ld;
     v0_ = (T *)put(v0.data(), sizeof(T) * v0.size());
     const size_t cells = (size_t)n[0] * n[1] * ld_;
@@ -1216,7 +1239,19 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
         std::vector<T> sc(nghost_);
         for (int q = 0; q < nghost_; q++) sc[q] = (T)(1.0 / std::max(1.0 - h.gwself[q], 1e-3));
         gscale_ = (T *)put(sc.data(), sizeof(T) * nghost_);
-        if (!build_patches(A, h, gw, put)) return -1;
+        FpPatchTables t;
+        if (!build_patches(A64, h, gw, FP_CUBE<T>, t)) return 1;
+        auto ints = [&](const std::vector<int> &v) { return (const int *)put(v.data(), sizeof(int) * v.size()); };
+        auto reals = [&](const std::vector<double> &v) {
+            const std::vector<T> c(v.begin(), v.end());
+            return (const T *)put(c.data(), sizeof(T) * c.size());
+        };
+        npatch_ = (int)t.start.size();
+        near_outer_ = t.near_outer;
+        patch_ = FpPatches<T>{ints(t.P), ints(t.to), reals(t.w), reals(t.self), reals(t.rw), (int)t.P.size(),
+                              ints(t.start), ints(t.count), ints(t.loc),
+                              (const int16_t *)put(t.ref.data(), sizeof(int16_t) * t.ref.size()), (int)t.loc.size()};
+        near_val_ = (T *)put(nullptr, sizeof(T) * t.P.size());
     }
     if (!ok) return -1;
     return cudaStreamSynchronize(s) == cudaSuccess ? 0 : -1;
@@ -1295,14 +1330,17 @@ void FastPoisson<T>::backward(cudaStream_t s, int axis, const T *in, T *out, con
 template <typename T>
 template <typename S>
 void FastPoisson<T>::run(cudaStream_t s, const S *r, T *z, const int *gate) {
-    // FP64, and FP32 grids with fewer 64 x 64 tiles than SMs (times two:
-    // below that a 32-tile grid's shorter blocks win), take 32 x 32 tiles.
+    // The smaller tile where the larger would leave SMs without work: FP32
+    // below two 64-tiles per SM, FP64 (two multiply-adds per clock and SM, so
+    // an uneven share of tiles is an uneven share of the time) below twelve
+    // 32-tiles per SM.
+    const Grid &g = A_.g;
+    auto tiles = [&](int t) { return (long long)((g.nx * g.ny + t - 1) / t) * ((ld_ + t - 1) / t); };
     if constexpr (sizeof(T) == 8) {
-        run_tiled<32, S>(s, r, z, gate);
+        if (tiles(32) < 12 * 152) run_tiled<16, S>(s, r, z, gate);
+        else run_tiled<32, S>(s, r, z, gate);
     } else {
-        const Grid &g = A_.g;
-        const long long tiles = (long long)((g.nx * g.ny + 63) / 64) * ((ld_ + 63) / 64);
-        if (tiles < 2 * 152) run_tiled<32, S>(s, r, z, gate);
+        if (tiles(64) < 2 * 152) run_tiled<32, S>(s, r, z, gate);
         else run_tiled<64, S>(s, r, z, gate);
     }
 }
@@ -1374,7 +1412,7 @@ void FastPoisson<T>::run_tiled(cudaStream_t s, const S *r, T *z, const int *gate
     const int nout = A_.sw.nout;
     auto edges = [&](int outer, int solids, int swept) {
         launch_pdl(k_fp_edges<T, S>, (outer + solids + swept + 255) / 256, 256, 0, s, A_, r, z, A_.sw.outer, outer,
-                   (const int *)solid_, solids, near_cell_, (const T *)near_val_, swept, gate);
+                   (const int *)solid_, solids, patch_.P, (const T *)near_val_, swept, gate);
         k++;
     };
     k += 3;
@@ -1382,10 +1420,10 @@ void FastPoisson<T>::run_tiled(cudaStream_t s, const S *r, T *z, const int *gate
         if (near_outer_) edges(nout, nsolid_, 0);   // the sweeps read outer values
         launch_pdl(k_fp_patch<T, S>, npatch_, FP_PT, 0, s, patch_, r, (const T *)z, near_val_, FP_SWEEPS, gate);
         k++;
-        if (near_outer_) edges(0, 0, nnear_);
+        if (near_outer_) edges(0, 0, patch_.ncell);
     }
     if (near_outer_ || nghost_ == 0) edges(nout, nsolid_, 0);
-    else edges(nout, nsolid_, nnear_);
+    else edges(nout, nsolid_, patch_.ncell);
     note_launches(k);
     launches_ = k;
 }

@@ -25,12 +25,9 @@
 //
 // Measured (GB300, per application and BiCGSTAB iterations per step, against
 // the multigrid V-cycle that served these cases before): channel
-// 128x96x128 FP32 0.12 ms, 1 iteration (0.47 ms, 14); cavity 64^3 FP64
-// 0.37 ms, 1 (0.31 ms, 10); sphere 192x128x128 FP32 0.17 ms, 3.7 (0.53 ms,
-// 3.9); boxes 95x61x47 FP32 0.073 ms, 6.2 (0.25 ms, 4.9).  In FP64 with a
-// body the transforms, bound by the FP64 pipe, cost more than the V-cycles
-// they replace (3.2 GFLOP at 1.05 TFLOP/s against 1.2 ms on the sphere), so
-// the multigrid stays there, and where an axis exceeds the limits below.
+// 128x96x128 FP32 0.09 ms, 1 iteration (0.47 ms, 14); cavity 64^3 FP64
+// 0.17 ms, 1 (0.31 ms, 10); sphere 192x128x128 FP32 0.14 ms, 3.4 (0.53 ms,
+// 3.9); boxes 95x61x47 FP32 0.062 ms, 4.8 (0.25 ms, 4.9).
 #pragma once
 
 #include <vector>
@@ -38,6 +35,14 @@
 #include "krylov.h"
 
 namespace ibm {
+
+// Host tables of the patches near the body (FpPatches).
+struct FpPatchTables {
+    std::vector<int> P, to, start, count, loc;
+    std::vector<int16_t> ref;
+    std::vector<double> w, self, rw;
+    bool near_outer = false;   // a swept cell is the partner of an outer row
+};
 
 // Host description of the pressure rows (interior cells, per axis).
 struct FastPoissonGeom {
@@ -69,27 +74,35 @@ struct FpModes {
 constexpr int FP_LAYERS = 3;     // fluid layers around the ghosts
 constexpr int FP_OVERLAP = 3;    // layers a patch takes beyond its own cells
 constexpr int FP_SWEEPS = 8;     // sweeps of a patch
-constexpr int FP_CUBE = 8;       // side of the cubes the cells are cut by
+// Side of the cubes the cells are cut by.  FP32: 8 (6 or 5: +4 and +13 % on a
+// boxes 95x61x47 step, more overlap); FP64, bound by each SM's two
+// multiply-adds per clock: 5, more and smaller patches (6: +15 % on boxes
+// 64x48x40, 8: +30 %).
+template <typename T>
+constexpr int FP_CUBE = sizeof(T) == 4 ? 8 : 5;
 template <typename T>
 struct FpPatches {
-    const int *start;      // [patch]: its first local cell in the arrays below
-    const int *count;      // [3 patch]: red, black and ghost cells
-    const int *P;          // padded index
-    const int *slot;       // position of the value in `out` (-1: another patch's cell)
-    const int *ref;        // [8][nloc]: local cell of a coupling, ~padded index outside the patch, or FP_NONE
-    const T *w;            // [8][nloc]: weights
-    const T *self;         // weight of the old value (ghost rows; 0 for fluid ones)
-    const T *rw;           // weight of the residual
+    // Per cell: padded index, couplings (padded index, -1: none, and weight,
+    // [8][ncell]), weights of the old value (ghost rows; 0 for fluid ones) and
+    // of the residual.
+    const int *P, *to;
+    const T *w, *self, *rw;
+    int ncell;
+    // Per patch: its first local cell, its red, black and ghost cells; per
+    // local cell: the cell (~cell when it belongs to another patch), and the
+    // local cells it couples to ([8][nloc]; -1: outside the patch or none).
+    const int *start, *count, *loc;
+    const int16_t *ref;
     int nloc;
 };
-constexpr int FP_NONE = 0x7fffffff;
 
 template <typename T>
 class FastPoisson : public Preconditioner<T> {
   public:
     ~FastPoisson() override;
-    // 0: ready; 1: not for this case (the multigrid serves it); -1: error.
-    int setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &A, const FastPoissonGeom &h);
+    // 0: ready; 1: not for this case (the multigrid serves it: an axis is too
+    // long, or the transforms take more than max_ops operations); -1: error.
+    int setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &A, const FastPoissonGeom &h, double max_ops);
     void apply(cudaStream_t s, const T *r, T *z, const int *gate) override;
     bool apply_from64(cudaStream_t s, const double *r, T *z, const int *gate) override;
     bool apply_from_df(cudaStream_t s, const dfloat *r, T *z, const int *gate) override;
@@ -109,15 +122,12 @@ class FastPoisson : public Preconditioner<T> {
     int zero_[3] = {0, 0, 0};      // each axis's constant mode
     T *gscale_ = nullptr;          // per ghost id: 1 / max(1 - w_self, 1e-3)
     FpPatches<T> patch_{};
-    const int *near_cell_ = nullptr;   // cells near the body, and their swept values
-    T *near_val_ = nullptr;
-    int npatch_ = 0, nnear_ = 0, nghost_ = 0, nsolid_ = 0;
+    T *near_val_ = nullptr;        // swept values of the cells near the body
+    int npatch_ = 0, nghost_ = 0, nsolid_ = 0;
     int *solid_ = nullptr;
     bool near_outer_ = false;
     int launches_ = 0;
     std::vector<void *> allocs_;
-    template <typename Put>
-    bool build_patches(const OpT<T> &A, const FastPoissonGeom &h, const std::vector<double> &gw, Put put);
     template <typename S>
     void run(cudaStream_t s, const S *r, T *z, const int *gate);
     template <int TM, typename S>

@@ -1299,6 +1299,66 @@ GMG<T>::~GMG() {
     for (void *p : allocs_) cudaFree(p);
 }
 
+// Finest width of the grid over the axes that can coarsen.
+static double finest_width(const MGGeometry &geom) {
+    double h = 0.0;
+    for (int a = 0; a < 3; a++) {
+        if (geom.f[a].size() < 3) continue;
+        for (size_t i = 0; i + 1 < geom.f[a].size(); i++) {
+            const double w = geom.f[a][i + 1] - geom.f[a][i];
+            if (h == 0.0 || w < h) h = w;
+        }
+    }
+    return h;
+}
+
+// Groups of the level below `faces` along each axis (multigrid.h).
+static void coarse_groups(const std::vector<double> (&faces)[3], const GMGConfig &cfg, int level, double hmin0,
+                          std::vector<int> (&ch)[3]) {
+    long long nfine = 1;
+    for (int a = 0; a < 3; a++) {
+        ch[a] = halve_groups((int)faces[a].size() - 1);
+        nfine *= (long long)faces[a].size() - 1;
+    }
+    if (cfg.coarsening != MG_COARSEN_SPACING) return;
+    // Widest pair on any axis: at that threshold every pair merges.
+    double hmax = 0.0;
+    for (int a = 0; a < 3; a++)
+        for (int i = 0; i + 2 < (int)faces[a].size(); i++) hmax = std::max(hmax, faces[a][i + 2] - faces[a][i]);
+    for (double H = cfg.width_ratio * std::ldexp(hmin0, level + 1);; H *= 1.25) {
+        long long m = 1;
+        for (int a = 0; a < 3; a++) {
+            ch[a] = spacing_groups(faces[a], H);
+            m *= (long long)ch[a].size() - 1;
+        }
+        if (2 * m <= nfine || H >= hmax) break;
+    }
+}
+
+int mg_level_count(const MGGeometry &geom, const GMGConfig &cfg) {
+    std::vector<double> faces[3] = {geom.f[0], geom.f[1], geom.f[2]};
+    const double hmin0 = finest_width(geom);
+    auto cells = [&]() {
+        long long m = 1;
+        for (int a = 0; a < 3; a++) m *= (long long)faces[a].size() - 1;
+        return m;
+    };
+    int levels = 0;
+    while (cells() > 1 && (levels == 0 || cells() > 64)) {
+        std::vector<int> ch[3];
+        coarse_groups(faces, cfg, levels, hmin0, ch);
+        const long long fine = cells();
+        for (int a = 0; a < 3; a++) {
+            std::vector<double> cf;
+            for (int q : ch[a]) cf.push_back(faces[a][q]);
+            faces[a] = cf;
+        }
+        if (cells() == fine) break;   // nothing merges
+        levels++;
+    }
+    return levels + 1;
+}
+
 template <typename T>
 int GMG<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &A, const int *ghost_cell, int nghost,
                   const MGGeometry &geom, const GMGConfig &cfg) {
@@ -1409,36 +1469,13 @@ int GMG<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &A, const
         if (p && bytes) cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, s);
         return p;
     };
-    // Finest width of the grid over the axes that can coarsen.
-    double hmin0 = 0.0;
-    for (int a = 0; a < 3; a++) {
-        if (geom.f[a].size() < 3) continue;
-        for (size_t i = 0; i + 1 < geom.f[a].size(); i++) {
-            const double w = geom.f[a][i + 1] - geom.f[a][i];
-            if (hmin0 == 0.0 || w < hmin0) hmin0 = w;
-        }
-    }
+    const double hmin0 = finest_width(geom);
     for (int level = 0;; level++) {
         const int fn[3] = {nx, ny, nz};
         if (nx < 2 && ny < 2 && nz < 2) break;
         if ((long long)nx * ny * nz <= 64 && !lv64.empty()) break;
         std::vector<int> ch[3];
-        for (int a = 0; a < 3; a++) ch[a] = halve_groups(fn[a]);
-        if (cfg.coarsening == MG_COARSEN_SPACING) {
-            // Widest pair on any axis: at that threshold every pair merges.
-            double hmax = 0.0;
-            for (int a = 0; a < 3; a++)
-                for (int i = 0; i + 2 < (int)faces[a].size(); i++) hmax = std::max(hmax, faces[a][i + 2] - faces[a][i]);
-            const long long nfine = (long long)nx * ny * nz;
-            for (double H = cfg.width_ratio * std::ldexp(hmin0, level + 1);; H *= 1.25) {
-                long long m = 1;
-                for (int a = 0; a < 3; a++) {
-                    ch[a] = spacing_groups(faces[a], H);
-                    m *= (long long)ch[a].size() - 1;
-                }
-                if (2 * m <= nfine || H >= hmax) break;
-            }
-        }
+        coarse_groups(faces, cfg, level, hmin0, ch);
         MGLevel<double> L{};
         L.cx = nx >= 2 && ch[0] == halve_groups(nx);
         L.cy = ny >= 2 && ch[1] == halve_groups(ny);

@@ -106,6 +106,9 @@ struct MGGeometry {
     std::vector<double> f[3];
 };
 
+// Levels (the fine grid included) a multigrid set up so would have.
+int mg_level_count(const MGGeometry &geom, const GMGConfig &cfg);
+
 // The coarsest levels, run inside one thread block (k_mg_tail): each
 // level's place in the block's shared memory, as byte offsets into an
 // image that setup builds once in global memory (conductances, diagonal,

@@ -119,6 +119,7 @@ struct ibm3d_device {
     IRWork irmom, irpres;
     MomSweep msweep;              // momentum by Jacobi sweeps (msweep.use) instead of BiCGSTAB
     GMG<double> *mg = nullptr;
+    int mg_levels = 0;            // of the pressure multigrid, whether built or not
     GMG<float> *mg32 = nullptr;
     // Fast-diagonalisation preconditioners, null where the multigrid serves
     // the case (pres_pc32, pres_pc64).
@@ -312,6 +313,7 @@ void release_device(ibm3d_device *d) {
     if (!d) return;
     delete d->mg;
     d->mg = nullptr;
+    d->mg_levels = 0;
     delete d->mg32;
     d->mg32 = nullptr;
     delete d->fp64;
@@ -847,8 +849,15 @@ bool build_ops(IBMSolver *sv) {
 }
 
 // Tables of the momentum sweeps (momsweep.h), and the fast-diagonalisation
-// preconditioners (fastpoisson.h): in FP32 for every case its axes allow,
-// in FP64 without a body.
+// preconditioners (fastpoisson.h): in FP32 for every case its axes allow; in
+// FP64, where the transforms are bound by the FP64 pipe, always without a
+// body (one iteration instead of 5-18) and with one up to kBodyOps
+// operations per application.  FP64 steps against the multigrid's: boxes
+// 64x48x40 3.6 against 5.0 ms, sphere 96x64x64 4.4 against 7.4, 128x96x96
+// (0.45e9 operations) 9.4 against 14.0, 192x128x128 (1.6e9) 30 against 24.
+// A caller who has the multigrid halve every axis asks for the multigrid.
+constexpr double kBodyOps = 0.7e9;
+
 bool build_sweeps_and_poisson(IBMSolver *sv) {
     ibm3d_device *d = sv->dev;
     const Grid &g = d->g;
@@ -885,9 +894,9 @@ bool build_sweeps_and_poisson(IBMSolver *sv) {
         set_status(sv, IBM3D_ECUDA, "momentum sweep tables failed");
         return false;
     }
-    auto make = [&](auto *&fp, auto &A) {
+    auto make = [&](auto *&fp, auto &A, double max_ops) {
         fp = new std::remove_reference_t<decltype(*fp)>();
-        const int rc = fp->setup(d->s, d->A64, A, h);
+        const int rc = fp->setup(d->s, d->A64, A, h, max_ops);
         if (rc != 0) {
             delete fp;
             fp = nullptr;
@@ -895,7 +904,47 @@ bool build_sweeps_and_poisson(IBMSolver *sv) {
         if (rc < 0) set_status(sv, IBM3D_ECUDA, "preconditioner setup failed");
         return rc >= 0;
     };
-    return make(d->fp32, d->A32) && (body || make(d->fp64, d->A64));
+    return make(d->fp32, d->A32, INFINITY) &&
+           make(d->fp64, d->A64, !body ? INFINITY : d->mg_coarsening == IBM3D_COARSEN_HALVE ? 0.0 : kBodyOps);
+}
+
+MGGeometry mg_geometry(const IBMSolver *sv) {
+    MGGeometry geom;
+    const double *D[3] = {sv->dx, sv->dy, sv->dz};
+    const int Ns[3] = {sv->Nx, sv->Ny, sv->Nz};
+    for (int a = 0; a < 3; a++) {
+        geom.f[a].assign(Ns[a] + 1, 0.0);
+        for (int i = 0; i < Ns[a]; i++) geom.f[a][i + 1] = geom.f[a][i] + D[a][i + 2];
+    }
+    return geom;
+}
+
+GMGConfig mg_config(const ibm3d_device *d) {
+    GMGConfig mc;
+    mc.nu_pre = d->mg_sweeps[0];
+    mc.nu_post = d->mg_sweeps[1];
+    mc.nuc_pre = d->mg_sweeps[2];
+    mc.nuc_post = d->mg_sweeps[3];
+    mc.coarse_sweeps = d->mg_sweeps[4];
+    mc.omega = d->mg_omega;
+    mc.coarsening = d->mg_coarsening == IBM3D_COARSEN_HALVE ? MG_COARSEN_HALVE : MG_COARSEN_SPACING;
+    mc.width_ratio = d->mg_width_ratio;
+    return mc;
+}
+
+// The pressure multigrid in one precision (null, with the status set, on
+// failure), built where it preconditions, or when its kernel is timed.
+template <typename T>
+GMG<T> *build_multigrid(IBMSolver *sv, const OpT<T> &A) {
+    ibm3d_device *d = sv->dev;
+    GMG<T> *mg = new GMG<T>();
+    if (mg->setup(d->s, d->A64, A, d->nghost ? d->gargs.cell : nullptr, d->nghost, mg_geometry(sv), mg_config(d)) != 0) {
+        set_status(sv, IBM3D_ECUDA, "multigrid setup failed");
+        delete mg;
+        return nullptr;
+    }
+    mg->set_prof(&d->prof);
+    return mg;
 }
 
 void swap3(double *a[3], double *b[3]) {
@@ -1831,33 +1880,10 @@ void IBMSolver_assemble(IBMSolver *s) {
     d->kpres_df = dfloat_view(d->kpres);
     d->pp_df = dmalloc<dfloat>(s, g.ncell, "Krylov workspace");
     if (!d->pp_df) return;
-    MGGeometry geom;
-    const double *D[3] = {s->dx, s->dy, s->dz};
-    const int Ns[3] = {s->Nx, s->Ny, s->Nz};
-    for (int a = 0; a < 3; a++) {
-        geom.f[a].assign(Ns[a] + 1, 0.0);
-        for (int i = 0; i < Ns[a]; i++) geom.f[a][i + 1] = geom.f[a][i] + D[a][i + 2];
-    }
-    GMGConfig mc;
-    mc.nu_pre = d->mg_sweeps[0];
-    mc.nu_post = d->mg_sweeps[1];
-    mc.nuc_pre = d->mg_sweeps[2];
-    mc.nuc_post = d->mg_sweeps[3];
-    mc.coarse_sweeps = d->mg_sweeps[4];
-    mc.omega = d->mg_omega;
-    mc.coarsening = d->mg_coarsening == IBM3D_COARSEN_HALVE ? MG_COARSEN_HALVE : MG_COARSEN_SPACING;
-    mc.width_ratio = d->mg_width_ratio;
-    const int *gcell = d->nghost ? d->gargs.cell : nullptr;
-    d->mg = new GMG<double>();
-    d->mg32 = new GMG<float>();
-    if (d->mg->setup(d->s, d->A64, d->A64, gcell, d->nghost, geom, mc) != 0 ||
-        d->mg32->setup(d->s, d->A64, d->A32, gcell, d->nghost, geom, mc) != 0) {
-        set_status(s, IBM3D_ECUDA, "multigrid setup failed");
-        return;
-    }
-    d->mg->set_prof(&d->prof);
-    d->mg32->set_prof(&d->prof);
     if (!build_sweeps_and_poisson(s)) return;
+    d->mg_levels = mg_level_count(mg_geometry(s), mg_config(d));
+    if (!d->fp64 && !(d->mg = build_multigrid<double>(s, d->A64))) return;
+    if (!d->fp32 && !(d->mg32 = build_multigrid<float>(s, d->A32))) return;
     if (d->pc64.allocate(g.ncell, pres_pc32(d)) != 0) {
         set_status(s, IBM3D_ECUDA, "preconditioner workspace allocation failed");
         return;
@@ -2488,7 +2514,7 @@ void IBMSolver_set_coarsening(IBMSolver *s, int mode, double width_ratio) {
         set_status(s, IBM3D_EARG, "IBMSolver_set_coarsening: width ratio %g outside [1, 64]", width_ratio);
         return;
     }
-    if (s->dev->mg) {
+    if (s->dev->mg_levels > 0) {
         set_status(s, IBM3D_EARG, "IBMSolver_set_coarsening: call it before IBMSolver_assemble");
         return;
     }
@@ -2632,7 +2658,7 @@ void IBMSolver_get_stats(const IBMSolver *s, IBMSolverStats *out) {
     out->iters_p = d->rep_p.iters[0];
     out->res_p = d->rep_p.relres[0];
     out->max_div = d->max_div;
-    out->mg_levels = d->mg ? d->mg->nlevels() : 0;
+    out->mg_levels = d->mg_levels;
     out->outer_u = d->rep_mom.outer;
     out->outer_p = d->rep_p.outer;
     out->cpt_fallback = d->cpt_fallback;
@@ -2739,6 +2765,8 @@ double IBMSolver_time_kernel(IBMSolver *s, int which, int reps, double *bytes) {
     std::function<void()> launch;
     switch (which) {
     case IBM3D_K_MG_COLOR:
+        if (mixed && !d->mg32 && !(d->mg32 = build_multigrid<float>(s, d->A32))) return -1;
+        if (!mixed && !d->mg && !(d->mg = build_multigrid<double>(s, d->A64))) return -1;
         // Scratch vectors of the pressure solve of the current precision.
         launch = [&]() {
             double bb;
