@@ -678,75 +678,89 @@ k_fp_edges(const OpT<T> c, const S *__restrict__ r, T *z, const int *__restrict_
 
 // Sweeps over the cells near the body: an overlapping Schwarz step.  The
 // cells (fluid ones within FP_LAYERS of a ghost, and the ghosts) are cut
-// into patches of neighbouring cells; a block takes one patch with
-// FP_OVERLAP more layers of them, loads values and rows into shared memory
-// (couplings to cells outside go into the right-hand side), runs its sweeps
-// there (red, black, then the ghost rows Jacobi-style) and returns the
-// values of its own cells, which k_fp_edges writes to z.  A pass is one
-// block barrier, so the sweeps cost less than loading the patch.  (Sweeps
-// over all the cells at once with a barrier per pass, across the blocks of
-// a cluster or as launches, spend 3-4 us per pass on the L2 round trip.)
-// Bound by latency: one load of the rows, FP_SWEEPS x 4 block barriers.
-constexpr int FP_PT = 256;       // threads of a patch block
-constexpr int FP_PMAX = 1536;    // cells of a patch, overlap included
+// into patches by the cubes of the grid; a block takes one patch with the
+// cells FP_OVERLAP beyond it, keeps their rows in registers (at most FP_PU
+// cells per thread) and their values in shared memory (couplings to cells
+// outside go into the right-hand side), runs its sweeps there (red, black,
+// then the ghost rows Jacobi-style) and returns the values of its own cells,
+// which k_fp_edges writes to z.  (Sweeps over all the cells at once with a
+// barrier per pass, across the blocks of a cluster or as launches, spend 3-4
+// us per pass on the L2 round trip; rows read again from L1 in every pass
+// made an application of boxes 95x61x47 62 us, in registers PATCHN.)  Bound
+// by latency: one load of the rows, FP_SWEEPS x 4 block barriers.
+constexpr int FP_PT = 512;               // threads of a patch block
+constexpr int FP_PU = 3;                 // cells per thread
+constexpr int FP_PMAX = FP_PT * FP_PU;   // cells of a patch, overlap included
 
 template <typename T, typename S>
 __global__ void __launch_bounds__(FP_PT)
 k_fp_patch(const FpPatches<T> p, const S *__restrict__ r, const T *__restrict__ z, T *__restrict__ out,
            const int sweeps, const int *gate) {
     FP_GATE(gate);
-    __shared__ T v[FP_PMAX], f[FP_PMAX];
-    const int b = blockIdx.x, s0 = p.start[b], nr = p.count[3 * b], nb = p.count[3 * b + 1], ng = p.count[3 * b + 2];
-    const int n = nr + nb + ng;
-    auto cell = [&](int q) {
-        const int c = p.loc[s0 + q];
-        return c < 0 ? ~c : c;
-    };
-    for (int q = threadIdx.x; q < n; q += FP_PT) {
-        const int c = cell(q), P = p.P[c];
+    __shared__ T v[FP_PMAX];
+    const int b = blockIdx.x, s0 = p.start[b], nr = p.count[3 * b], nf = nr + p.count[3 * b + 1];
+    const int n = nf + p.count[3 * b + 2];
+    T w[FP_PU][8], f[FP_PU], self[FP_PU];
+    int m[FP_PU][8], own[FP_PU];
+#pragma unroll
+    for (int u = 0; u < FP_PU; u++) {
+        const int q = u * FP_PT + threadIdx.x;
+        own[u] = -1;
+        if (q >= n) continue;
+        own[u] = p.loc[s0 + q];
+        const int c = own[u] < 0 ? ~own[u] : own[u], P = p.P[c];
         v[q] = z[P];
-        T t = p.rw[c] * fp_value<T, S>(r[P]);
+        self[u] = p.self[s0 + q];
+        f[u] = p.rw[s0 + q] * fp_value<T, S>(r[P]);
 #pragma unroll
         for (int e = 0; e < 8; e++) {
-            const int Q = p.to[e * p.ncell + c];
-            if (Q >= 0 && p.ref[(size_t)e * p.nloc + s0 + q] < 0) t += p.w[e * p.ncell + c] * z[Q];
+            w[u][e] = p.w[(size_t)e * p.nloc + s0 + q];
+            m[u][e] = p.ref[(size_t)e * p.nloc + s0 + q];
+            if (m[u][e] < 0) {   // outside the patch, or no coupling
+                const int Q = p.to[e * p.ncell + c];
+                if (Q >= 0) f[u] += w[u][e] * z[Q];
+                w[u][e] = 0;
+                m[u][e] = q;
+            }
         }
-        f[q] = t;
     }
     __syncthreads();
-    // Rows of this thread's cells: couplings inside the patch.
-    auto row = [&](int q, int ne) {
-        const int c = cell(q);
-        T t = f[q];
-        for (int e = 0; e < ne; e++) {
-            const int m = p.ref[(size_t)e * p.nloc + s0 + q];
-            if (m >= 0) t += p.w[e * p.ncell + c] * v[m];
+    // The rows of this thread's cells [lo, hi): a pass over one colour.
+    auto pass = [&](int lo, int hi) {
+#pragma unroll
+        for (int u = 0; u < FP_PU; u++) {
+            const int q = u * FP_PT + threadIdx.x;
+            if (q < lo || q >= hi) continue;
+            T t = f[u];
+#pragma unroll
+            for (int e = 0; e < 6; e++) t += w[u][e] * v[m[u][e]];
+            v[q] = t;
         }
-        return t;
+        __syncthreads();
     };
     for (int s = 0; s < sweeps; s++) {
-        for (int q = threadIdx.x; q < nr; q += FP_PT) v[q] = row(q, 6);
-        __syncthreads();
-        for (int q = nr + threadIdx.x; q < nr + nb; q += FP_PT) v[q] = row(q, 6);
-        __syncthreads();
-        T g[(FP_PMAX + FP_PT - 1) / FP_PT];
+        pass(0, nr);
+        pass(nr, nf);
+        T g[FP_PU];
 #pragma unroll
-        for (int u = 0; u < (FP_PMAX + FP_PT - 1) / FP_PT; u++) {
-            const int q = nr + nb + u * FP_PT + threadIdx.x;
-            if (q < n) g[u] = row(q, 8) + p.self[cell(q)] * v[q];
+        for (int u = 0; u < FP_PU; u++) {
+            const int q = u * FP_PT + threadIdx.x;
+            if (q < nf || q >= n) continue;
+            g[u] = f[u] + self[u] * v[q];
+#pragma unroll
+            for (int e = 0; e < 8; e++) g[u] += w[u][e] * v[m[u][e]];
         }
         __syncthreads();
 #pragma unroll
-        for (int u = 0; u < (FP_PMAX + FP_PT - 1) / FP_PT; u++) {
-            const int q = nr + nb + u * FP_PT + threadIdx.x;
-            if (q < n) v[q] = g[u];
+        for (int u = 0; u < FP_PU; u++) {
+            const int q = u * FP_PT + threadIdx.x;
+            if (q >= nf && q < n) v[q] = g[u];
         }
         __syncthreads();
     }
-    for (int q = threadIdx.x; q < n; q += FP_PT) {
-        const int c = p.loc[s0 + q];
-        if (c >= 0) out[c] = v[q];
-    }
+#pragma unroll
+    for (int u = 0; u < FP_PU; u++)
+        if (own[u] >= 0) out[own[u]] = v[u * FP_PT + threadIdx.x];
 }
 
 // ----------------------------------------------------------------- set-up --
@@ -863,8 +877,9 @@ FastPoisson<T>::~FastPoisson() {
 
 // The cells near the body, their rows and the patches (k_fp_patch), cut by
 // cubes of side `cube`; false when a patch cannot be made small enough.
+template <typename T>
 static bool build_patches(const OpT<double> &A, const FastPoissonGeom &h, const std::vector<double> &gw, int cube,
-                          FpPatchTables &t_) {
+                          FpPatchTables<T> &t_) {
     const Grid &g = A.g;
     const int n[3] = {g.nx, g.ny, g.nz};
     const long long st[3] = {g.sx, g.sy, 1};
@@ -922,9 +937,7 @@ static bool build_patches(const OpT<double> &A, const FastPoissonGeom &h, const 
     // Rows: couplings (padded index, weight), weight of the old value and of
     // the residual.  Ghost rows are relaxed as the multigrid relaxes them.
     t_.to.assign((size_t)nc * 8, -1);
-    t_.w.assign((size_t)nc * 8, 0.0);
-    t_.self.assign(nc, 0.0);
-    t_.rw.assign(nc, 1.0);
+    std::vector<T> w((size_t)nc * 8, (T)0), self(nc, (T)0), rw(nc, (T)1);   // w: [cell][8]
     std::vector<int> &to = t_.to;   // [8][nc]
     for (int q = 0; q < nc; q++) {
         const int *x = &ijk[3 * (size_t)q];
@@ -938,18 +951,18 @@ static bool build_patches(const OpT<double> &A, const FastPoissonGeom &h, const 
             const double dg = 1.0 - h.gwself[q], dv = 1.0 / std::max({dg, 2.0 * off, 1e-3});
             for (int e = 0; e < 8; e++) {
                 to[(size_t)e * nc + q] = h.gidx[8 * (size_t)q + e];
-                t_.w[(size_t)e * nc + q] = dv * gw[8 * (size_t)q + e];
+                w[8 * (size_t)q + e] = (T)(dv * gw[8 * (size_t)q + e]);
             }
-            t_.self[q] = 1.0 - dg * dv;
-            t_.rw[q] = dv;
+            self[q] = (T)(1.0 - dg * dv);
+            rw[q] = (T)dv;
         } else {
             double sum = 0;
             for (int a = 0; a < 3; a++) sum += h.km[a][x[a]] + h.kp[a][x[a]];
             for (int a = 0; a < 3; a++) {
                 to[(size_t)(2 * a) * nc + q] = (int)(cells[q] - st[a]);
                 to[(size_t)(2 * a + 1) * nc + q] = (int)(cells[q] + st[a]);
-                t_.w[(size_t)(2 * a) * nc + q] = h.km[a][x[a]] / sum;
-                t_.w[(size_t)(2 * a + 1) * nc + q] = h.kp[a][x[a]] / sum;
+                w[8 * (size_t)q + 2 * a] = (T)(h.km[a][x[a]] / sum);
+                w[8 * (size_t)q + 2 * a + 1] = (T)(h.kp[a][x[a]] / sum);
             }
         }
     }
@@ -960,97 +973,96 @@ static bool build_patches(const OpT<double> &A, const FastPoissonGeom &h, const 
             const int Q = to[(size_t)e * nc + q];
             nbr[8 * (size_t)q + e] = Q >= 0 ? id[Q] : -1;
         }
-    // Patches: cubes of the grid, halved until each fits with its overlap.
-    std::vector<std::vector<int>> todo;
+    // Patches: the occupied cubes of the grid, halved until each fits with
+    // the cells within FP_OVERLAP of it (along every axis).
+    struct Box {
+        int lo[3], hi[3];
+    };
+    std::vector<Box> todo;
     {
         const int cy = (n[1] + cube - 1) / cube, cz = (n[2] + cube - 1) / cube;
-        std::vector<int> at((size_t)((n[0] + cube - 1) / cube) * cy * cz, -1);
+        std::vector<uint8_t> seen((size_t)((n[0] + cube - 1) / cube) * cy * cz, 0);
         for (int q = 0; q < nc; q++) {
-            const int *x = &ijk[3 * (size_t)q];
-            int &b = at[((size_t)(x[0] / cube) * cy + x[1] / cube) * cz + x[2] / cube];
-            if (b < 0) {
-                b = (int)todo.size();
-                todo.emplace_back();
+            const int *x = &ijk[3 * (size_t)q], b[3] = {x[0] / cube, x[1] / cube, x[2] / cube};
+            uint8_t &s = seen[((size_t)b[0] * cy + b[1]) * cz + b[2]];
+            if (s) continue;
+            s = 1;
+            Box box;
+            for (int a = 0; a < 3; a++) {
+                box.lo[a] = b[a] * cube;
+                box.hi[a] = std::min(box.lo[a] + cube, n[a]);
             }
-            todo[b].push_back(q);
+            todo.push_back(box);
         }
     }
-    std::vector<int> mark(nc, -1), all, list[3], pos(nc);
+    std::vector<int> mark(nc, -1), list[3], pos(nc);
     std::vector<int16_t> refs;   // [local][8] of every patch
+    std::vector<T> lw;
     for (size_t t = 0; t < todo.size(); t++) {
-        const std::vector<int> own = todo[t];
+        const Box box = todo[t];
         const int stamp = (int)t;
-        all = own;
-        for (int q : own) mark[q] = stamp;
-        size_t from = 0;
-        for (int o = 0; o < FP_OVERLAP; o++) {
-            const size_t upto = all.size();
-            for (size_t l = from; l < upto; l++) {
-                const int q = all[l];
-                auto grow = [&](int m) {
-                    if (m < 0 || mark[m] == stamp) return;
-                    mark[m] = stamp;
-                    all.push_back(m);
-                };
-                for (int e = 0; e < 8; e++) grow(nbr[8 * (size_t)q + e]);
-                for (int a = 0; q < ng && a < 3; a++) {
-                    grow(id[cells[q] - st[a]]);
-                    grow(id[cells[q] + st[a]]);
-                }
-            }
-            from = upto;
+        int lo[3], hi[3], own = 0;
+        for (int a = 0; a < 3; a++) {
+            lo[a] = std::max(0, box.lo[a] - FP_OVERLAP<T>);
+            hi[a] = std::min(n[a], box.hi[a] + FP_OVERLAP<T>);
         }
-        if ((int)all.size() > FP_PMAX) {   // split the cube along its longest side
-            if (own.size() < 2) return false;
-            int best = 0, lo = 0, hi = -1;
-            for (int a = 0; a < 3; a++) {
-                int l = ijk[3 * (size_t)own[0] + a], u = l;
-                for (int q : own) {
-                    l = std::min(l, ijk[3 * (size_t)q + a]);
-                    u = std::max(u, ijk[3 * (size_t)q + a]);
-                }
-                if (u - l > hi - lo) {
-                    best = a;
-                    lo = l;
-                    hi = u;
+        // Local order: red, black, ghost; by padded index within each.
+        for (auto &l : list) l.clear();
+        for (i = lo[0]; i < hi[0]; i++)
+            for (j = lo[1]; j < hi[1]; j++) {
+                const bool in = i >= box.lo[0] && i < box.hi[0] && j >= box.lo[1] && j < box.hi[1];
+                const long long P0 = cidx(g, i, j, 0);
+                for (k = lo[2]; k < hi[2]; k++) {
+                    const int q = id[P0 + k];
+                    if (q < 0) continue;
+                    const bool mine = in && k >= box.lo[2] && k < box.hi[2];
+                    own += mine;
+                    list[q < ng ? 2 : (i + j + k) & 1].push_back(mine ? q : ~q);
+                    mark[q] = stamp;
                 }
             }
-            const int mid = (lo + hi + 1) / 2;
-            std::vector<int> a0, a1;
-            for (int q : own) (ijk[3 * (size_t)q + best] < mid ? a0 : a1).push_back(q);
-            todo.push_back(a0);
-            todo.push_back(a1);
+        if (own == 0) continue;   // half of a split cube
+        const int total = (int)(list[0].size() + list[1].size() + list[2].size());
+        if (total > FP_PMAX) {
+            int a = 0;
+            for (int b = 1; b < 3; b++)
+                if (box.hi[b] - box.lo[b] > box.hi[a] - box.lo[a]) a = b;
+            if (box.hi[a] - box.lo[a] < 2) return false;
+            Box b0 = box, b1 = box;
+            b0.hi[a] = b1.lo[a] = (box.lo[a] + box.hi[a]) / 2;
+            todo.push_back(b0);
+            todo.push_back(b1);
             continue;
         }
-        // Local order: red, black, ghost; the patch's own cells are the
-        // first own.size() of `all`.
-        for (auto &l : list) l.clear();
-        for (size_t l = 0; l < all.size(); l++) {
-            const int q = all[l], *x = &ijk[3 * (size_t)q];
-            list[q < ng ? 2 : (x[0] + x[1] + x[2]) & 1].push_back(l < own.size() ? q : ~q);
-        }
         t_.start.push_back((int)t_.loc.size());
-        int k_ = 0;
+        int at = 0;
         for (const auto &l : list) {
             t_.count.push_back((int)l.size());
             for (int u : l) {
                 t_.loc.push_back(u);
-                pos[u < 0 ? ~u : u] = k_++;
+                pos[u < 0 ? ~u : u] = at++;
             }
         }
         for (const auto &l : list)
             for (int u : l) {
                 const int q = u < 0 ? ~u : u;
+                t_.self.push_back(self[q]);
+                t_.rw.push_back(rw[q]);
                 for (int e = 0; e < 8; e++) {
                     const int m = nbr[8 * (size_t)q + e];
                     refs.push_back(m >= 0 && mark[m] == stamp ? (int16_t)pos[m] : (int16_t)-1);
+                    lw.push_back(w[8 * (size_t)q + e]);
                 }
             }
     }
     const size_t nloc = t_.loc.size();
     t_.ref.resize(8 * nloc);
+    t_.w.resize(8 * nloc);
     for (size_t l = 0; l < nloc; l++)
-        for (int e = 0; e < 8; e++) t_.ref[e * nloc + l] = refs[8 * l + e];
+        for (int e = 0; e < 8; e++) {
+            t_.ref[e * nloc + l] = refs[8 * l + e];
+            t_.w[e * nloc + l] = lw[8 * l + e];
+        }
     t_.P = cells;
     return true;
 }
@@ -1239,18 +1251,15 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
         std::vector<T> sc(nghost_);
         for (int q = 0; q < nghost_; q++) sc[q] = (T)(1.0 / std::max(1.0 - h.gwself[q], 1e-3));
         gscale_ = (T *)put(sc.data(), sizeof(T) * nghost_);
-        FpPatchTables t;
+        FpPatchTables<T> t;
         if (!build_patches(A64, h, gw, FP_CUBE<T>, t)) return 1;
         auto ints = [&](const std::vector<int> &v) { return (const int *)put(v.data(), sizeof(int) * v.size()); };
-        auto reals = [&](const std::vector<double> &v) {
-            const std::vector<T> c(v.begin(), v.end());
-            return (const T *)put(c.data(), sizeof(T) * c.size());
-        };
+        auto reals = [&](const std::vector<T> &v) { return (const T *)put(v.data(), sizeof(T) * v.size()); };
         npatch_ = (int)t.start.size();
         near_outer_ = t.near_outer;
-        patch_ = FpPatches<T>{ints(t.P), ints(t.to), reals(t.w), reals(t.self), reals(t.rw), (int)t.P.size(),
-                              ints(t.start), ints(t.count), ints(t.loc),
-                              (const int16_t *)put(t.ref.data(), sizeof(int16_t) * t.ref.size()), (int)t.loc.size()};
+        patch_ = FpPatches<T>{ints(t.P), ints(t.to), (int)t.P.size(), ints(t.start), ints(t.count), ints(t.loc),
+                              (const int16_t *)put(t.ref.data(), sizeof(int16_t) * t.ref.size()), reals(t.w),
+                              reals(t.self), reals(t.rw), (int)t.loc.size()};
         near_val_ = (T *)put(nullptr, sizeof(T) * t.P.size());
     }
     if (!ok) return -1;

@@ -37,10 +37,11 @@
 namespace ibm {
 
 // Host tables of the patches near the body (FpPatches).
+template <typename T>
 struct FpPatchTables {
     std::vector<int> P, to, start, count, loc;
     std::vector<int16_t> ref;
-    std::vector<double> w, self, rw;
+    std::vector<T> w, self, rw;
     bool near_outer = false;   // a swept cell is the partner of an outer row
 };
 
@@ -72,27 +73,27 @@ struct FpModes {
 // per 3 sweeps: 8 is the fastest step everywhere.  Thinner or thicker layers
 // and overlaps are within 3 %.
 constexpr int FP_LAYERS = 3;     // fluid layers around the ghosts
-constexpr int FP_OVERLAP = 3;    // layers a patch takes beyond its own cells
 constexpr int FP_SWEEPS = 8;     // sweeps of a patch
-// Side of the cubes the cells are cut by.  FP32: 8 (6 or 5: +4 and +13 % on a
-// boxes 95x61x47 step, more overlap); FP64, bound by each SM's two
-// multiply-adds per clock: 5, more and smaller patches (6: +15 % on boxes
-// 64x48x40, 8: +30 %).
+// Side of the cubes the cells are cut by, and the cells a patch takes beyond
+// them.  FP64, bound by each SM's two multiply-adds per clock: more and
+// smaller patches (boxes 64x48x40: 3.38 ms per step, with FP32's sizes 3.75);
+// FP32 steps are within 3 % for sides of 6 and 8 and overlaps of 2 to 4.
 template <typename T>
 constexpr int FP_CUBE = sizeof(T) == 4 ? 8 : 5;
 template <typename T>
+constexpr int FP_OVERLAP = sizeof(T) == 4 ? 3 : 2;
+template <typename T>
 struct FpPatches {
-    // Per cell: padded index, couplings (padded index, -1: none, and weight,
-    // [8][ncell]), weights of the old value (ghost rows; 0 for fluid ones) and
-    // of the residual.
-    const int *P, *to;
-    const T *w, *self, *rw;
+    const int *P, *to;     // per cell: padded index, couplings ([8][ncell] padded indices, -1: none)
     int ncell;
-    // Per patch: its first local cell, its red, black and ghost cells; per
-    // local cell: the cell (~cell when it belongs to another patch), and the
-    // local cells it couples to ([8][nloc]; -1: outside the patch or none).
-    const int *start, *count, *loc;
+    const int *start, *count;   // per patch: its first local cell; its red, black and ghost cells
+    // Per local cell: the cell (~cell when another patch owns it), the local
+    // cells it couples to ([8][nloc]; -1: outside the patch or none) and the
+    // weights ([8][nloc]), the weights of the old value (ghost rows; 0 for
+    // fluid ones) and of the residual.
+    const int *loc;
     const int16_t *ref;
+    const T *w, *self, *rw;
     int nloc;
 };
 
