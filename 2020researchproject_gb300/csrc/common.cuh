@@ -456,8 +456,8 @@ __device__ inline void block_max(double (&v)[NV], double *smem) {
 // [NS, NV) maxed (all >= 0).  The warp stage runs in the accumulator type
 // A (an FP32 kernel keeps its adds off the FP64 pipe); one value per warp
 // is widened to double for the stage across warps.  Fixed shape, so the
-// result is bitwise reproducible.  Valid in warp 0; smem holds 32 * NV
-// doubles.
+// result is bitwise reproducible.  Valid in warp 0; smem holds 8 * NV
+// doubles, at most 8 warps a block.
 template <int NV, int NS, typename A>
 __device__ inline void block_reduce(const A (&v)[NV], double (&out)[NV], double *smem) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -478,7 +478,7 @@ __device__ inline void block_reduce(const A (&v)[NV], double (&out)[NV], double 
         for (int q = 0; q < NV; q++) {
             double x = lane < nw ? smem[lane * NV + q] : 0.0;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
+            for (int o = 4; o > 0; o >>= 1) {
                 const double y = __shfl_down_sync(0xffffffffu, x, o);
                 x = q < NS ? x + y : nanmax(x, y);
             }
@@ -507,50 +507,35 @@ __device__ inline bool publish_partials(const double (&v)[NV], double *partials,
 
 // Reduces every block's partials inside the last block: entries [0, NS)
 // are summed, entries [NS, NV) maxed (all maxed quantities are >= 0, so 0
-// is their identity).  Thread t folds blocks t, t + blockDim, ... in that
-// order and a fixed-shape tree combines the threads, so the result does
-// not depend on block scheduling (bitwise reproducible).  Valid in thread
-// 0; smem holds 32 * NV doubles and must be free on entry.
+// is their identity).  Warp q takes entry q (q + the warps, ...): lane t
+// folds blocks t, t + 32, ... in that order and a fixed-shape tree combines
+// the lanes, so the result does not depend on block scheduling (bitwise
+// reproducible).  One warp per entry, not all of them for each: a warp's
+// FP64 addition takes the SM's FP64 unit 16 cycles, and 608 blocks' three
+// entries take 72 of them instead of 190.  Valid in thread 0; smem holds NV
+// doubles and must be free on entry.
 template <int NV, int NS>
 __device__ inline void reduce_partials(const double *partials, int nblocks, double (&out)[NV], double *smem) {
-    double v[NV];
-#pragma unroll
-    for (int q = 0; q < NV; q++) v[q] = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-#pragma unroll
-        for (int q = 0; q < NV; q++) {
-            const double x = __ldcg(partials + (size_t)b * NV + q);
-            v[q] = q < NS ? v[q] + x : nanmax(v[q], x);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int q = warp; q < NV; q += nw) {
+        double x = 0.0;
+        const double *p = partials + q;
+#pragma unroll 8
+        for (int b = lane; b < nblocks; b += 32) {
+            const double y = __ldcg(p + (size_t)b * NV);
+            x = q < NS ? x + y : nanmax(x, y);
         }
-    }
-#pragma unroll
-    for (int q = 0; q < NV; q++) {
-        double x = v[q];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const double y = __shfl_down_sync(0xffffffffu, x, o);
             x = q < NS ? x + y : nanmax(x, y);
         }
-        v[q] = x;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; q++) smem[warp * NV + q] = v[q];
+        if (lane == 0) smem[q] = x;
     }
     __syncthreads();
-    if (warp == 0) {
-        const int nw = blockDim.x >> 5;
+    if (threadIdx.x == 0) {
 #pragma unroll
-        for (int q = 0; q < NV; q++) {
-            double x = lane < nw ? smem[lane * NV + q] : 0.0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double y = __shfl_down_sync(0xffffffffu, x, o);
-                x = q < NS ? x + y : nanmax(x, y);
-            }
-            out[q] = x;
-        }
+        for (int q = 0; q < NV; q++) out[q] = smem[q];
     }
 }
 

@@ -36,9 +36,9 @@ template <> struct AccT<double> { using type = double; };
 template <> struct AccT<float> { using type = float; };
 template <> struct AccT<dfloat> { using type = dfloat; };
 
-// 16-byte packs for the streaming vector kernels: with n % 4 == 0 every
-// vector (and every component of a 3-component vector) starts on a 16-byte
-// boundary, and a thread moves PW elements per load.
+// 16-byte packs for the streaming vector kernels: a thread moves PW elements
+// per load.  Every vector starts on a 16-byte boundary, and with n % 4 == 0
+// so does every component of a 3-component vector.
 template <typename T>
 struct alignas(16) Pack {
     T v[16 / sizeof(T)];
@@ -62,6 +62,28 @@ struct alignas(sizeof(E) * N) PackN {
 template <typename T, typename E>
 __device__ __forceinline__ PackN<E, PW<T>> ldpn(const E *p, long long q) {
     return reinterpret_cast<const PackN<E, PW<T>> *>(p)[q];
+}
+
+// Runs use(ld(q), q) for every pack q < np of a vector, two packs of a
+// thread at a time with both packs' loads issued before either is used
+// (bound by their bytes and by the loads in flight: k_bicg_xr on sphere
+// 192x128x128, double-float, 45 -> 38 us, cold).
+template <typename Ld, typename Use>
+__device__ __forceinline__ void stream_packs(const long long np, Ld ld, Use use) {
+    const long long st = (long long)gridDim.x * blockDim.x;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < np; q += 2 * st) {
+        const bool two = q + st < np;
+        const auto a = ld(q);
+        const auto b = ld(two ? q + st : q);
+        use(a, q);
+        if (two) use(b, q + st);
+    }
+}
+// The entries of a vector past its last whole pack: f(P).
+template <typename T, typename F>
+__device__ __forceinline__ void stream_rest(const long long n, F f) {
+    const long long P = n / PW<T> * PW<T> + threadIdx.x;
+    if (blockIdx.x == gridDim.x - 1 && P < n) f(P);
 }
 
 // Weighted |r| for the divergence criterion (FP32 is ample for a stopping
@@ -167,7 +189,7 @@ k_bicg_init(const long long n, const B *__restrict__ b, T *x, T *r, KScal *sc, d
 
 // ------------------------------------------------- p = r + beta (p - w v) --
 template <typename T, int NC, bool VEC>
-__global__ void __launch_bounds__(KTHREADS)
+__global__ void __launch_bounds__(KTHREADS, NC == 1 ? 4 : 1)
 k_bicg_p(const long long n, const T *__restrict__ r, T *__restrict__ p, const T *__restrict__ v, T *__restrict__ r0,
          const KScal *sc) {
     pdl_enter();
@@ -186,13 +208,18 @@ k_bicg_p(const long long n, const T *__restrict__ r, T *__restrict__ p, const T 
         }
         if (VEC) {
             const long long np = n / PW<T>, op = o / PW<T>;
-            GRID_STRIDE(q, np) {
-                const Pack<T> rr = ldp(r, op + q), vv = ldp(v, op + q);
-                Pack<T> pp = ldp(p, op + q);
+            struct In {
+                Pack<T> r, v, p;
+            };
+            stream_packs(
+                np, [&](long long q) { return In{ldp(r, op + q), ldp(v, op + q), ldp(p, op + q)}; },
+                [&](const In &d, long long q) {
+                    Pack<T> pp;
 #pragma unroll
-                for (int l = 0; l < PW<T>; l++) pp.v[l] = p_update(rr.v[l], beta, pp.v[l], om, vv.v[l]);
-                stp(p, op + q, pp);
-            }
+                    for (int l = 0; l < PW<T>; l++) pp.v[l] = p_update(d.r.v[l], beta, d.p.v[l], om, d.v.v[l]);
+                    stp(p, op + q, pp);
+                });
+            if (NC == 1) stream_rest<T>(n, [&](long long P) { p[P] = p_update(r[P], beta, p[P], om, v[P]); });
         } else {
             GRID_STRIDE(P, n) { p[o + P] = p_update(r[o + P], beta, p[o + P], om, v[o + P]); }
         }
@@ -225,6 +252,77 @@ __device__ __forceinline__ void sweep_rows(const OpT<T> &A, const bool (&run)[NC
 #pragma unroll
         for (int c = 0; c < NC; c++)
             if (run[c]) fo(c, P);
+    }
+}
+
+// sweep_rows for the pressure rows (one component): calls fi(P, y, e) with
+// y = (A x)_P and e = ld(P), the caller's own values of the cell, for every
+// interior row of this thread's column, and fo(P) for its outer row.  FP32
+// and double-float kernels load a plane ahead of the one they compute, with
+// ld's loads (sphere 192x128x128, double-float: k_bicg_spmv_v 54 -> 49 us,
+// k_bicg_spmv_t 59 -> 54, init_guess 86 -> 79); FP64 ones are bound by the FP64 pipe.
+template <typename T, typename X, typename Ld, typename FI, typename FO>
+__device__ __forceinline__ void sweep_pres(const OpT<T> &A, const X *__restrict__ x, Ld ld, FI fi, FO fo) {
+    int i0, i1, j, k;
+    if (sweep_column(A.sw, A.g, i0, i1, j, k)) {
+        if (j >= A.g.ny || k >= A.g.nz) return;
+        const Column<T> q = column(A, j, k);
+        const long long sx = A.g.sx, sy = A.g.sy;
+        long long P = cidx(A.g, i0, j, k);
+        struct Plane {
+            X e, s, n, d, u;
+            T dinv;
+            decltype(ld(0LL)) own;
+            uint8_t fl;
+        };
+        auto fetch = [&](long long Q) {
+            Plane L;
+            L.fl = A.flag[Q];
+            L.e = x[Q + sx];
+            L.s = x[Q - sy];
+            L.n = x[Q + sy];
+            L.d = x[Q - 1];
+            L.u = x[Q + 1];
+            L.dinv = A.dinv[Q];
+            L.own = ld(Q);
+            return L;
+        };
+        constexpr bool AHEAD = !std::is_same<T, double>::value;
+        X xw = x[P - sx], xc = x[P];
+        Plane cur;
+        if (AHEAD) cur = fetch(P);
+        for (int i = i0; i < i1; i++, P += sx) {
+            Plane nxt;
+            if (AHEAD) {
+                if (i + 1 < i1) nxt = fetch(P + sx);
+            } else {
+                cur = fetch(P);
+            }
+            const int I = i + 2;
+            const T c = T(xc);
+            const T nb = sum6(A.km[0][I], T(xw), A.kp[0][I], T(cur.e), q.kmy, T(cur.s), q.kpy, T(cur.n), q.kmz, T(cur.d),
+                              q.kpz, T(cur.u));
+            T y = sub_mul(c, cur.dinv, nb);
+            const bool pinned = A.p_singular && P == A.pinned;
+            if (cur.fl != FLUID || pinned) y = c;
+            if (cur.fl == GHOST && !pinned) {
+                const int g = A.gid[P];
+                T sum = 0;
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const int m = A.gidx[8 * g + e];
+                    if (m >= 0) sum += A.gw[8 * g + e] * T(x[m]);
+                }
+                y = ((T)1 - A.gwself[g]) * c - sum;
+            }
+            fi(P, y, cur.own);
+            xw = xc;
+            xc = cur.e;
+            if (AHEAD) cur = nxt;
+        }
+    } else {
+        const int t = sweep_outer(A.sw);
+        if (t < A.sw.nout) fo((long long)A.sw.outer[t]);
     }
 }
 
@@ -262,16 +360,26 @@ k_bicg_init_guess(const OpT<T> A, const int op, const long long n, const B *__re
         mac(a[NC + c], y, y);
         if (divtol > 0) dmax = fmaxf(dmax, divw(A, P, y));
     };
-    sweep_rows<T, NC>(
-        A, run,
-        [&](int c, long long P, int i, const Column<T> &q) {
-            const T bv = (T)b[c * n + P];
-            put(c, P, bv, bv - interior_row(A, op, x + c * n, P, i, q));
-        },
-        [&](int c, long long P) {
-            const T bv = (T)b[c * n + P];
-            put(c, P, bv, bv - op_row(A, op, c, x + c * n, P));
-        });
+    if constexpr (NC == 1) {
+        sweep_pres(
+            A, x, [&](long long P) { return b[P]; },
+            [&](long long P, T y, B bv) { put(0, P, (T)bv, (T)bv - y); },
+            [&](long long P) {
+                const T bv = (T)b[P];
+                put(0, P, bv, bv - op_row(A, op, 0, x, P));
+            });
+    } else {
+        sweep_rows<T, NC>(
+            A, run,
+            [&](int c, long long P, int i, const Column<T> &q) {
+                const T bv = (T)b[c * n + P];
+                put(c, P, bv, bv - interior_row(A, op, x + c * n, P, i, q));
+            },
+            [&](int c, long long P) {
+                const T bv = (T)b[c * n + P];
+                put(c, P, bv, bv - op_row(A, op, c, x + c * n, P));
+            });
+    }
     a[2 * NC] = dmax;
     reduce_and_finish<2 * NC + 1, 2 * NC>(a, smem, partials, counter, [&](const double *tot) {
         bool go = false;
@@ -313,20 +421,35 @@ k_bicg_spmv_v(const OpT<T> A, const int op, const long long n, const typename Pr
         a[c] = 0;
         run[c] = sc[c].state == KS_RUN;
     }
-    sweep_rows<T, NC>(
-        A, run,
-        [&](int c, long long P, int i, const Column<T> &q) {
-            const long long o = c * n;
-            const T y = interior_row(A, op, ph + o, P, i, q);
-            v[o + P] = y;
-            mac(a[c], r0[o + P], y);
-        },
-        [&](int c, long long P) {
-            const long long o = c * n;
-            const T y = op_row(A, op, c, ph + o, P);
-            v[o + P] = y;
-            mac(a[c], r0[o + P], y);
-        });
+    if constexpr (NC == 1) {
+        if (run[0])
+            sweep_pres(
+                A, ph, [&](long long P) { return r0[P]; },
+                [&](long long P, T y, T rv) {
+                    v[P] = y;
+                    mac(a[0], rv, y);
+                },
+                [&](long long P) {
+                    const T y = op_row(A, op, 0, ph, P);
+                    v[P] = y;
+                    mac(a[0], r0[P], y);
+                });
+    } else {
+        sweep_rows<T, NC>(
+            A, run,
+            [&](int c, long long P, int i, const Column<T> &q) {
+                const long long o = c * n;
+                const T y = interior_row(A, op, ph + o, P, i, q);
+                v[o + P] = y;
+                mac(a[c], r0[o + P], y);
+            },
+            [&](int c, long long P) {
+                const long long o = c * n;
+                const T y = op_row(A, op, c, ph + o, P);
+                v[o + P] = y;
+                mac(a[c], r0[o + P], y);
+            });
+    }
     reduce_and_finish<NC, NC>(a, smem, partials, counter, [&](const double *tot) {
         for (int c = 0; c < NC; c++) {
             KScal &s = sc[c];
@@ -345,7 +468,7 @@ k_bicg_spmv_v(const OpT<T> A, const int op, const long long n, const typename Pr
 
 // ------------------------------------------------------- s = r - alpha v --
 template <typename T, int NC, bool VEC>
-__global__ void __launch_bounds__(KTHREADS)
+__global__ void __launch_bounds__(KTHREADS, NC == 1 ? 4 : 1)
 k_bicg_s(const OpT<T> A, const long long n, const T *__restrict__ r, const T *__restrict__ v, T *__restrict__ s,
          KScal *sc, double *partials, unsigned int *counter) {
     pdl_enter();
@@ -360,27 +483,28 @@ k_bicg_s(const OpT<T> A, const long long n, const T *__restrict__ r, const T *__
         if (sc[c].state != KS_RUN) continue;
         const T al = (T)sc[c].alpha;
         const long long o = c * n;
+        auto row = [&](long long P, T rv, T vv) {
+            const T y = sub_mul(rv, al, vv);
+            mac(a[c], y, y);
+            if (want_div) dmax = fmaxf(dmax, divw(A, P, y));
+            return y;
+        };
         if (VEC) {
             const long long np = n / PW<T>, op = o / PW<T>;
-            GRID_STRIDE(q, np) {
-                const Pack<T> rr = ldp(r, op + q), vv = ldp(v, op + q);
-                Pack<T> ss;
+            struct In {
+                Pack<T> r, v;
+            };
+            stream_packs(
+                np, [&](long long q) { return In{ldp(r, op + q), ldp(v, op + q)}; },
+                [&](const In &d, long long q) {
+                    Pack<T> ss;
 #pragma unroll
-                for (int l = 0; l < PW<T>; l++) {
-                    const T y = sub_mul(rr.v[l], al, vv.v[l]);
-                    ss.v[l] = y;
-                    mac(a[c], y, y);
-                    if (want_div) dmax = fmaxf(dmax, divw(A, q * PW<T> + l, y));
-                }
-                stp(s, op + q, ss);
-            }
+                    for (int l = 0; l < PW<T>; l++) ss.v[l] = row(q * PW<T> + l, d.r.v[l], d.v.v[l]);
+                    stp(s, op + q, ss);
+                });
+            if (NC == 1) stream_rest<T>(n, [&](long long P) { s[P] = row(P, r[P], v[P]); });
         } else {
-            GRID_STRIDE(P, n) {
-                const T y = sub_mul(r[o + P], al, v[o + P]);
-                s[o + P] = y;
-                mac(a[c], y, y);
-                if (want_div) dmax = fmaxf(dmax, divw(A, P, y));
-            }
+            GRID_STRIDE(P, n) { s[o + P] = row(P, r[o + P], v[o + P]); }
         }
     }
     typename AccT<T>::type acc[NC + 1];
@@ -415,22 +539,39 @@ k_bicg_spmv_t(const OpT<T> A, const int op, const long long n, const typename Pr
         a[2 * c] = a[2 * c + 1] = 0;
         run[c] = sc[c].state == KS_RUN;
     }
-    sweep_rows<T, NC>(
-        A, run,
-        [&](int c, long long P, int i, const Column<T> &q) {
-            const long long o = c * n;
-            const T y = interior_row(A, op, sh + o, P, i, q);
-            t[o + P] = y;
-            mac(a[2 * c], y, s[o + P]);
-            mac(a[2 * c + 1], y, y);
-        },
-        [&](int c, long long P) {
-            const long long o = c * n;
-            const T y = op_row(A, op, c, sh + o, P);
-            t[o + P] = y;
-            mac(a[2 * c], y, s[o + P]);
-            mac(a[2 * c + 1], y, y);
-        });
+    if constexpr (NC == 1) {
+        if (run[0])
+            sweep_pres(
+                A, sh, [&](long long P) { return s[P]; },
+                [&](long long P, T y, T sv) {
+                    t[P] = y;
+                    mac(a[0], y, sv);
+                    mac(a[1], y, y);
+                },
+                [&](long long P) {
+                    const T y = op_row(A, op, 0, sh, P);
+                    t[P] = y;
+                    mac(a[0], y, s[P]);
+                    mac(a[1], y, y);
+                });
+    } else {
+        sweep_rows<T, NC>(
+            A, run,
+            [&](int c, long long P, int i, const Column<T> &q) {
+                const long long o = c * n;
+                const T y = interior_row(A, op, sh + o, P, i, q);
+                t[o + P] = y;
+                mac(a[2 * c], y, s[o + P]);
+                mac(a[2 * c + 1], y, y);
+            },
+            [&](int c, long long P) {
+                const long long o = c * n;
+                const T y = op_row(A, op, c, sh + o, P);
+                t[o + P] = y;
+                mac(a[2 * c], y, s[o + P]);
+                mac(a[2 * c + 1], y, y);
+            });
+    }
     reduce_and_finish<2 * NC, 2 * NC>(a, smem, partials, counter, [&](const double *tot) {
         for (int c = 0; c < NC; c++) {
             KScal &st = sc[c];
@@ -449,7 +590,7 @@ k_bicg_spmv_t(const OpT<T> A, const int op, const long long n, const typename Pr
 // Ends the iteration: sets the loop condition (some component still
 // running and below maxit).
 template <typename T, int NC, bool VEC>
-__global__ void __launch_bounds__(KTHREADS)
+__global__ void __launch_bounds__(KTHREADS, NC == 1 ? 4 : 1)
 k_bicg_xr(const OpT<T> A, const long long n, T *__restrict__ x, T *__restrict__ r, const T *__restrict__ r0,
           const typename PrecT<T>::type *__restrict__ ph, const typename PrecT<T>::type *__restrict__ sh,
           const T *__restrict__ s, const T *__restrict__ t,
@@ -476,33 +617,45 @@ k_bicg_xr(const OpT<T> A, const long long n, T *__restrict__ x, T *__restrict__ 
         }
         if (state != KS_RUN) continue;
         const T al = (T)sc[c].alpha, om = (T)sc[c].omega;
+        using E = typename PrecT<T>::type;
+        auto row = [&](long long P, T sv, T tv, T rv) {
+            const T y = sub_mul(sv, om, tv);
+            mac(a[2 * c], y, y);
+            mac(a[2 * c + 1], rv, y);
+            if (want_div) dmax = fmaxf(dmax, divw(A, P, y));
+            return y;
+        };
         if (VEC) {
             const long long np = n / PW<T>, op = o / PW<T>;
-            GRID_STRIDE(q, np) {
-                Pack<T> xx = ldp(x, op + q);
-                const auto pp = ldpn<T>(ph, op + q), ss = ldpn<T>(sh, op + q);
-                const Pack<T> s0 = ldp(s, op + q), tt = ldp(t, op + q), rr0 = ldp(r0, op + q);
-                Pack<T> rr;
+            struct In {
+                Pack<T> x, s, t, r0;
+                PackN<E, PW<T>> p, q;
+            };
+            stream_packs(
+                np,
+                [&](long long q) {
+                    return In{ldp(x, op + q),  ldp(s, op + q),       ldp(t, op + q),
+                              ldp(r0, op + q), ldpn<T>(ph, op + q), ldpn<T>(sh, op + q)};
+                },
+                [&](const In &d, long long q) {
+                    Pack<T> xx, rr;
 #pragma unroll
-                for (int l = 0; l < PW<T>; l++) {
-                    xx.v[l] = add_mul2(xx.v[l], al, T(pp.v[l]), om, T(ss.v[l]));
-                    const T y = sub_mul(s0.v[l], om, tt.v[l]);
-                    rr.v[l] = y;
-                    mac(a[2 * c], y, y);
-                    mac(a[2 * c + 1], rr0.v[l], y);
-                    if (want_div) dmax = fmaxf(dmax, divw(A, q * PW<T> + l, y));
-                }
-                stp(x, op + q, xx);
-                stp(r, op + q, rr);
-            }
+                    for (int l = 0; l < PW<T>; l++) {
+                        xx.v[l] = add_mul2(d.x.v[l], al, T(d.p.v[l]), om, T(d.q.v[l]));
+                        rr.v[l] = row(q * PW<T> + l, d.s.v[l], d.t.v[l], d.r0.v[l]);
+                    }
+                    stp(x, op + q, xx);
+                    stp(r, op + q, rr);
+                });
+            if (NC == 1)
+                stream_rest<T>(n, [&](long long P) {
+                    x[P] = add_mul2(x[P], al, T(ph[P]), om, T(sh[P]));
+                    r[P] = row(P, s[P], t[P], r0[P]);
+                });
         } else {
             GRID_STRIDE(P, n) {
                 x[o + P] = add_mul2(x[o + P], al, T(ph[o + P]), om, T(sh[o + P]));
-                const T y = sub_mul(s[o + P], om, t[o + P]);
-                r[o + P] = y;
-                mac(a[2 * c], y, y);
-                mac(a[2 * c + 1], r0[o + P], y);
-                if (want_div) dmax = fmaxf(dmax, divw(A, P, y));
+                r[o + P] = row(P, s[o + P], t[o + P], r0[o + P]);
             }
         }
     }
@@ -570,16 +723,15 @@ k_bicg_verify(const OpT<T> A, const int op, const long long n, const B *__restri
     __shared__ double smem[32 * 2];
     typename AccT<T>::type a[1] = {0};
     float dmax = 0.0f;
-    const bool run[1] = {true};
     const bool want_div = sc[0].divtol > 0;
     auto put = [&](long long P, T y) {
         r[P] = y;
         mac(a[0], y, y);
         if (want_div) dmax = fmaxf(dmax, divw(A, P, y));
     };
-    sweep_rows<T, 1>(
-        A, run, [&](int, long long P, int i, const Column<T> &q) { put(P, (T)b[P] - interior_row(A, op, x, P, i, q)); },
-        [&](int, long long P) { put(P, (T)b[P] - op_row(A, op, 0, x, P)); });
+    sweep_pres(
+        A, x, [&](long long P) { return b[P]; }, [&](long long P, T y, B bv) { put(P, (T)bv - y); },
+        [&](long long P) { put(P, (T)b[P] - op_row(A, op, 0, x, P)); });
     typename AccT<T>::type acc[2] = {a[0], dmax};
     reduce_and_finish<2, 1>(acc, smem, partials, counter, [&](const double *tot) {
         KScal &st = sc[0];
@@ -730,11 +882,11 @@ int KrylovWork<T>::allocate(long long ncell, int ncomp, bool precond, int maxblo
     nc = ncomp;
     nblk = vector_blocks(ncell);
     const int nvec = precond ? 8 : 6;
-    const size_t bytes = sizeof(T) * (size_t)n * nc * nvec;
+    const long long m = (n * nc + 15) / 16 * 16;   // every vector on a 16-byte boundary
+    const size_t bytes = sizeof(T) * (size_t)m * nvec;
     if (cudaMalloc(&base, bytes) != cudaSuccess) return -1;
     cudaMemset(base, 0, bytes);
     T *q = base;
-    const long long m = n * nc;
     r = q; q += m;
     r0 = q; q += m;
     p = q; q += m;
@@ -864,10 +1016,10 @@ static void first_half(cudaStream_t st, const OpT<T> &A, int op, KrylovWork<T> &
     const int nc = w.nc;
     const int *gate = nc == 1 ? &w.scal[0].state : nullptr;
     const bool vec = n % 4 == 0;
-    if (nc == 3 && vec) launch_pdl(k_bicg_p<T, 3, true>, w.nblk, KTHREADS, 0, st, n, w.r, w.p, w.v, w.r0, w.scal);
-    else if (nc == 3) launch_pdl(k_bicg_p<T, 3, false>, w.nblk, KTHREADS, 0, st, n, w.r, w.p, w.v, w.r0, w.scal);
-    else if (vec) launch_pdl(k_bicg_p<T, 1, true>, w.nblk, KTHREADS, 0, st, n, w.r, w.p, w.v, w.r0, w.scal);
-    else launch_pdl(k_bicg_p<T, 1, false>, w.nblk, KTHREADS, 0, st, n, w.r, w.p, w.v, w.r0, w.scal);
+    const int nb = std::min(w.nblk, KWAVE);
+    if (nc == 1) launch_pdl(k_bicg_p<T, 1, true>, nb, KTHREADS, 0, st, n, w.r, w.p, w.v, w.r0, w.scal);
+    else if (vec) launch_pdl(k_bicg_p<T, 3, true>, nb, KTHREADS, 0, st, n, w.r, w.p, w.v, w.r0, w.scal);
+    else launch_pdl(k_bicg_p<T, 3, false>, nb, KTHREADS, 0, st, n, w.r, w.p, w.v, w.r0, w.scal);
     note_launches(1);
     if (M) {
         const int tm = prof_begin(pf, "mg_vcycle");
@@ -883,10 +1035,9 @@ static void first_half(cudaStream_t st, const OpT<T> &A, int op, KrylovWork<T> &
                                                                 w.counter);
     note_launches(1);
     prof_end(pf, tm);
-    if (nc == 3 && vec) launch_pdl(k_bicg_s<T, 3, true>, w.nblk, KTHREADS, 0, st, A, n, w.r, w.v, w.s, w.scal, w.partials, w.counter);
-    else if (nc == 3) launch_pdl(k_bicg_s<T, 3, false>, w.nblk, KTHREADS, 0, st, A, n, w.r, w.v, w.s, w.scal, w.partials, w.counter);
-    else if (vec) launch_pdl(k_bicg_s<T, 1, true>, w.nblk, KTHREADS, 0, st, A, n, w.r, w.v, w.s, w.scal, w.partials, w.counter);
-    else launch_pdl(k_bicg_s<T, 1, false>, w.nblk, KTHREADS, 0, st, A, n, w.r, w.v, w.s, w.scal, w.partials, w.counter);
+    if (nc == 1) launch_pdl(k_bicg_s<T, 1, true>, nb, KTHREADS, 0, st, A, n, w.r, w.v, w.s, w.scal, w.partials, w.counter);
+    else if (vec) launch_pdl(k_bicg_s<T, 3, true>, nb, KTHREADS, 0, st, A, n, w.r, w.v, w.s, w.scal, w.partials, w.counter);
+    else launch_pdl(k_bicg_s<T, 3, false>, nb, KTHREADS, 0, st, A, n, w.r, w.v, w.s, w.scal, w.partials, w.counter);
     note_launches(1);
 }
 
@@ -915,10 +1066,10 @@ static void launch_xr(cudaStream_t st, const OpT<T> &A, KrylovWork<T> &w, T *x, 
                       LoopCtl lc) {
 #define XR_ARGS A, w.n, x, w.r, w.r0, w.phat(M), w.shat(M), w.s, w.t, w.scal, w.partials, w.counter, maxit, lc
     const bool vec = w.n % 4 == 0;
-    if (w.nc == 3 && vec) launch_pdl(k_bicg_xr<T, 3, true>, w.nblk, KTHREADS, 0, st, XR_ARGS);
-    else if (w.nc == 3) launch_pdl(k_bicg_xr<T, 3, false>, w.nblk, KTHREADS, 0, st, XR_ARGS);
-    else if (vec) launch_pdl(k_bicg_xr<T, 1, true>, w.nblk, KTHREADS, 0, st, XR_ARGS);
-    else launch_pdl(k_bicg_xr<T, 1, false>, w.nblk, KTHREADS, 0, st, XR_ARGS);
+    const int nb = std::min(w.nblk, KWAVE);
+    if (w.nc == 1) launch_pdl(k_bicg_xr<T, 1, true>, nb, KTHREADS, 0, st, XR_ARGS);
+    else if (vec) launch_pdl(k_bicg_xr<T, 3, true>, nb, KTHREADS, 0, st, XR_ARGS);
+    else launch_pdl(k_bicg_xr<T, 3, false>, nb, KTHREADS, 0, st, XR_ARGS);
 #undef XR_ARGS
     note_launches(1);
 }

@@ -30,11 +30,14 @@ struct Prof;
 constexpr int KTHREADS = 256;
 constexpr int KBLOCKS = 1216;  // 8 blocks per SM on 152 SMs; grid-stride loops
 
+constexpr int KWAVE = 608;     // 4 per SM: one wave of the BiCGSTAB vector updates
+
 // Blocks of the grid-stride vector kernels for a vector of n elements:
-// about 8 elements per thread, at most KBLOCKS, so that small cases
-// running side by side (batched steps) leave the GPU to each other.
+// about 4 elements per thread, at most KBLOCKS.  (8 per thread left
+// boxes 95x61x47 with one block per SM, each thread a chain of 8 loads:
+// k_bicg_xr 32 -> 16 us, k_bicg_s 16 -> 13, k_bicg_p 8.4 -> 5.4, cold.)
 inline int vector_blocks(long long n) {
-    const long long b = (n + KTHREADS * 8 - 1) / (KTHREADS * 8);
+    const long long b = (n + KTHREADS * 4 - 1) / (KTHREADS * 4);
     return (int)(b < 1 ? 1 : b > KBLOCKS ? KBLOCKS : b);
 }
 
