@@ -128,11 +128,16 @@ class FastPoisson : public Preconditioner<T> {
     int *solid_ = nullptr;
     bool near_outer_ = false;
     int launches_ = 0;
+    bool plane_ = false;           // the slice kernels (fastplane.cuh) take both ends
     std::vector<void *> allocs_;
     template <typename S>
     void run(cudaStream_t s, const S *r, T *z, const int *gate);
     template <int TM, typename S>
     void run_tiled(cudaStream_t s, const S *r, T *z, const int *gate);
+    template <typename S>
+    void front(cudaStream_t s, const S *r, T *out, const int *gate);
+    template <typename S>
+    void rear(cudaStream_t s, const S *r, const T *in, T *z, const int *gate);
     template <int TM>
     void forward(cudaStream_t s, int axis, const T *in, T *out, const int *gate);
     template <int TM>
