@@ -102,7 +102,8 @@ void launch_ustar_prhs(cudaStream_t s, const Grid &g, const Axis &ax, const Axis
                        const BCSet &bc, const uint8_t *flag, const UstarArgs &a, double dt, double Re);
 // when: 0 fills with the values at the step's start time, 1 at its end
 // time (the two differ only for VAL_FUNC faces).
-void launch_fill_outer(cudaStream_t s, const Grid &g, const BCSet &bc, double *const u[3], double *p, int when);
+void launch_fill_outer(cudaStream_t s, const Grid &g, const BCSet &bc, const int *outer, int nout, double *const u[3],
+                       double *p, int when);
 // x[l n + P] = u[l][P] (NaN, as on solid cells, becomes 0): the initial
 // guess of the momentum solve.
 void launch_velocity_guess(cudaStream_t s, const Grid &g, double *const u[3], double *x);

@@ -993,7 +993,7 @@ void calc_tau(IBMSolver *sv) {
 // when: 0 at the step's start time (iterate prologue), 1 at its end.
 void fill_outer(IBMSolver *sv, int when) {
     ibm3d_device *d = sv->dev;
-    launch_fill_outer(d->s, d->g, d->bc, d->u, d->p, when);
+    launch_fill_outer(d->s, d->g, d->bc, d->A64.sw.outer, d->A64.sw.nout, d->u, d->p, when);
 }
 
 // ------------------------------------------------- VAL_FUNC sampling ---
