@@ -719,7 +719,9 @@ __global__ void __launch_bounds__(SW_THREADS, std::is_same<T, dfloat>::value ? 4
 k_bicg_verify(const OpT<T> A, const int op, const long long n, const B *__restrict__ b, const T *__restrict__ x,
               T *r, KScal *sc, double *partials, unsigned int *counter, const int maxit, const LoopCtl lc) {
     pdl_enter();
-    if (sc[0].state != KS_DONE) return;   // the same value in every block: written only by the last one below
+    // The same values in every block: written only by the last one below.  No
+    // iteration: the residual that passed was the true one.
+    if (sc[0].state != KS_DONE || sc[0].iters == 0) return;
     __shared__ double smem[32 * 2];
     typename AccT<T>::type a[1] = {0};
     float dmax = 0.0f;
@@ -1383,17 +1385,27 @@ static int end_while(cudaStream_t body_stream) {
 }
 
 // Init (already recorded by the caller with lc) + while loop of iterations
-// (vb as in host_loop).
+// (vb as in host_loop).  The first `ahead` iterations are recorded before the
+// loop, since each pass of a while node costs some microseconds beside its
+// kernels, and kernels of a solve that has ended return at once (the first
+// pressure iteration and sweep pair ahead: cavity 32^3 5.13 -> 5.01 ms for 20
+// steps, 213x32x59 8.70 -> 8.48 for 10).
 template <typename T, typename B = T>
 static int record_loop(cudaStream_t st, cudaStream_t body, const OpT<T> &A, int op, KrylovWork<T> &w, T *x,
-                       int maxit, Preconditioner<T> *M, const LoopCtl &lc, int *per_iter, const B *vb = nullptr) {
+                       int maxit, Preconditioner<T> *M, const LoopCtl &lc, int *per_iter, int ahead,
+                       const B *vb = nullptr) {
+    auto iteration = [&](cudaStream_t q) {
+        first_half(q, A, op, w, M, nullptr);
+        second_half(q, A, op, w, M, nullptr);
+        launch_xr(q, A, w, x, maxit, M, lc);
+        if (vb) launch_verify(q, A, op, w, vb, x, maxit, lc);
+    };
+    for (int i = 0; i < ahead; i++) iteration(st);
     if (begin_while(st, lc, body) != 0) return -1;
-    first_half(body, A, op, w, M, nullptr);
-    second_half(body, A, op, w, M, nullptr);
-    launch_xr(body, A, w, x, maxit, M, lc);
-    if (vb) launch_verify(body, A, op, w, vb, x, maxit, lc);
+    iteration(body);
     if (end_while(body) != 0) return -1;
     *per_iter = 5 + (vb ? 1 : 0) + (M ? 2 * M->launches() : 0);
+    note_launches(-ahead * *per_iter);   // counted with the solve's iterations
     return 0;
 }
 
@@ -1404,7 +1416,7 @@ int record_bicgstab(cudaStream_t st, const cudaStream_t *aux, const OpT<T> &A, i
     if (new_loop(st, lc) != 0) return -1;
     if (prm.x_given) launch_init_guess(st, A, op, w, b, x, prm.tol, prm.divtol, lc, prm.maxit);
     else launch_init(st, w, b, x, prm.tol, prm.divtol, nullptr, 0.0, 0.0, lc);
-    if (record_loop(st, aux[0], A, op, w, x, prm.maxit, M, lc, per_iter) != 0) return -1;
+    if (record_loop(st, aux[0], A, op, w, x, prm.maxit, M, lc, per_iter, op == OP_PRES ? 1 : 0) != 0) return -1;
     cudaMemcpyAsync(w.scal_h, w.scal, sizeof(KScal) * w.nc, cudaMemcpyDeviceToHost, st);
     *fixed = 1;
     return 0;
@@ -1430,7 +1442,7 @@ int record_bicgstab_df(cudaStream_t st, const cudaStream_t *aux, const OpT<dfloa
     } else {
         launch_init(st, w, b, xw, prm.tol, prm.divtol, nullptr, 0.0, 0.0, lc);
     }
-    if (record_loop(st, aux[0], A, op, w, xw, prm.maxit, M, lc, per_iter, b) != 0) return -1;
+    if (record_loop(st, aux[0], A, op, w, xw, prm.maxit, M, lc, per_iter, 1, b) != 0) return -1;
     launch_from_dfloat(st, m, xw, x);
     cudaMemcpyAsync(w.scal_h, w.scal, sizeof(KScal) * w.nc, cudaMemcpyDeviceToHost, st);
     *fixed = prm.x_given ? 3 : 2;
@@ -1453,7 +1465,7 @@ int record_ir(cudaStream_t st, const cudaStream_t *aux, const OpT<double> &A64, 
         LoopCtl inner;
         if (new_loop(bs, inner) != 0) return -1;
         launch_init(bs, w.inner, w.b32, w.e32, prm.inner_tol, 0.0, w.scal, prm.tol, prm.divtol, inner);
-        if (record_loop(bs, aux[1], A32, op, w.inner, w.e32, prm.maxit, M32, inner, per_iter) != 0) return -1;
+        if (record_loop(bs, aux[1], A32, op, w.inner, w.e32, prm.maxit, M32, inner, per_iter, 0) != 0) return -1;
         launch_update(bs, w, x);
         launch_residual(bs, A64, op, w, b, x, IR_NEXT, prm, outer);
     }
@@ -1469,7 +1481,7 @@ int record_inc(cudaStream_t st, const cudaStream_t *aux, const OpT<float> &A32, 
     LoopCtl lc;
     if (new_loop(st, lc) != 0) return -1;
     launch_init(st, w.inner, w.b32, w.e32, prm.inner_tol, 0.0, w.scal, prm.tol, 0.0, lc);
-    if (record_loop<float>(st, aux[0], A32, op, w.inner, w.e32, prm.maxit, nullptr, lc, per_iter) != 0) return -1;
+    if (record_loop<float>(st, aux[0], A32, op, w.inner, w.e32, prm.maxit, nullptr, lc, per_iter, 0) != 0) return -1;
     cudaMemcpyAsync(w.inner.scal_h, w.inner.scal, sizeof(KScal) * w.nc, cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(w.scal_h, w.scal, sizeof(IRScal) * w.nc, cudaMemcpyDeviceToHost, st);
     *fixed = 1;
@@ -1900,13 +1912,16 @@ int record_sweeps(cudaStream_t st, const cudaStream_t *aux, const OpT<T> &A, Mom
     int k = 0, body = 0;
     if (!launch_first(st, A, ms, w, b, x, prm, ir, limit, sweeps, &k))
         k += launch_sweep(st, A, ms, w, b, x, prm, ir, limit, true, sweeps);
+    // The pair that nearly every solve needs, before the loop (record_loop).
+    launch_sweep(st, A, ms, w, b, x, prm, ir, limit, false, sweeps);
+    launch_sweep(st, A, ms, w, b, x, prm, ir, limit, true, sweeps);
     if (begin_while(st, sweeps, aux[0]) != 0) return -1;
     body += launch_sweep(aux[0], A, ms, w, b, x, prm, ir, limit, false, sweeps);
     body += launch_sweep(aux[0], A, ms, w, b, x, prm, ir, limit, true, sweeps);
     if (end_while(aux[0]) != 0) return -1;
     k += launch_end(st, A, ms, w, b, x, prm, ir, rest);
     int it = 0;
-    if (record_loop<T>(st, aux[0], A, OP_MOM, w, x, prm.maxit, nullptr, rest, &it) != 0) return -1;
+    if (record_loop<T>(st, aux[0], A, OP_MOM, w, x, prm.maxit, nullptr, rest, &it, 0) != 0) return -1;
     cudaMemcpyAsync(w.scal_h, w.scal, sizeof(KScal) * w.nc, cudaMemcpyDeviceToHost, st);
     note_launches(k + body);
     *per_iter = (body + 1) / 2;
