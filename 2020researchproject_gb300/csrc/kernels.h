@@ -95,9 +95,10 @@ struct GhostArgs {
 void launch_conv_rhs(cudaStream_t s, const Grid &g, const Axis &ax, const Axis &ay, const Axis &az,
                      const BCSet &bc, const uint8_t *flag, const ConvArgs &a, double dt, const double f[3],
                      int les);
+void launch_les_delta(cudaStream_t s, const Grid &g, const Axis &ax, const Axis &ay, const Axis &az, double *delta);
 void launch_smagorinsky(cudaStream_t s, const Grid &g, const Axis &ax, const Axis &ay, const Axis &az,
-                        const uint8_t *flag, const double *lvset, const double *const u[3], const TauArgs &t,
-                        double cs);
+                        const uint8_t *flag, const double *lvset, const double *delta, const double *const u[3],
+                        const TauArgs &t, double cs);
 void launch_ustar_prhs(cudaStream_t s, const Grid &g, const Axis &ax, const Axis &ay, const Axis &az,
                        const BCSet &bc, const uint8_t *flag, const UstarArgs &a, double dt, double Re);
 // when: 0 fills with the values at the step's start time, 1 at its end

@@ -86,6 +86,7 @@ struct ibm3d_device {
     int *gid = nullptr;
     // Pressure-guess extrapolation (IBMSolver_set_pressure_guess): the
     // increment before the last one, and how many increments are known.
+    double *les_delta = nullptr;  // Smagorinsky filter width per cell (LES cases)
     double *pp_prev = nullptr;
     int *pp_hist = nullptr;
     int p_guess = 1;   // warm-started (mixed) pressure solves start from the extrapolation
@@ -343,6 +344,7 @@ void release_device(ibm3d_device *d) {
     }
     dfree(d->fields);
     dfree(d->f32);
+    dfree(d->les_delta);
     dfree(d->pp_prev);
     dfree(d->pp_hist);
     dfree(d->flag);
@@ -481,7 +483,7 @@ bool alloc_fields(IBMSolver *sv) {
     for (int l = 0; l < 3; l++) d->Us[l] = take(1);
     d->p = take(1);
     d->pn = take(1);
-    d->pp = take(1);
+    d->pp = take(1);   // 20 fields precede it: on a 16-byte boundary for any n (BiCGSTAB's packs)
     for (int l = 0; l < 3; l++) d->N[l] = take(1);
     for (int l = 0; l < 3; l++) d->Np[l] = take(1);
     for (int l = 0; l < 6; l++) d->tau[l] = take(1);
@@ -494,6 +496,11 @@ bool alloc_fields(IBMSolver *sv) {
     d->pp_prev = dmalloc<double>(sv, n, "pressure increment history");
     d->pp_hist = dmalloc<int>(sv, 1, "pressure increment count");
     if (!d->pp_prev || !d->pp_hist) return false;
+    if (d->les) {
+        d->les_delta = dmalloc<double>(sv, n, "filter width");
+        if (!d->les_delta) return false;
+        launch_les_delta(d->s, d->g, d->ax[0], d->ax[1], d->ax[2], d->les_delta);
+    }
     for (int l = 0; l < 3; l++) {
         d->N32[l] = d->f32 + (size_t)l * n;
         d->Np32[l] = d->f32 + (size_t)(3 + l) * n;
@@ -987,7 +994,8 @@ void calc_tau(IBMSolver *sv) {
     TauArgs t{};
     for (int q = 0; q < 6; q++) t.tau[q] = d->tau[q];
     const double *u[3] = {d->u[0], d->u[1], d->u[2]};
-    launch_smagorinsky(d->s, d->g, d->ax[0], d->ax[1], d->ax[2], d->flag, d->lvset, u, t, sv->turb_model.Cs);
+    launch_smagorinsky(d->s, d->g, d->ax[0], d->ax[1], d->ax[2], d->flag, d->lvset, d->les_delta, u, t,
+                       sv->turb_model.Cs);
 }
 
 // when: 0 at the step's start time (iterate prologue), 1 at its end.
