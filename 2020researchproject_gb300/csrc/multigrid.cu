@@ -514,22 +514,18 @@ k_mg0_restrict_g(const OpT<T> c, const FineRows<T> fr, const T *__restrict__ z, 
     }
 }
 
-// Prolongation into the fine grid from a level 1 of uneven groups: each
-// thread takes one fine (j, k) on mg0_pplanes<T>() consecutive planes (four
-// in FP32; one in FP64, whose blend is bound by the FP64 pipe rather than
-// by latency), reads its j and k transfer tables once, addresses coarse
-// cells in 32-bit arithmetic (a level has fewer than 2^31 cells) and
-// issues every load (flags, z, the x tables, the coarse values) before any
-// store; a cell that takes no correction stores z back.  Same arithmetic
-// as prolong_value.  Grid (ceil(nz/32), ceil(ny/8), ceil(nx/planes)) of
-// 32 x 8 threads.
-template <typename T>
-__host__ __device__ constexpr int mg0_pplanes() { return sizeof(T) == 4 ? 4 : 1; }
+// Prolongation into the fine grid from a level 1 of uneven groups, FP32: each
+// thread takes one fine (j, k) on MG0_PPLANES consecutive planes, reads its j
+// and k transfer tables once, addresses coarse cells in 32-bit arithmetic (a
+// level has fewer than 2^31 cells) and issues every load (flags, z, the x
+// tables, the coarse values) before any store; a cell that takes no
+// correction stores z back.  Same arithmetic as prolong_value.  Grid
+// (ceil(nz/32), ceil(ny/8), ceil(nx/planes)) of 32 x 8 threads.
+constexpr int MG0_PPLANES = 4;
 
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_mg0_prolong(const OpT<T> c, T *z, const MGLevel<T> C, const int *gate) {
-    constexpr int MG0_PPLANES = mg0_pplanes<T>();
     MG_GATE(gate);
     const Grid &g = c.g;
     const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
@@ -566,14 +562,69 @@ k_mg0_prolong(const OpT<T> c, T *z, const MGLevel<T> C, const int *gate) {
                     act[a][b][cc] = active_bits(C.diag[q]);
                 }
         const bool take = (fl == FLUID || fl == GHOST) && !(c.p_singular && P == c.pinned);
-        // As in the restriction: the FP64 blend only where it is used.
-        const T corr = sizeof(T) == 4 || take ? trilinear(v, act, wxs, wys, wzs) : (T)0;
+        const T corr = trilinear(v, act, wxs, wys, wzs);
         out[p] = take ? zp + corr : zp;
         Ps[p] = P;
     }
 #pragma unroll
     for (int p = 0; p < MG0_PPLANES; p++)
         if (i0 + p < g.nx) z[Ps[p]] = out[p];
+}
+
+// The same in FP64, bound by the FP64 pipe: a thread walks MG0_LPLANES planes
+// of its (j, k) and keeps the blend along j and k of the two coarse planes at
+// hand (the walk is the same for every thread), so a plane's six operations
+// serve every fine plane beside it and a plane that is a group of its own
+// (weight 1) takes no blend along x.  Where a coarse cell is inactive:
+// prolong_value.  Sphere 192x128x128: 188 -> 102 us.
+constexpr int MG0_LPLANES = 8;
+
+__global__ void __launch_bounds__(256)
+k_mg0_prolong_lines(const OpT<double> c, double *z, const MGLevel<double> C, const int *gate) {
+    MG_GATE(gate);
+    const Grid &g = c.g;
+    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+    if (k >= g.nz || j >= g.ny) return;
+    const int i0 = blockIdx.z * MG0_LPLANES, i1 = min(i0 + MG0_LPLANES, g.nx);
+    const int cny = C.ny, cnz = C.nz;
+    const double wy = C.pw[1][j], wz = C.pw[2][k], vy = 1.0 - wy, vz = 1.0 - wz;
+    // Weight 1: the covering cell alone (there may be none beside it).
+    const int y0 = C.pa[1][j], y1 = wy == 1.0 ? y0 : C.po[1][j], k0 = C.pa[2][k], k1 = wz == 1.0 ? k0 : C.po[2][k];
+    struct Line {
+        int I;
+        bool full;
+        double v;
+    };
+    auto line = [&](int I) {
+        Line l{I, I >= 0 && y1 >= 0 && k1 >= 0, 0.0};
+        if (!l.full) return l;
+        const int q0 = (I * cny + y0) * cnz, q1 = (I * cny + y1) * cnz;
+        const double a = C.Z[q0 + k0], b = C.Z[q0 + k1], d = C.Z[q1 + k0], e = C.Z[q1 + k1];
+        l.full = active_bits(C.diag[q0 + k0]) && active_bits(C.diag[q0 + k1]) && active_bits(C.diag[q1 + k0]) &&
+                 active_bits(C.diag[q1 + k1]);
+        if (l.full) l.v = wy * (wz * a + vz * b) + vy * (wz * d + vz * e);
+        return l;
+    };
+    Line own{-2, false, 0.0}, beside{-2, false, 0.0};
+    long long P = cidx(g, i0, j, k);
+    for (int i = i0; i < i1; i++, P += g.sx) {
+        const int I = C.pa[0][i], J = C.po[0][i];
+        const double wx = C.pw[0][i];
+        const uint8_t fl = c.flag[P];
+        const double zp = z[P];
+        if (own.I != I) {
+            const Line last = own;
+            own = beside.I == I ? beside : line(I);
+            beside = last;
+        }
+        const bool alone = wx == 1.0;
+        if (!alone && beside.I != J) beside = line(J);
+        if ((fl != FLUID && fl != GHOST) || (c.p_singular && P == c.pinned)) continue;
+        double corr;
+        if (own.full && (alone || beside.full)) corr = alone ? own.v : wx * own.v + (1.0 - wx) * beside.v;
+        else corr = prolong_value(C, i, j, k);
+        z[P] = zp + corr;
+    }
 }
 
 // Restriction when level 1 halves every axis: one thread per fine (j, k)
@@ -1796,10 +1847,12 @@ void GMG<T>::cycle(cudaStream_t s, const FineRows<T> &fr, T *z, const int *gate)
     tp = tb("mg0_prolong");
     if (L1.cx && L1.cy && L1.cz)
         launch_pdl(k_mg0_prolong2<T>, l3_grid(g.nx, g.ny, g.nz), l3_block(), 0, s, A_, z, L1, gate);
+    else if constexpr (sizeof(T) == 8)
+        launch_pdl(k_mg0_prolong_lines, dim3((g.nz + 31) / 32, (g.ny + 7) / 8, (g.nx + MG0_LPLANES - 1) / MG0_LPLANES),
+                   dim3(32, 8), 0, s, A_, z, L1, gate);
     else
-        launch_pdl(k_mg0_prolong<T>,
-                   dim3((g.nz + 31) / 32, (g.ny + 7) / 8, (g.nx + mg0_pplanes<T>() - 1) / mg0_pplanes<T>()), dim3(32, 8), 0,
-                   s, A_, z, L1, gate);
+        launch_pdl(k_mg0_prolong<T>, dim3((g.nz + 31) / 32, (g.ny + 7) / 8, (g.nx + MG0_PPLANES - 1) / MG0_PPLANES),
+                   dim3(32, 8), 0, s, A_, z, L1, gate);
     k++;
     te(tp);
     k += smooth0(s, fr, z, cfg_.nu_post, false, gate);
