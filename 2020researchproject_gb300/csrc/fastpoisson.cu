@@ -126,9 +126,9 @@ k_fp_gather(const OpT<T> c, const S *__restrict__ r, T *__restrict__ f, const Fp
 // x_(n-1-i) = E - O (k_fp_back).
 //
 // Sphere 192x128x128 FP32, cold: forward z 26 -> 16, forward y 25 -> 21,
-// backward y 25 -> 25, backward z 27 -> 22 us (half the products; the loads
-// of both halves and the register tiles' shared-memory reads bound them
-// now); cavity 64^3 FP64, an application: 0.36 -> 0.23 ms.
+// backward y 25 -> 18 (25 with four blocks to an SM, a wave and a quarter;
+// six), backward z 27 -> 22 us (half the products; the loads of both halves
+// and the register tiles' shared-memory reads bound them now); cavity 64^3 FP64, an application: 0.36 -> 0.23 ms.
 //
 // Tiles: TM = 64 (R = 8) or 32 in FP32, 32 (R = 4) or 16 in FP64 (run).
 template <typename T, int TM>
@@ -320,7 +320,7 @@ struct FpBack {
 };
 
 template <typename T, int TM, bool ROWS, bool FOLD, typename S>
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(64, sizeof(T) == 4 && TM == 64 && !ROWS ? 6 : 1)
 k_fp_back(const FpBack<T> p, const FpScatter<T, S> sc, const int *gate) {
     FP_GATE(gate);
     using Tile = FpTile<T, TM>;
