@@ -11,7 +11,7 @@ seeded inputs (the reference has no public dataset).
 Metric: Mcell-steps/s = interior cells x steps / seconds, for the
 mixed-precision step (the autotuner's choice among the mixed forms; on this
 workload IBM3D_MIXED32: FP32 explicit stages and momentum solve, the
-pressure BiCGSTAB on double-float vectors with the FP32 multigrid, FP64
+pressure BiCGSTAB on double-float vectors with the FP32 preconditioner, FP64
 right-hand side, solution, scalars and divergence check), with the plain
 FP64 step measured beside it on the same state ("fp64", "mixed_vs_fp64")
 and the velocity difference between the two after the run
@@ -23,8 +23,8 @@ and the velocity difference between the two after the run
           uploads u1, u2, u3, p from pinned host memory
           (IBMSolver_init_flow_array), runs IBMSolver_iterate(1) and reads
           the four fields back (IBMSolver_get_field); host wall clock.
-  roofline: the dominant kernel (fine-grid colour pass of the pressure
-          multigrid) timed with CUDA events on the solver's stream, against
+  roofline: the largest kernel per launch (mixed: the projection; FP64: the
+          fine-grid colour pass of the pressure multigrid) timed with CUDA events on the solver's stream, against
           the measured HBM copy bandwidth.
 Default run: N=1, K=10 timed steps after W=3 warm-up steps;
 --precision fp64 makes the plain FP64 step the headline.
@@ -307,8 +307,8 @@ def _vel_rel_l2(a, b):
 def step_roofline(ms_per_step, cells, k_u, k_p, mixed, les, peak):
     """Step-level roofline from the algorithmic-bytes model of the step:
     B_step = 336 + 3 k_u 144 + k_p B_pois (+ 104 with LES) bytes per cell,
-    B_pois = 492 with the FP64 multigrid, 318 with the FP32 one, with k_u
-    and k_p the measured Krylov iterations per step (momentum per
+    B_pois = 492 with the FP64 preconditioner, 318 with the FP32 one, with k_u
+    and k_p the measured iterations per step (momentum per
     component, pressure)."""
     b_pois = 318.0 if mixed else 492.0
     b_step = 336.0 + 3 * k_u * 144.0 + k_p * b_pois + (104.0 if les else 0.0)
@@ -465,21 +465,23 @@ def bench_gb300(args):
     prof = s.profile()
     s.set_profiling(False)
 
-    # --- roofline of the dominant kernel: the fine-grid colour pass of the
-    # pressure multigrid (FP32 in the mixed step, FP64 in the plain one),
-    # back to back (as inside a V-cycle, L2-warm) and with the L2
-    # overwritten before each launch (cold).
-    k_ms, k_bytes = s.time_kernel("mg_color", reps=50)
-    kc_ms, _ = s.time_kernel("mg_color", reps=20, cold=True)
-    kname = "k_mg0_color_f32" if args.precision == "mixed" else "k_mg0_color_f64"
+    # --- roofline of the largest kernel per launch, back to back and with the
+    # L2 overwritten before each launch (cold): the projection in the mixed
+    # step, the fine-grid colour pass of the pressure multigrid in the plain
+    # FP64 one.
+    kind, kname, what = (("update_next", "k_update_next_tiled_f32", "projection, new velocity and divergence check")
+                         if args.precision == "mixed" else
+                         ("mg_color", "k_mg0_color_f64", "fine-grid Gauss-Seidel colour pass, pressure multigrid"))
+    k_ms, k_bytes = s.time_kernel(kind, reps=50)
+    kc_ms, _ = s.time_kernel(kind, reps=20, cold=True)
     ach_cold = k_bytes / (kc_ms / 1e3) / 1e9
-    roof = {"bound": "hbm", "kernel": f"{kname} (fine-grid Gauss-Seidel colour pass, pressure multigrid)",
+    roof = {"bound": "hbm", "kernel": f"{kname} ({what})",
             "achieved": round(ach_cold, 1), "peak": peak, "unit": "GB/s", "frac": round(ach_cold / peak, 4),
             "peak_source": peak_src, "traffic": traffic_per_launch(kname), "bytes_per_launch": k_bytes,
             "avg_launch_us": round(kc_ms * 1e3, 2), "timing": "cold L2 (256 MB written before each launch)",
             "warm": {"avg_launch_us": round(k_ms * 1e3, 2), "achieved": round(k_bytes / (k_ms / 1e3) / 1e9, 1),
                      "frac": round(k_bytes / (k_ms / 1e3) / 1e9 / peak, 4),
-                     "timing": "back-to-back launches, L2-resident as inside a V-cycle"},
+                     "timing": "back-to-back launches"},
             "step": roof_step[args.precision]}
     sp_ms, sp_bytes = s.time_kernel("spmv_p", reps=50)
     spmv = {"achieved_gbs": round(sp_bytes / (sp_ms / 1e3) / 1e9, 1), "avg_launch_us": round(sp_ms * 1e3, 2),

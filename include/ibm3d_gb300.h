@@ -60,14 +60,18 @@ void IBMSolver_set_smagorinsky(IBMSolver *, double Cs);
    default) keeps the reference's ||r||/||b|| < tol rule. */
 void IBMSolver_set_div_tol(IBMSolver *, double div_tol);
 
-/* Arithmetic of the linear solves.  IBM3D_FP64 (default): FP64 BiCGSTAB
-   with an FP64 multigrid preconditioner, as the reference.  IBM3D_MIXED:
-   FP64 iterative refinement (residuals, updates and the stopping test in
-   FP64, on the exact FP64 rows) around FP32 BiCGSTAB solves with an FP32
-   multigrid preconditioner; it stops on the same FP64 criterion.
-   IBM3D_MIXED_MG: momentum as IBM3D_MIXED; the pressure solve is FP64
-   BiCGSTAB whose preconditioner is the FP32 multigrid V-cycle (input
-   rounded to FP32, output widened to FP64).  In these three modes every
+/* Arithmetic of the linear solves.  Momentum: Jacobi sweeps in FP64 (the
+   two `32` modes: FP32) where the diffusion numbers are small, else Krylov
+   solves.  Pressure: BiCGSTAB preconditioned (PRECOND_AMG) by a fast
+   diagonalisation of the rows without the body, with sweeps near it, or by
+   a geometric multigrid V-cycle (axes past 512 or under 3 cells; FP64 with a
+   large body, or with IBM3D_COARSEN_HALVE and a body).
+   IBM3D_FP64 (default): everything in FP64, as the reference.  IBM3D_MIXED:
+   the pressure by FP64 iterative refinement (residuals, updates and the
+   stopping test in FP64, on the exact FP64 rows) around FP32 BiCGSTAB
+   solves with the FP32 preconditioner; it stops on the same FP64 criterion.
+   IBM3D_MIXED_MG: the pressure solve is FP64 BiCGSTAB with the FP32
+   preconditioner (input rounded to FP32, output widened to FP64).  In these three modes every
    other part of the step stays FP64.
    IBM3D_MIXED32: the explicit stages in FP32 as well - convection and the
    momentum right-hand side, u~ and U* - and the momentum solve in FP32 on
@@ -79,8 +83,8 @@ void IBMSolver_set_div_tol(IBMSolver *, double div_tol);
    from the FP64 step by the FP32 rounding of O(dt) increments (~1e-7
    relative velocity after a few hundred steps); max|div U| is driven to
    the same bound.  IBM3D_MIXED32_IR: the same, with the pressure solved
-   as in IBM3D_MIXED (FP64 refinement around FP32 BiCGSTAB with the FP32
-   multigrid). */
+   as in IBM3D_MIXED (FP64 refinement around preconditioned FP32
+   BiCGSTAB). */
 enum { IBM3D_FP64 = 0, IBM3D_MIXED = 1, IBM3D_MIXED_MG = 2, IBM3D_MIXED32 = 3, IBM3D_MIXED32_IR = 4 };
 void IBMSolver_set_precision(IBMSolver *, int mode);
 
@@ -97,7 +101,8 @@ void IBMSolver_set_graphs(IBMSolver *, int on);
    coarse levels (nuc_pre, nuc_post), sweeps on the coarsest level, and the
    over-relaxation weight of the fine-grid fluid rows (0 < omega < 2;
    defaults 3, 3, 2, 2, 16, 1.0).  Tuning only: the solve still stops on the
-   same residual or divergence test. */
+   same residual or divergence test.  Without effect where the fast
+   diagonalisation preconditions (IBMSolver_set_precision). */
 void IBMSolver_set_multigrid(IBMSolver *, int nu_pre, int nu_post, int nuc_pre, int nuc_post, int coarse_sweeps,
                              double omega);
 
@@ -137,8 +142,8 @@ void IBMSolver_set_pressure_guess(IBMSolver *, int mode);
    projection.  GB300 issues FP64 operations at 1/72 of its FP32 rate:
    the FP64 vectors make the solve FP64-bound, the double-float ones bring
    it near the memory bound.  The preconditioned vectors are the FP32
-   multigrid's output as it comes (FP32 entries); without the multigrid
-   preconditioner (PRECOND_AMG) the vectors stay FP64.  Other precision
+   preconditioner's output as it comes (FP32 entries); without one
+   (PRECOND_AMG) the vectors stay FP64.  Other precision
    modes ignore the setting. */
 enum { IBM3D_PVEC_FP64 = 0, IBM3D_PVEC_DFLOAT = 1 };
 void IBMSolver_set_pressure_vectors(IBMSolver *, int kind);
@@ -164,14 +169,15 @@ void IBMSolver_set_coarsening(IBMSolver *, int mode, double width_ratio);
 
 /* Restart length of SOLVER_GMRES pressure solves (1..32; default 10, the
    reference's KDim).  The GMRES is flexible (it keeps every preconditioned
-   vector), so the FP32 multigrid of the mixed modes may precondition it. */
+   vector), so the FP32 preconditioner of the mixed modes may serve it. */
 void IBMSolver_set_gmres_restart(IBMSolver *, int restart);
 
 /* Autotuner: times `steps` recorded steps of this case, from its current
    state, under each of a fixed set of multigrid sweep configurations
    (fine pre/post, coarse pre/post, coarsest), keeps the fastest (written
    to best[5] when best is not NULL) and returns its milliseconds per step.
-   The solver's state is restored, so the run continues unchanged. */
+   The solver's state is restored, so the run continues unchanged.  The
+   candidates are alike where the multigrid does not precondition. */
 double IBMSolver_autotune(IBMSolver *, int steps, int *best);
 
 /* Mixed path (IBM3D_MIXED): relative tolerance of each FP32 inner solve of
@@ -211,14 +217,14 @@ int IBMSolver_num_ghost_levels(IBMSolver *);
 typedef struct {
     int iter;               /* solver->iter after the step */
     double time;
-    int iters_u[3];         /* BiCGSTAB iterations, momentum components */
+    int iters_u[3];         /* momentum components: sweeps, plus BiCGSTAB iterations where those ran */
     int iters_p;            /* BiCGSTAB iterations, pressure */
     double res_u[3];        /* final relative residual norms */
     double res_p;
     double max_div;         /* max |div U^{n+1}| over fluid cells (pinned cell excluded) */
-    int mg_levels;          /* pressure multigrid levels (incl. the fine grid) */
+    int mg_levels;          /* pressure multigrid levels this grid has (incl. the fine grid) */
     int cpt_fallback;       /* level-set points settled by the full extrusion scan */
-    int outer_u;            /* refinement cycles of the momentum solve (IBM3D_MIXED) */
+    int outer_u;            /* refinement cycles of the momentum solve (IBM3D_MIXED, where no sweeps serve it) */
     int outer_p;            /* refinement cycles of the pressure solve (IBM3D_MIXED) */
     /* Totals over every step since IBMSolver_assemble (averages over a run
        are differences of two reads). */
@@ -238,7 +244,8 @@ double IBMSolver_time_iterate(IBMSolver *, int nsteps);
    in the current precision: the average over reps launches between CUDA
    events on the solver's stream (ms), and its algorithmic bytes per launch
    in *bytes (for a roofline).  IBM3D_K_MG_COLOR: one colour pass of the
-   pressure multigrid's fine-grid smoother; IBM3D_K_SPMV_P: one pressure
+   pressure multigrid's fine-grid smoother (built for the measurement where
+   it does not precondition); IBM3D_K_SPMV_P: one pressure
    operator application (both on scratch vectors of the pressure solve).
    IBM3D_K_CONV_RHS, IBM3D_K_USTAR_PRHS, IBM3D_K_UPDATE_NEXT: the step's
    explicit kernels of the current mode (FP64, or the FP32 stages of
