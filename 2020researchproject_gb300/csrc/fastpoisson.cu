@@ -320,7 +320,7 @@ struct FpBack {
 };
 
 template <typename T, int TM, bool ROWS, bool FOLD, typename S>
-__global__ void __launch_bounds__(64, sizeof(T) == 4 && TM == 64 && !ROWS ? 6 : 1)
+__global__ void __launch_bounds__(64, sizeof(T) == 4 && TM == 64 ? 6 : 0)
 k_fp_back(const FpBack<T> p, const FpScatter<T, S> sc, const int *gate) {
     FP_GATE(gate);
     using Tile = FpTile<T, TM>;

@@ -189,7 +189,7 @@ k_bicg_init(const long long n, const B *__restrict__ b, T *x, T *r, KScal *sc, d
 
 // ------------------------------------------------- p = r + beta (p - w v) --
 template <typename T, int NC, bool VEC>
-__global__ void __launch_bounds__(KTHREADS, NC == 1 ? 4 : 1)
+__global__ void __launch_bounds__(KTHREADS, NC == 1 ? 4 : 3)
 k_bicg_p(const long long n, const T *__restrict__ r, T *__restrict__ p, const T *__restrict__ v, T *__restrict__ r0,
          const KScal *sc) {
     pdl_enter();
@@ -468,7 +468,7 @@ k_bicg_spmv_v(const OpT<T> A, const int op, const long long n, const typename Pr
 
 // ------------------------------------------------------- s = r - alpha v --
 template <typename T, int NC, bool VEC>
-__global__ void __launch_bounds__(KTHREADS, NC == 1 ? 4 : 1)
+__global__ void __launch_bounds__(KTHREADS, NC == 1 ? 4 : 3)
 k_bicg_s(const OpT<T> A, const long long n, const T *__restrict__ r, const T *__restrict__ v, T *__restrict__ s,
          KScal *sc, double *partials, unsigned int *counter) {
     pdl_enter();
@@ -590,7 +590,7 @@ k_bicg_spmv_t(const OpT<T> A, const int op, const long long n, const typename Pr
 // Ends the iteration: sets the loop condition (some component still
 // running and below maxit).
 template <typename T, int NC, bool VEC>
-__global__ void __launch_bounds__(KTHREADS, NC == 1 ? 4 : 1)
+__global__ void __launch_bounds__(KTHREADS, NC == 1 ? 4 : 3)
 k_bicg_xr(const OpT<T> A, const long long n, T *__restrict__ x, T *__restrict__ r, const T *__restrict__ r0,
           const typename PrecT<T>::type *__restrict__ ph, const typename PrecT<T>::type *__restrict__ sh,
           const T *__restrict__ s, const T *__restrict__ t,
