@@ -516,18 +516,16 @@ __global__ void __launch_bounds__(MAXT)
 k_fp_tri(const T *__restrict__ iv, const T *__restrict__ km, const T *__restrict__ kp,
          const int n, const long long st, const long long outer, const int ld, const FpPin<T> pin, const T *fin,
          T *out, const int *gate) {
-    FP_GATE(gate);
     __shared__ T sa[32][33], sh[32][33];
     const int c = blockIdx.x * 32 + threadIdx.x, seg = threadIdx.y, ns = blockDim.y;
     const long long base = blockIdx.y * outer + min(c, ld - 1);
     const int i0 = seg * FP_SEG;
     T h[FP_SEG], v[FP_SEG];
 #pragma unroll
-    for (int q = 0; q < FP_SEG; q++) {
-        const bool ok = i0 + q < n;
-        h[q] = ok ? fin[base + (i0 + q) * st] : (T)0;
-        v[q] = ok ? iv[base + (i0 + q) * st] : (T)0;
-    }
+    for (int q = 0; q < FP_SEG; q++) v[q] = i0 + q < n ? iv[base + (i0 + q) * st] : (T)0;
+    FP_GATE(gate);
+#pragma unroll
+    for (int q = 0; q < FP_SEG; q++) h[q] = i0 + q < n ? fin[base + (i0 + q) * st] : (T)0;
     if (pin.singular) {
         const T cc = fp_pin(pin, fin, n, st, &sa[0][0]);
         if (seg == 0) h[0] += cc * pin.f1[blockIdx.y] * pin.f2[min(c, ld - 1)];
@@ -639,21 +637,17 @@ __global__ void __launch_bounds__(256)
 k_fp_edges(const OpT<T> c, const S *__restrict__ r, T *z, const int *__restrict__ outer, const int nout,
            const int *__restrict__ solid, const int nsolid, const int *__restrict__ cell, const T *__restrict__ val,
            const int ncell, const int *gate) {
+    const int t = blockIdx.x * 256 + threadIdx.x, ts = t - nout, tc = ts - nsolid;
+    const int own = t < nout ? outer[t] : ts < nsolid ? solid[ts] : tc < ncell ? cell[tc] : -1;
     FP_GATE(gate);
-    int t = blockIdx.x * 256 + threadIdx.x;
+    if (own < 0) return;
     if (t >= nout) {
-        t -= nout;
-        if (t < nsolid) {
-            const int P = solid[t];
-            z[P] = fp_value<T, S>(r[P]);
-        } else if (t - nsolid < ncell) {
-            z[cell[t - nsolid]] = val[t - nsolid];
-        }
+        z[own] = ts < nsolid ? fp_value<T, S>(r[own]) : val[tc];
         return;
     }
     long long chain[3];
     int face[3], layer[3], n = 0;
-    long long Q = outer[t];
+    long long Q = own;
     while (true) {
         int i, j, k, L;
         cijk_fast(c.g, c.fdx, c.fdy, Q, i, j, k);
@@ -679,7 +673,7 @@ k_fp_edges(const OpT<T> c, const S *__restrict__ r, T *z, const int *__restrict_
         else
             v = rv + v;
     }
-    z[outer[t]] = v;
+    z[own] = v;
 }
 
 // Sweeps over the cells near the body: an overlapping Schwarz step.  The
@@ -692,8 +686,9 @@ k_fp_edges(const OpT<T> c, const S *__restrict__ r, T *z, const int *__restrict_
 // which k_fp_edges writes to z.  (Sweeps over all the cells at once with a
 // barrier per pass, across the blocks of a cluster or as launches, spend 3-4
 // us per pass on the L2 round trip; rows read again from L1 in every pass
-// made an application of boxes 95x61x47 62 us, in registers PATCHN.)  Bound
-// by latency: one load of the rows, FP_SWEEPS x 4 block barriers.
+// made an application of boxes 95x61x47 62 us, in registers 56.)  Bound by
+// latency: FP_SWEEPS x 4 block barriers; the tables' chain of loads runs
+// before the wait for the predecessor.
 constexpr int FP_PT = 512;               // threads of a patch block
 constexpr int FP_PU = 3;                 // cells per thread
 constexpr int FP_PMAX = FP_PT * FP_PU;   // cells of a patch, overlap included
@@ -702,32 +697,47 @@ template <typename T, typename S>
 __global__ void __launch_bounds__(FP_PT)
 k_fp_patch(const FpPatches<T> p, const S *__restrict__ r, const T *__restrict__ z, T *__restrict__ out,
            const int sweeps, const int *gate) {
-    FP_GATE(gate);
     __shared__ T v[FP_PMAX];
     const int b = blockIdx.x, s0 = p.start[b], nr = p.count[3 * b], nf = nr + p.count[3 * b + 1];
     const int n = nf + p.count[3 * b + 2];
     T w[FP_PU][8], f[FP_PU], self[FP_PU];
-    int m[FP_PU][8], own[FP_PU];
+    int m[FP_PU][8], own[FP_PU], P[FP_PU];
+    // The tables, before the wait for the values.
 #pragma unroll
     for (int u = 0; u < FP_PU; u++) {
         const int q = u * FP_PT + threadIdx.x;
         own[u] = -1;
+        P[u] = -1;
         if (q >= n) continue;
         own[u] = p.loc[s0 + q];
-        const int c = own[u] < 0 ? ~own[u] : own[u], P = p.P[c];
-        v[q] = z[P];
+        const int c = own[u] < 0 ? ~own[u] : own[u];
+        P[u] = p.P[c];
         self[u] = p.self[s0 + q];
-        f[u] = p.rw[s0 + q] * fp_value<T, S>(r[P]);
+        f[u] = p.rw[s0 + q];
 #pragma unroll
         for (int e = 0; e < 8; e++) {
             w[u][e] = p.w[(size_t)e * p.nloc + s0 + q];
             m[u][e] = p.ref[(size_t)e * p.nloc + s0 + q];
-            if (m[u][e] < 0) {   // outside the patch, or no coupling
-                const int Q = p.to[e * p.ncell + c];
-                if (Q >= 0) f[u] += w[u][e] * z[Q];
-                w[u][e] = 0;
-                m[u][e] = q;
+            if (m[u][e] < 0) m[u][e] = ~p.to[e * p.ncell + c];   // outside: ~its index; 0: no coupling
+            else m[u][e]++;                                       // inside: its place + 1
+        }
+    }
+    FP_GATE(gate);
+#pragma unroll
+    for (int u = 0; u < FP_PU; u++) {
+        const int q = u * FP_PT + threadIdx.x;
+        if (P[u] < 0) continue;
+        v[q] = z[P[u]];
+        f[u] *= fp_value<T, S>(r[P[u]]);
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            if (m[u][e] > 0) {
+                m[u][e]--;
+                continue;
             }
+            if (m[u][e] < 0) f[u] += w[u][e] * z[~m[u][e]];
+            w[u][e] = 0;
+            m[u][e] = q;
         }
     }
     __syncthreads();
