@@ -1514,7 +1514,7 @@ void FastPoisson<T>::run_tiled(cudaStream_t s, const S *r, T *z, const int *gate
     k += 3;
     if (nghost_ > 0) {
         if (near_outer_) edges(nout, nsolid_, 0);   // the sweeps read outer values
-        launch_pdl(k_fp_patch<T, S>, npatch_, FP_PT, 0, s, patch_, r, (const T *)z, near_val_, FP_SWEEPS, gate);
+        launch_pdl(k_fp_patch<T, S>, npatch_, FP_PT, 0, s, patch_, r, (const T *)z, near_val_, FP_SWEEPS<T>, gate);
         k++;
         if (near_outer_) edges(0, 0, patch_.ncell);
     }

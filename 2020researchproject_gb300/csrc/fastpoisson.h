@@ -26,8 +26,8 @@
 // Measured (GB300, per application and BiCGSTAB iterations per step, against
 // the multigrid V-cycle that served these cases before): channel
 // 128x96x128 FP32 0.09 ms, 1 iteration (0.47 ms, 14); cavity 64^3 FP64
-// 0.17 ms, 1 (0.31 ms, 10); sphere 192x128x128 FP32 0.14 ms, 3.4 (0.53 ms,
-// 3.9); boxes 95x61x47 FP32 0.062 ms, 4.8 (0.25 ms, 4.9).
+// 0.17 ms, 1 (0.31 ms, 10); sphere 192x128x128 FP32 0.13 ms, 3.1 (0.53 ms,
+// 3.9); boxes 95x61x47 FP32 0.05 ms, 4.4 (0.25 ms, 4.9).
 #pragma once
 
 #include <vector>
@@ -69,11 +69,14 @@ struct FpModes {
 // The cells near the body, cut into patches (k_fp_patch).  Pressure
 // iterations per step with 2, 3, 5, 8 and 16 sweeps: sphere 192x128x128 3.7,
 // 3.5, 3.35, 3.35, 3.15; boxes 95x61x47 6.2, 6.0, 5.35, 4.75, 4.4; the
-// twelve-case ensemble 5.75, 5.0, 4.5, 3.9, 3.8, at 1 us of an application
-// per 3 sweeps: 8 is the fastest step everywhere.  Thinner or thicker layers
-// and overlaps are within 3 %.
+// twelve-case ensemble 5.75, 5.0, 4.5, 3.9, 3.8.  Sweeps of a patch: 16 in
+// FP32, whose sweep is barriers (8 against 16, ms for 20 steps: boxes 20.1,
+// 19.4; sphere 256x128x128, 15 steps, 54.0, 51.9; the others equal), 8 in
+// FP64, whose sweep is arithmetic (boxes 64x48x40, 4 steps: 13.3, 14.3).
+// Thinner or thicker layers and overlaps are within 3 %.
 constexpr int FP_LAYERS = 3;     // fluid layers around the ghosts
-constexpr int FP_SWEEPS = 8;     // sweeps of a patch
+template <typename T>
+constexpr int FP_SWEEPS = sizeof(T) == 4 ? 16 : 8;
 // Side of the cubes the cells are cut by, and the cells a patch takes beyond
 // them.  FP64, bound by each SM's two multiply-adds per clock: more and
 // smaller patches (boxes 64x48x40: 3.38 ms per step, with FP32's sizes 3.75);
