@@ -1726,8 +1726,12 @@ k_mom_sweep(const OpT<T> A, const long long n, const T *__restrict__ b, const T 
             all = all && ok;
             finite = finite && isfinite(s.rn2[c]);
         }
+        // The first sweep leaves a complete x when it ends the solve: MODE 1 by
+        // its own row pass (always), MODE 2 untouched.  A later row pass into
+        // x (ends) would read a second buffer no sweep of this solve wrote.
+        const bool in_progress = MODE == 0 && into_first;
         if (all) {
-            s.state = MODE == 1 || into_first ? MS_B : MS_A;
+            s.state = in_progress ? MS_B : MS_A;
             for (int c = 0; c < 3; c++) {
                 KScal &q = sc[c];
                 q.bnorm2 = s.bn2[c];
@@ -1737,7 +1741,7 @@ k_mom_sweep(const OpT<T> A, const long long n, const T *__restrict__ b, const T 
                 q.divmax = 0.0;
             }
         } else if (s.sweeps >= limit || !finite) {
-            s.state = into_first ? MS_FALL_B : MS_FALL;
+            s.state = in_progress ? MS_FALL_B : MS_FALL;
         }
         if (s.state != MS_A && s.state != MS_FALL) s.sweeps++;
         set_loop(lc, s.state == MS_RUN);
