@@ -629,7 +629,9 @@ __global__ void k_fp_sums(const double *__restrict__ l0, const double *__restric
 // Outer rows solved for the outer values, each through its chain of
 // partners down to an interior cell (as the multigrid's outer pass), the
 // identity rows of solid cells, and the swept values of the cells near the
-// body (cell[q] takes val[q]).  The three lists touch different cells; a
+// body (cell[q] takes val[q]).  The three lists write different cells, and no
+// outer row reads a cell that another thread of the launch writes: a partner
+// that is solid gives its residual, the value its identity row takes, and a
 // body whose swept cells are partners of outer rows gets its outer rows in
 // a launch of their own.
 template <typename T, typename S>
@@ -664,7 +666,7 @@ k_fp_edges(const OpT<T> c, const S *__restrict__ r, T *z, const int *__restrict_
             Q += (2 * L - 1) * (face_low(f) ? s : -s);
         }
     }
-    T v = z[Q];
+    T v = nsolid > 0 && c.flag[Q] == SOLID ? fp_value<T, S>(r[Q]) : z[Q];
     for (int q = n - 1; q >= 0; q--) {
         const BCRow<T> &F = c.bc[face[q]];
         const T rv = fp_value<T, S>(r[chain[q]]);
