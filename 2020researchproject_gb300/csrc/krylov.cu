@@ -170,7 +170,7 @@ k_bicg_init(const long long n, const B *__restrict__ b, T *x, T *r, KScal *sc, d
             s.alpha = 1.0;
             s.omega = 1.0;
             s.beta = 0.0;
-            s.iters = 0;
+            s.iters = s.before = 0;
             s.state = tot[c] == 0.0 ? KS_DONE : KS_RUN;
             s.divmax = 0.0;
             s.restart = 1;   // the first p update sets p = r0 = r
@@ -334,7 +334,8 @@ __device__ __forceinline__ void sweep_pres(const OpT<T> &A, const X *__restrict_
 // the stopping test ends the solve before its first iteration.  b as in
 // k_bicg_init.
 // after (momentum only): the sweeps that came before; when they ended the
-// solve nothing runs, else their count starts the iteration count.  outer
+// solve nothing runs, else their count starts the iteration count (of which
+// maxit are this solve's own).  outer
 // (increment solves): the norms that fix the stopping test, as in
 // k_bicg_init.
 template <typename T, int NC, typename B = T>
@@ -391,7 +392,7 @@ k_bicg_init_guess(const OpT<T> A, const int op, const long long n, const B *__re
             s.alpha = 1.0;
             s.omega = 1.0;
             s.beta = 0.0;
-            s.iters = after ? after->sweeps : 0;
+            s.iters = s.before = after ? after->sweeps : 0;
             s.tol = tol;
             if (outer && outer[c].rnorm2 > 0)
                 s.tol = fmax(tol, 0.5 * outer_tol * sqrt(outer[c].bnorm2 / outer[c].rnorm2));
@@ -400,7 +401,7 @@ k_bicg_init_guess(const OpT<T> A, const int op, const long long n, const B *__re
             s.restart = 1;   // the first p update sets p = r0 = r
             const bool done = tot[NC + c] == 0.0 || converged(tot[NC + c], s.bnorm2, tot[2 * NC], s.tol, divtol);
             s.state = done ? KS_DONE : KS_RUN;
-            go = go || (!done && s.iters < maxit);
+            go = go || (!done && maxit > 0);
         }
         set_loop(lc, go);
     });
@@ -689,7 +690,7 @@ k_bicg_xr(const OpT<T> A, const long long n, T *__restrict__ x, T *__restrict__ 
                 st.rho = tot[2 * c];
                 st.beta = 0.0;
             }
-            run = run || (st.state == KS_RUN && st.iters < maxit);
+            run = run || (st.state == KS_RUN && st.iters - st.before < maxit);
         }
         set_loop(lc, run);
     });
@@ -1903,7 +1904,7 @@ int solve_sweeps(cudaStream_t st, const OpT<T> &A, MomSweep &ms, KrylovWork<T> &
     k += launch_end(st, A, ms, w, b, x, prm, ir, none);
     note_launches(k);
     if (h.state == MS_A || h.state == MS_B) fetch(st, w);
-    else host_loop<T>(st, A, OP_MOM, w, x, std::max(0, prm.maxit - h.sweeps), nullptr, prm.prof);
+    else host_loop<T>(st, A, OP_MOM, w, x, prm.maxit, nullptr, prm.prof);
     return report(w, rep);
 }
 

@@ -48,7 +48,8 @@ struct KScal {
     double rho, alpha, omega, beta;
     double divmax;
     double tol, divtol;  // this solve's stopping test (set by the init kernel)
-    int iters;
+    int iters;     // sweeps that came before (momentum) included
+    int before;    // those sweeps
     int state;
     int restart;   // the next p update restarts the recurrence (r0 = r, p = r)
 };

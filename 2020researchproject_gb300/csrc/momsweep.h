@@ -12,8 +12,8 @@
 // bytes and gains about what two sweeps do.
 //
 // With rho above MS_RHO, or where the sweeps reach their limit, BiCGSTAB
-// takes (over) the solve; the stopping test is the same one, on the true
-// residual.  A BiCGSTAB iteration that passes it lands a digit or two below;
+// takes (over) the solve, with the caller's iteration cap for itself; the
+// stopping test is the same one, on the true residual.  A BiCGSTAB iteration that passes it lands a digit or two below;
 // the sweeps stop at the first pass, so their own test is MS_MARGIN of it
 // (down to FP64's rounding), about one sweep more, and the solution is no
 // further from the exact one (64^3 cavity, 200 steps from u^n at 1e-6:

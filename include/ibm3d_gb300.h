@@ -150,6 +150,8 @@ void IBMSolver_set_pressure_vectors(IBMSolver *, int kind);
 
 /* Krylov iteration caps of the momentum and pressure solves (defaults
    200 and 1000, the reference's hypre settings, src/ibm3d_setup.c:1411-1563).
+   Momentum: of the sweeps (at most 60), and again of the Krylov solve that
+   takes over from them.
    A solve that reaches its cap prints the reference's warning
    ("warning: u0_star did not converge", "warning: p_prime did not
    converge") and the step continues, as in the reference. */
