@@ -362,7 +362,8 @@ class IBMSolver:
 
     def set_coarsening(self, mode=COARSEN_SPACING, width_ratio=0.0):
         """Pressure multigrid coarsening (before assemble): COARSEN_SPACING
-        (width_ratio: its merge threshold, 0 = default) or COARSEN_HALVE."""
+        (width_ratio: its merge threshold, 0 = default) or COARSEN_HALVE.
+        The call has the multigrid precondition every pressure solve."""
         self._lib.IBMSolver_set_coarsening(self._s, int(mode), float(width_ratio))
         self._check("set_coarsening")
 

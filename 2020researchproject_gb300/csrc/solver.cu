@@ -163,6 +163,7 @@ struct ibm3d_device {
     int mg_sweeps[5] = {3, 3, 2, 2, 16};  // multigrid sweeps: fine pre/post, coarse pre/post, coarsest
     double mg_omega = 1.0;               // over-relaxation of the fine-grid smoother
     int mg_coarsening = IBM3D_COARSEN_SPACING;
+    bool mg_asked = false;   // the caller set the coarsening: the multigrid serves every solve
     int warm_start = 1;                  // mixed modes: momentum solve from the current velocity
     int maxit_mom = 200, maxit_p = 1000; // Krylov iteration caps (src/ibm3d_setup.c:1411-1432, 1435-1563)
     double mg_width_ratio = 1.5;
@@ -862,7 +863,8 @@ bool build_ops(IBMSolver *sv) {
 // operations per application.  FP64 steps against the multigrid's: boxes
 // 64x48x40 3.6 against 5.0 ms, sphere 96x64x64 4.4 against 7.4, 128x96x96
 // (0.45e9 operations) 9.4 against 14.0, 192x128x128 (1.6e9) 30 against 24.
-// A caller who has the multigrid halve every axis asks for the multigrid.
+// A caller who sets the coarsening (IBMSolver_set_coarsening) asks for the
+// multigrid, in either precision.
 constexpr double kBodyOps = 0.7e9;
 
 bool build_sweeps_and_poisson(IBMSolver *sv) {
@@ -911,8 +913,7 @@ bool build_sweeps_and_poisson(IBMSolver *sv) {
         if (rc < 0) set_status(sv, IBM3D_ECUDA, "preconditioner setup failed");
         return rc >= 0;
     };
-    return make(d->fp32, d->A32, INFINITY) &&
-           make(d->fp64, d->A64, !body ? INFINITY : d->mg_coarsening == IBM3D_COARSEN_HALVE ? 0.0 : kBodyOps);
+    return d->mg_asked || (make(d->fp32, d->A32, INFINITY) && make(d->fp64, d->A64, body ? kBodyOps : INFINITY));
 }
 
 MGGeometry mg_geometry(const IBMSolver *sv) {
@@ -2527,6 +2528,7 @@ void IBMSolver_set_coarsening(IBMSolver *s, int mode, double width_ratio) {
         return;
     }
     s->dev->mg_coarsening = mode;
+    s->dev->mg_asked = true;
     s->dev->mg_width_ratio = width_ratio == 0.0 ? 1.5 : width_ratio;
 }
 
@@ -2698,9 +2700,11 @@ double IBMSolver_time_iterate(IBMSolver *s, int nsteps) {
 // Picks the pressure multigrid's smoother sweeps for this case and
 // arithmetic mode by measurement: from the current state, each candidate
 // runs `steps` recorded steps (after one untimed step that records its
-// graphs) and the fastest wins.  The state (every field a step reads, time
-// and iteration count) is restored after each trial and at the end, so the
-// run continues exactly as if the tuner had not run.
+// graphs) and the fastest wins.  Where another preconditioner serves the
+// solves the sweeps decide nothing: the current setting is timed and kept.
+// The state (every field a step reads, time and iteration count) is restored
+// after each trial and at the end, so the run continues exactly as if the
+// tuner had not run.
 double IBMSolver_autotune(IBMSolver *s, int steps, int *best_out) {
     if (!check_ready(s, "IBMSolver_autotune")) return -1;
     ibm3d_device *d = s->dev;
@@ -2708,7 +2712,8 @@ double IBMSolver_autotune(IBMSolver *s, int steps, int *best_out) {
     static const int cand[][5] = {{5, 5, 1, 1, 8},  {4, 4, 1, 1, 8},  {6, 6, 1, 1, 8},  {3, 3, 1, 1, 8},
                                   {4, 4, 2, 2, 8},  {3, 3, 2, 2, 8},  {5, 5, 2, 2, 16}, {2, 2, 2, 2, 8},
                                   {4, 4, 2, 2, 16}, {6, 6, 2, 2, 16}, {3, 3, 2, 2, 16}, {5, 5, 1, 1, 16}};
-    const int ncand = (int)(sizeof cand / sizeof cand[0]);
+    const bool multigrid = use_mg(s) && !(d->precision == IBM3D_FP64 ? (void *)d->fp64 : (void *)d->fp32);
+    const int ncand = multigrid ? (int)(sizeof cand / sizeof cand[0]) : 1;
     const size_t n = (size_t)d->g.ncell;
     double *save = nullptr;
     if (!cuda_check(s, cudaMalloc(&save, sizeof(double) * (n * kStateFields + 1)), "autotune state")) return -1;
@@ -2732,7 +2737,8 @@ double IBMSolver_autotune(IBMSolver *s, int steps, int *best_out) {
     double best = -1;
     int bi = -1;
     for (int c = 0; c < ncand && d->status != IBM3D_ECUDA; c++) {
-        IBMSolver_set_multigrid(s, cand[c][0], cand[c][1], cand[c][2], cand[c][3], cand[c][4], omega);
+        const int *t = multigrid ? cand[c] : keep;
+        IBMSolver_set_multigrid(s, t[0], t[1], t[2], t[3], t[4], omega);
         copy_state(false);
         s->iter = iter0;
         s->time = time0;
@@ -2749,7 +2755,7 @@ double IBMSolver_autotune(IBMSolver *s, int steps, int *best_out) {
             bi = c;
         }
     }
-    const int *w = bi >= 0 ? cand[bi] : keep;
+    const int *w = multigrid && bi >= 0 ? cand[bi] : keep;
     IBMSolver_set_multigrid(s, w[0], w[1], w[2], w[3], w[4], omega);
     copy_state(false);
     s->iter = iter0;

@@ -65,7 +65,7 @@ void IBMSolver_set_div_tol(IBMSolver *, double div_tol);
    solves.  Pressure: BiCGSTAB preconditioned (PRECOND_AMG) by a fast
    diagonalisation of the rows without the body, with sweeps near it, or by
    a geometric multigrid V-cycle (axes past 512 or under 3 cells; FP64 with a
-   large body, or with IBM3D_COARSEN_HALVE and a body).
+   large body; every solve after IBMSolver_set_coarsening).
    IBM3D_FP64 (default): everything in FP64, as the reference.  IBM3D_MIXED:
    the pressure by FP64 iterative refinement (residuals, updates and the
    stopping test in FP64, on the exact FP64 rows) around FP32 BiCGSTAB
@@ -157,7 +157,9 @@ void IBMSolver_set_pressure_vectors(IBMSolver *, int kind);
    converge") and the step continues, as in the reference. */
 void IBMSolver_set_max_iters(IBMSolver *, int max_mom, int max_p);
 
-/* Coarsening of the pressure multigrid (before IBMSolver_assemble).
+/* Coarsening of the pressure multigrid (before IBMSolver_assemble).  The call,
+   with either mode, also has the multigrid precondition every pressure solve
+   (IBMSolver_set_precision names what does otherwise).
    IBM3D_COARSEN_SPACING (default): a coarse level merges neighbouring
    cells along an axis only while their joint width is at most
    width_ratio x 2^(level+1) x the finest width (width_ratio in [1, 64];
@@ -178,8 +180,8 @@ void IBMSolver_set_gmres_restart(IBMSolver *, int restart);
    state, under each of a fixed set of multigrid sweep configurations
    (fine pre/post, coarse pre/post, coarsest), keeps the fastest (written
    to best[5] when best is not NULL) and returns its milliseconds per step.
-   The solver's state is restored, so the run continues unchanged.  The
-   candidates are alike where the multigrid does not precondition. */
+   The solver's state is restored, so the run continues unchanged.  Where the
+   multigrid does not precondition, the current setting is timed and kept. */
 double IBMSolver_autotune(IBMSolver *, int steps, int *best);
 
 /* Mixed path (IBM3D_MIXED): relative tolerance of each FP32 inner solve of
