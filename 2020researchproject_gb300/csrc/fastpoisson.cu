@@ -894,10 +894,11 @@ FastPoisson<T>::~FastPoisson() {
 }
 
 // The cells near the body, their rows and the patches (k_fp_patch), cut by
-// cubes of side `cube`; false when a patch cannot be made small enough.
+// cubes of side `cube`; false when the cells are more than `most` or a patch
+// cannot be made small enough.
 template <typename T>
 static bool build_patches(const OpT<double> &A, const FastPoissonGeom &h, const std::vector<double> &gw, int cube,
-                          FpPatchTables<T> &t_) {
+                          size_t most, FpPatchTables<T> &t_) {
     const Grid &g = A.g;
     const int n[3] = {g.nx, g.ny, g.nz};
     const long long st[3] = {g.sx, g.sy, 1};
@@ -951,6 +952,7 @@ static bool build_patches(const OpT<double> &A, const FastPoissonGeom &h, const 
         }
         first = last;
     }
+    if (cells.size() > most) return false;
     const int nc = (int)cells.size();
     // Rows: couplings (padded index, weight), weight of the old value and of
     // the residual.  Ghost rows are relaxed as the multigrid relaxes them.
@@ -1101,6 +1103,59 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
         if (n[a] < 3 || (a != tri_ && n[a] > FP_MAX_DENSE)) return 1;
     A_ = A;
     nghost_ = (int)h.gcell.size();
+    // The 1-D problems (diagonal dg, off-diagonals e, wrap couples the ends of
+    // a periodic axis), mirror-symmetric up to the rounding of the face
+    // coordinates, and the transforms' operations.
+    std::vector<double> dg[3], e[3];
+    double wrap[3], ops = 0;
+    for (int a = 0; a < 3; a++) {
+        const int N = n[a];
+        const std::vector<double> &km = h.km[a], &kp = h.kp[a], &d = h.d[a];
+        dg[a].resize(N);
+        for (int i = 0; i < N; i++) dg[a][i] = km[i] + kp[i];
+        if (!per[a]) {
+            const BCRow<double> &L = A64.bc[lo[a]], &U = A64.bc[hi[a]];
+            dg[a][0] += dirichlet_face(L.type) ? km[0] * (L.dir_m[0] / L.dir_o[0]) : -km[0];
+            dg[a][N - 1] += dirichlet_face(U.type) ? kp[N - 1] * (U.dir_m[0] / U.dir_o[0]) : -kp[N - 1];
+        }
+        if (a == tri_) continue;
+        e[a].assign(N, 0.0);
+        for (int i = 0; i + 1 < N; i++) e[a][i] = -std::sqrt(kp[i] * km[i + 1]);
+        wrap[a] = per[a] ? -std::sqrt(km[0] * kp[N - 1]) : 0.0;
+        auto near_ = [](double x, double y) { return std::fabs(x - y) <= 1e-11 * (std::fabs(x) + std::fabs(y)); };
+        bool sym = true;
+        for (int i = 0; i < N; i++) sym = sym && near_(d[i], d[N - 1 - i]) && near_(dg[a][i], dg[a][N - 1 - i]);
+        for (int i = 0; i + 1 < N; i++) sym = sym && near_(e[a][i], e[a][N - 2 - i]);
+        FpModes &m = modes_[a];
+        m.fold = sym;
+        m.no = sym ? N / 2 : 0;
+        m.ne = N - m.no;
+        // Columns of the odd modes start on a vector boundary along z.
+        m.off = a == 2 ? (m.ne + 3) & ~3 : m.ne;
+        m.ld = a == 2 ? m.off + ((m.no + 3) & ~3) : N;
+        ops += 4.0 * n[0] * n[1] * n[2] * m.ne;
+    }
+    if (ops > max_ops) return 1;
+    std::vector<int> solid;
+    size_t fluid = 0;
+    for (int i = 0; i < n[0]; i++)
+        for (int j = 0; j < n[1]; j++) {
+            const long long P0 = cidx(g, i, j, 0);
+            for (int k = 0; k < n[2]; k++) {
+                if (h.flag[P0 + k] == SOLID) solid.push_back((int)(P0 + k));
+                else fluid += h.flag[P0 + k] == FLUID;
+            }
+        }
+    nsolid_ = (int)solid.size();
+    FpPatchTables<T> t;
+    if (nghost_ > 0) {
+        std::vector<double> gw(8 * (size_t)nghost_);
+        cudaMemcpyAsync(gw.data(), A64.gw, sizeof(double) * gw.size(), cudaMemcpyDeviceToHost, s);
+        if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
+        const bool large = (long long)n[0] * n[1] * n[2] > FP_NEAR_GRID<T>;
+        const size_t most = large ? (size_t)(FP_NEAR * (double)fluid) : (size_t)g.ncell;
+        if (!build_patches(A64, h, gw, FP_CUBE<T>, most, t)) return 1;
+    }
     bool ok = true;
     // Device arrays from chunks (an allocation each would be most of the
     // set-up of a small case).  A copy from pageable memory has read its
@@ -1122,36 +1177,14 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
         if (src && bytes) ok = cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess;
         return p;
     };
-    std::vector<double> lam[3], diag;
+    std::vector<double> lam[3];
     std::vector<T> row0[3], v0;
     for (int a = 0; a < 3 && ok; a++) {
+        if (a == tri_) continue;
         const int N = n[a];
-        const std::vector<double> &km = h.km[a], &kp = h.kp[a], &d = h.d[a];
-        std::vector<double> dg(N), e(N, 0.0);
-        for (int i = 0; i < N; i++) dg[i] = km[i] + kp[i];
-        if (!per[a]) {
-            const BCRow<double> &L = A64.bc[lo[a]], &U = A64.bc[hi[a]];
-            dg[0] += dirichlet_face(L.type) ? km[0] * (L.dir_m[0] / L.dir_o[0]) : -km[0];
-            dg[N - 1] += dirichlet_face(U.type) ? kp[N - 1] * (U.dir_m[0] / U.dir_o[0]) : -kp[N - 1];
-        }
-        if (a == tri_) {
-            diag = dg;
-            continue;
-        }
-        for (int i = 0; i + 1 < N; i++) e[i] = -std::sqrt(kp[i] * km[i + 1]);
-        const double wrap = per[a] ? -std::sqrt(km[0] * kp[N - 1]) : 0.0;   // couples cells 0 and N - 1
-        // Mirror symmetry, up to the rounding of the face coordinates.
-        auto near_ = [](double x, double y) { return std::fabs(x - y) <= 1e-11 * (std::fabs(x) + std::fabs(y)); };
-        bool sym = true;
-        for (int i = 0; i < N; i++) sym = sym && near_(d[i], d[N - 1 - i]) && near_(dg[i], dg[N - 1 - i]);
-        for (int i = 0; i + 1 < N; i++) sym = sym && near_(e[i], e[N - 2 - i]);
+        const std::vector<double> &d = h.d[a];
         FpModes &m = modes_[a];
-        m.fold = sym;
-        m.no = sym ? N / 2 : 0;
-        m.ne = N - m.no;
-        // Columns of the odd modes start on a vector boundary along z.
-        m.off = a == 2 ? (m.ne + 3) & ~3 : m.ne;
-        m.ld = a == 2 ? m.off + ((m.no + 3) & ~3) : N;
+        const bool sym = m.fold != 0;
         lam[a].assign(m.ld, __builtin_nan(""));
         row0[a].assign(m.ld, (T)0);
         if (a == 2) v0.assign(m.ld, (T)0);
@@ -1163,22 +1196,22 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
             if (!sym && per[a]) {
                 std::vector<double> f((size_t)N * N, 0.0);
                 for (int i = 0; i < N; i++) {
-                    f[(size_t)i * N + i] = dg[i];
-                    if (i + 1 < N) f[(size_t)i * N + i + 1] = f[(size_t)(i + 1) * N + i] = e[i];
+                    f[(size_t)i * N + i] = dg[a][i];
+                    if (i + 1 < N) f[(size_t)i * N + i + 1] = f[(size_t)(i + 1) * N + i] = e[a][i];
                 }
-                f[N - 1] = f[(size_t)(N - 1) * N] = wrap;
+                f[N - 1] = f[(size_t)(N - 1) * N] = wrap[a];
                 good = dense_eigen(N, f, w, q);
             } else {
                 // On vectors even (odd) about the middle: the first half's
                 // rows, the couplings to the mirrored half folded in.
                 for (int i = 0; i < H; i++) {
-                    w[i] = sym ? (dg[i] + dg[N - 1 - i]) / 2 : dg[i];
-                    if (i + 1 < H) eh[i] = sym ? (e[i] + e[N - 2 - i]) / 2 : e[i];
+                    w[i] = sym ? (dg[a][i] + dg[a][N - 1 - i]) / 2 : dg[a][i];
+                    if (i + 1 < H) eh[i] = sym ? (e[a][i] + e[a][N - 2 - i]) / 2 : e[a][i];
                 }
                 if (sym) {
                     const double sg = odd ? -1.0 : 1.0;
-                    w[0] += sg * wrap;
-                    if (N % 2 == 0) w[H - 1] += sg * e[N / 2 - 1];
+                    w[0] += sg * wrap[a];
+                    if (N % 2 == 0) w[H - 1] += sg * e[a][N / 2 - 1];
                     else if (!odd) eh[H - 2] *= std::sqrt(2.0);
                 }
                 q.assign((size_t)H * H, 0.0);
@@ -1211,10 +1244,6 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
         if (A.p_singular) lam[a][zero_[a]] = 0.0;   // the constants
         row0_[a] = (T *)put(row0[a].data(), sizeof(T) * row0[a].size());
     }
-    double ops = 0;
-    for (int a = 0; a < 3; a++)
-        if (a != tri_) ops += 4.0 * n[0] * n[1] * n[2] * modes_[a].ne;
-    if (ops > max_ops) return 1;
     ld_ = modes_[2].ld;
     v0_ = (T *)put(v0.data(), sizeof(T) * v0.size());
     const size_t cells = (size_t)n[0] * n[1] * ld_;
@@ -1231,7 +1260,7 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
     if (!ok) return -1;
     if (tri_ >= 0) {
         const int N = n[tri_], o = tri_ == 0 ? 1 : 0;
-        dk[0] = tmp(diag);
+        dk[0] = tmp(dg[tri_]);
         dk[1] = tmp(h.km[tri_]);
         dk[2] = tmp(h.kp[tri_]);
         std::vector<T> w(N);
@@ -1253,24 +1282,11 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
         k_fp_sums<T><<<dim3((ld_ + 127) / 128, n[1], n[0]), 128, 0, s>>>(dl[0], dl[1], dl[2], inv_, n[1], ld_,
                                                                          sing ? zero_[0] : -1, zero_[1], zero_[2]);
     }
-    std::vector<int> solid;
-    for (int i = 0; i < n[0]; i++)
-        for (int j = 0; j < n[1]; j++) {
-            const long long P0 = cidx(g, i, j, 0);
-            for (int k = 0; k < n[2]; k++)
-                if (h.flag[P0 + k] == SOLID) solid.push_back((int)(P0 + k));
-        }
-    nsolid_ = (int)solid.size();
     solid_ = (int *)put(solid.data(), sizeof(int) * solid.size());
     if (nghost_ > 0) {
-        std::vector<double> gw(8 * (size_t)nghost_);
-        cudaMemcpyAsync(gw.data(), A64.gw, sizeof(double) * gw.size(), cudaMemcpyDeviceToHost, s);
-        if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
         std::vector<T> sc(nghost_);
         for (int q = 0; q < nghost_; q++) sc[q] = (T)(1.0 / std::max(1.0 - h.gwself[q], 1e-3));
         gscale_ = (T *)put(sc.data(), sizeof(T) * nghost_);
-        FpPatchTables<T> t;
-        if (!build_patches(A64, h, gw, FP_CUBE<T>, t)) return 1;
         auto ints = [&](const std::vector<int> &v) { return (const int *)put(v.data(), sizeof(int) * v.size()); };
         auto reals = [&](const std::vector<T> &v) { return (const T *)put(v.data(), sizeof(T) * v.size()); };
         npatch_ = (int)t.start.size();

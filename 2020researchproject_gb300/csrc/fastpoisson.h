@@ -1,5 +1,6 @@
 // Fast diagonalisation of the pressure-Poisson rows: the BiCGSTAB
-// preconditioner of the mixed modes, and of FP64 solves without a body.
+// preconditioner of the mixed modes, and of FP64 solves without a body or
+// with transforms of few operations.
 //
 // Without a body the fluid rows are separable: coeffsum times the
 // normalised row is Ax + Ay + Az with one tridiagonal (periodic axes:
@@ -57,6 +58,24 @@ struct FastPoissonGeom {
 constexpr int FP_MAX_DENSE = 512, FP_MAX_TRI = 512;
 constexpr int FP_SEG = 16;   // rows of the tridiagonal axis per thread
 
+// A body is left to the multigrid where the cells near it (FP_LAYERS) are
+// more than FP_NEAR of the fluid ones on a grid of more than FP_NEAR_GRID
+// cells: the solve that ignores the body is then exact hardly anywhere, and
+// takes up to 1.8 times the multigrid's iterations.  On smaller grids the
+// multigrid's launches are short of work.  ms per step against the multigrid's,
+// near cells over fluid ones in brackets.  FP64: a square duct in a solid
+// block 48x32x32 (1.0) 2.2, 3.2; 64x40x40 (0.9) 4.5, 3.8; 72x48x48 (0.8) 5.5,
+// 4.5; 144x72x72 (0.5) 15.7, 8.2; three baffles 48x32x32 (0.42) 3.3, 4.7;
+// 96x48x48 (0.24) 9.3, 7.5; 144x72x72 (0.154) 28, 16; 18 square tubes 64x40x40
+// (0.6) 3.9, 4.8; 96x48x48 (0.5) 6.4, 5.6; a slit 72x48x48 (0.13) 5.1, 6.2;
+// two boxes 96x48x48 (0.08) 3.9, 4.5.  FP32: duct 120x64x64 (0.6) 2.3, 2.9;
+// 192x96x96 (0.4) 5.7, 4.9; tubes 120x64x64 (0.4) 3.8, 3.8; 192x96x96 (0.3)
+// 7.8, 6.9; baffles 120x64x64 (0.19) 4.6, 6.4; 144x72x72 (0.154) 9.3, 8.6;
+// 192x96x96 (0.12) 11.9, 12.4; a slit 192x96x96 (0.05) 5.9, 7.1.
+constexpr double FP_NEAR = 0.14;
+template <typename T>
+constexpr long long FP_NEAR_GRID = sizeof(T) == 4 ? 600000 : 131072;
+
 // Modes of a transformed axis.  fold: the axis is mirror-symmetric, its
 // modes split into ne even and no odd ones; otherwise all n are in the
 // first part.  The second part starts at off (along z: a column on a vector
@@ -105,7 +124,8 @@ class FastPoisson : public Preconditioner<T> {
   public:
     ~FastPoisson() override;
     // 0: ready; 1: not for this case (the multigrid serves it: an axis is too
-    // long, or the transforms take more than max_ops operations); -1: error.
+    // long, the transforms take more than max_ops operations, or the body is
+    // near too many cells); -1: error.
     int setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &A, const FastPoissonGeom &h, double max_ops);
     void apply(cudaStream_t s, const T *r, T *z, const int *gate) override;
     bool apply_from64(cudaStream_t s, const double *r, T *z, const int *gate) override;

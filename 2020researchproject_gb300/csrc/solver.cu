@@ -857,15 +857,22 @@ bool build_ops(IBMSolver *sv) {
 }
 
 // Tables of the momentum sweeps (momsweep.h), and the fast-diagonalisation
-// preconditioners (fastpoisson.h): in FP32 for every case its axes allow; in
-// FP64, where the transforms are bound by the FP64 pipe, always without a
-// body (one iteration instead of 5-18) and with one up to kBodyOps
-// operations per application.  FP64 steps against the multigrid's: boxes
-// 64x48x40 3.6 against 5.0 ms, sphere 96x64x64 4.4 against 7.4, 128x96x96
-// (0.45e9 operations) 9.4 against 14.0, 192x128x128 (1.6e9) 30 against 24.
+// preconditioners (fastpoisson.h) of the pressure solves that their axes and
+// the body (FP_NEAR) allow: in FP32 all of them; in FP64, where the transforms
+// are bound by the FP64 pipe, always without a body (one iteration instead of
+// 5-18) and with one up to kBodyOps operations per application.  FP64 steps
+// against the multigrid's (ms): boxes 64x48x40 2.8, 3.9; 95x61x47 4.6, 5.0;
+// sphere 96x64x64 (0.10e9 operations) 3.1, 5.2; 120x96x88 (0.37e9) 6.3, 9.3;
+// 128x96x96 (0.45e9) 6.8, 9.3; four kinds of boxes 128x96x96 10.3-11.2,
+// 11.5-12.2; a sphere on asymmetric axes 112x80x80 (0.46e9) 6.3, 7.8; sphere
+// 136x100x100 (0.54e9) 11.1, 10.7; boxes 17.8, 12.7; sphere 144x104x104
+// (0.65e9) 13.4, 10.9; asymmetric 128x96x96 (0.91e9) 10.4, 9.7; 192x128x128
+// (1.6e9) 21, 15.  FP32 is faster up to the largest measured, asymmetric axes
+// (twice the operations) included: spheres 256^3 16-19 against 31-33,
+// 512x256x256 34-45, 68-86, cavities 384^3 27-31, 115-273.
 // A caller who sets the coarsening (IBMSolver_set_coarsening) asks for the
 // multigrid, in either precision.
-constexpr double kBodyOps = 0.7e9;
+constexpr double kBodyOps = 0.5e9;
 
 bool build_sweeps_and_poisson(IBMSolver *sv) {
     ibm3d_device *d = sv->dev;
