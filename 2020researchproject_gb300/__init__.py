@@ -481,7 +481,7 @@ class IBMSolver:
                     outer_p_total=st.outer_p_total, max_div_max=st.max_div_max)
 
     def device_bytes(self):
-        """Device memory taken by assembly (bytes)."""
+        """Device memory taken by assembly and the preconditioners set up so far (bytes)."""
         return int(self._lib.IBMSolver_device_bytes(self._s))
 
     def set_profiling(self, on=True):

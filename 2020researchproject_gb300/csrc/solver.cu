@@ -126,6 +126,7 @@ struct ibm3d_device {
     // the case (pres_pc32, pres_pc64).
     FastPoisson<double> *fp64 = nullptr;
     FastPoisson<float> *fp32 = nullptr;
+    bool pc_ready[2] = {false, false};   // the FP64 and the FP32 one is built (ready_preconditioner)
     WidenedPreconditioner pc64;   // FP32 preconditioner under an FP64 Krylov solve
     // IBM3D_MIXED32 pressure solve on double-float vectors: a view of
     // kpres's buffers, the solution vector and the FP32 multigrid behind it.
@@ -322,6 +323,7 @@ void release_device(ibm3d_device *d) {
     d->fp64 = nullptr;
     delete d->fp32;
     d->fp32 = nullptr;
+    d->pc_ready[0] = d->pc_ready[1] = false;
     d->pc64.release();
     d->gm.release();
     d->kmom.release();
@@ -856,71 +858,45 @@ bool build_ops(IBMSolver *sv) {
     return cuda_check(sv, cudaStreamSynchronize(d->s), "operator tables");
 }
 
-// Tables of the momentum sweeps (momsweep.h), and the fast-diagonalisation
-// preconditioners (fastpoisson.h) of the pressure solves that their axes and
-// the body (FP_NEAR) allow: in FP32 all of them; in FP64, where the transforms
-// are bound by the FP64 pipe, always without a body (one iteration instead of
-// 5-18) and with one up to kBodyOps operations per application.  FP64 steps
-// against the multigrid's (ms): boxes 64x48x40 2.8, 3.9; 95x61x47 4.6, 5.0;
-// sphere 96x64x64 (0.10e9 operations) 3.1, 5.2; 120x96x88 (0.37e9) 6.3, 9.3;
-// 128x96x96 (0.45e9) 6.8, 9.3; four kinds of boxes 128x96x96 10.3-11.2,
-// 11.5-12.2; a sphere on asymmetric axes 112x80x80 (0.46e9) 6.3, 7.8; sphere
-// 136x100x100 (0.54e9) 11.1, 10.7; boxes 17.8, 12.7; sphere 144x104x104
-// (0.65e9) 13.4, 10.9; asymmetric 128x96x96 (0.91e9) 10.4, 9.7; 192x128x128
-// (1.6e9) 21, 15.  FP32 is faster up to the largest measured, asymmetric axes
-// (twice the operations) included: spheres 256^3 16-19 against 31-33,
-// 512x256x256 34-45, 68-86, cavities 384^3 27-31, 115-273.
-// A caller who sets the coarsening (IBMSolver_set_coarsening) asks for the
-// multigrid, in either precision.
-constexpr double kBodyOps = 0.5e9;
-
-bool build_sweeps_and_poisson(IBMSolver *sv) {
+// The grid, the body and its ghost rows as the momentum sweeps' and the
+// preconditioner's tables take them; false, with the status set, on failure.
+bool fast_geometry(IBMSolver *sv, FastPoissonGeom &h) {
     ibm3d_device *d = sv->dev;
     const Grid &g = d->g;
     const int Ns[3] = {sv->Nx, sv->Ny, sv->Nz};
     const double *KM[3] = {sv->kx_W, sv->ky_S, sv->kz_D}, *KP[3] = {sv->kx_E, sv->ky_N, sv->kz_U};
     const double *D[3] = {sv->dx, sv->dy, sv->dz};
-    FastPoissonGeom h;
     for (int a = 0; a < 3; a++) {
         h.km[a].assign(KM[a] + 2, KM[a] + 2 + Ns[a]);
         h.kp[a].assign(KP[a] + 2, KP[a] + 2 + Ns[a]);
         h.d[a].assign(D[a] + 2, D[a] + 2 + Ns[a]);
     }
     h.flag.resize(g.ncell);
-    bool body = false;
-    for (long long P = 0; P < g.ncell; P++) {
-        h.flag[P] = (uint8_t)sv->flag[P];
-        body = body || h.flag[P] != FLUID;
-    }
+    for (long long P = 0; P < g.ncell; P++) h.flag[P] = (uint8_t)sv->flag[P];
     const int ng = d->nghost;
     h.gcell.resize(ng);
     h.gidx.resize(8 * (size_t)ng);
     h.gwself.resize(ng);
-    if (ng > 0) {
-        cudaMemcpyAsync(h.gcell.data(), d->gargs.cell, sizeof(int) * ng, cudaMemcpyDeviceToHost, d->s);
-        cudaMemcpyAsync(h.gidx.data(), d->g_gidx, sizeof(int) * 8 * ng, cudaMemcpyDeviceToHost, d->s);
-        cudaMemcpyAsync(h.gwself.data(), d->g_gwself, sizeof(double) * ng, cudaMemcpyDeviceToHost, d->s);
-        if (!cuda_check(sv, cudaStreamSynchronize(d->s), "preconditioner tables")) return false;
-    }
+    if (ng == 0) return true;
+    cudaMemcpyAsync(h.gcell.data(), d->gargs.cell, sizeof(int) * ng, cudaMemcpyDeviceToHost, d->s);
+    cudaMemcpyAsync(h.gidx.data(), d->g_gidx, sizeof(int) * 8 * ng, cudaMemcpyDeviceToHost, d->s);
+    cudaMemcpyAsync(h.gwself.data(), d->g_gwself, sizeof(double) * ng, cudaMemcpyDeviceToHost, d->s);
+    return cuda_check(sv, cudaStreamSynchronize(d->s), "preconditioner tables");
+}
+
+// Tables of the momentum sweeps (momsweep.h).
+bool build_sweeps(IBMSolver *sv) {
+    ibm3d_device *d = sv->dev;
+    FastPoissonGeom h;
+    if (!fast_geometry(sv, h)) return false;
     std::vector<double> ks[3];
     for (int a = 0; a < 3; a++)
-        for (int q = 0; q < Ns[a]; q++) ks[a].push_back(h.km[a][q] + h.kp[a][q]);
+        for (size_t q = 0; q < h.km[a].size(); q++) ks[a].push_back(h.km[a][q] + h.kp[a][q]);
     const double *const kp[3] = {ks[0].data(), ks[1].data(), ks[2].data()};
-    if (d->msweep.setup(d->s, g, kp, h.flag.data(), d->gargs.cell, h.gcell.data(), h.gidx.data(), ng) != 0) {
-        set_status(sv, IBM3D_ECUDA, "momentum sweep tables failed");
-        return false;
-    }
-    auto make = [&](auto *&fp, auto &A, double max_ops) {
-        fp = new std::remove_reference_t<decltype(*fp)>();
-        const int rc = fp->setup(d->s, d->A64, A, h, max_ops);
-        if (rc != 0) {
-            delete fp;
-            fp = nullptr;
-        }
-        if (rc < 0) set_status(sv, IBM3D_ECUDA, "preconditioner setup failed");
-        return rc >= 0;
-    };
-    return d->mg_asked || (make(d->fp32, d->A32, INFINITY) && make(d->fp64, d->A64, body ? kBodyOps : INFINITY));
+    if (d->msweep.setup(d->s, d->g, kp, h.flag.data(), d->gargs.cell, h.gcell.data(), h.gidx.data(), d->nghost) == 0)
+        return true;
+    set_status(sv, IBM3D_ECUDA, "momentum sweep tables failed");
+    return false;
 }
 
 MGGeometry mg_geometry(const IBMSolver *sv) {
@@ -960,6 +936,67 @@ GMG<T> *build_multigrid(IBMSolver *sv, const OpT<T> &A) {
     }
     mg->set_prof(&d->prof);
     return mg;
+}
+
+// The pressure preconditioner in one precision: the fast diagonalisation
+// (fastpoisson.h) where the axes and the body (FP_NEAR) allow it: in FP32
+// always; in FP64, where the transforms are bound by the FP64 pipe, always
+// without a body (one iteration instead of 5-18) and with one up to kBodyOps
+// operations per application.  Otherwise the multigrid.  FP64 steps
+// against the multigrid's (ms): boxes 64x48x40 2.8, 3.9; 95x61x47 4.6, 5.0;
+// sphere 96x64x64 (0.10e9 operations) 3.1, 5.2; 120x96x88 (0.37e9) 6.3, 9.3;
+// 128x96x96 (0.45e9) 6.8, 9.3; four kinds of boxes 128x96x96 10.3-11.2,
+// 11.5-12.2; a sphere on asymmetric axes 112x80x80 (0.46e9) 6.3, 7.8; sphere
+// 136x100x100 (0.54e9) 11.1, 10.7; boxes 17.8, 12.7; sphere 144x104x104
+// (0.65e9) 13.4, 10.9; asymmetric 128x96x96 (0.91e9) 10.4, 9.7; 192x128x128
+// (1.6e9) 21, 15.  FP32 is faster up to the largest measured, asymmetric axes
+// (twice the operations) included: spheres 256^3 16-19 against 31-33,
+// 512x256x256 34-45, 68-86, cavities 384^3 27-31, 115-273.
+// A caller who sets the coarsening (IBMSolver_set_coarsening) asks for the
+// multigrid, in either precision.
+constexpr double kBodyOps = 0.5e9;
+
+template <typename T>
+bool build_preconditioner(IBMSolver *sv, const OpT<T> &A, FastPoisson<T> *&fp, GMG<T> *&mg) {
+    ibm3d_device *d = sv->dev;
+    if (!d->mg_asked) {
+        FastPoissonGeom h;
+        if (!fast_geometry(sv, h)) return false;
+        const bool body = std::any_of(h.flag.begin(), h.flag.end(), [](uint8_t f) { return f != FLUID; });
+        fp = new FastPoisson<T>();
+        const int rc = fp->setup(d->s, d->A64, A, h, body && sizeof(T) == 8 ? kBodyOps : INFINITY);
+        if (rc == 0) return true;
+        delete fp;
+        fp = nullptr;
+        if (rc < 0) {
+            set_status(sv, IBM3D_ECUDA, "preconditioner setup failed");
+            return false;
+        }
+    }
+    return (mg = build_multigrid<T>(sv, A)) != nullptr;
+}
+
+Preconditioner<float> *pres_pc32(const ibm3d_device *d);
+
+// The preconditioner of the current precision, built once: when the precision
+// is set after assembly, else before the first state or step.  (Assembly
+// cannot know which of the two will run; with both, boxes 95x61x47 took 15.1 ms
+// to be ready, with one 11.6.)  False, with the status set, on failure.
+bool ready_preconditioner(IBMSolver *sv) {
+    ibm3d_device *d = sv->dev;
+    bool &ready = d->pc_ready[d->precision != IBM3D_FP64];
+    if (ready) return true;
+    size_t free0 = 0, free1 = 0, total = 0;
+    cudaMemGetInfo(&free0, &total);
+    if (d->precision == IBM3D_FP64) {
+        ready = build_preconditioner(sv, d->A64, d->fp64, d->mg);
+    } else {
+        ready = build_preconditioner(sv, d->A32, d->fp32, d->mg32);
+        d->pc64.m32 = d->pcdf.m32 = pres_pc32(d);
+    }
+    cudaMemGetInfo(&free1, &total);
+    if (free0 > free1) d->dev_bytes += free0 - free1;
+    return ready;
 }
 
 void swap3(double *a[3], double *b[3]) {
@@ -1612,6 +1649,7 @@ bool check_ready(IBMSolver *sv, const char *fn) {
 
 void upload_state(IBMSolver *sv, const double *u1, const double *u2, const double *u3, const double *p) {
     ibm3d_device *d = sv->dev;
+    if (!ready_preconditioner(sv)) return;
     const size_t b = sizeof(double) * d->g.ncell;
     cudaMemcpyAsync(d->u[0], u1, b, cudaMemcpyHostToDevice, d->s);
     cudaMemcpyAsync(d->u[1], u2, b, cudaMemcpyHostToDevice, d->s);
@@ -1896,11 +1934,9 @@ void IBMSolver_assemble(IBMSolver *s) {
     d->kpres_df = dfloat_view(d->kpres);
     d->pp_df = dmalloc<dfloat>(s, g.ncell, "Krylov workspace");
     if (!d->pp_df) return;
-    if (!build_sweeps_and_poisson(s)) return;
+    if (!build_sweeps(s)) return;
     d->mg_levels = mg_level_count(mg_geometry(s), mg_config(d));
-    if (!d->fp64 && !(d->mg = build_multigrid<double>(s, d->A64))) return;
-    if (!d->fp32 && !(d->mg32 = build_multigrid<float>(s, d->A32))) return;
-    if (d->pc64.allocate(g.ncell, pres_pc32(d)) != 0) {
+    if (d->pc64.allocate(g.ncell, nullptr) != 0) {
         set_status(s, IBM3D_ECUDA, "preconditioner workspace allocation failed");
         return;
     }
@@ -2165,7 +2201,7 @@ void IBMSolver_export_result(IBMSolver *s, const char *name) {
 // exact FP64 state export_result writes beside the result file), else the
 // float fields, time and iter of "<name>.nc" as the reference does.
 void IBMSolver_init_flow_file(IBMSolver *s, const char *name) {
-    if (!check_ready(s, "IBMSolver_init_flow_file")) return;
+    if (!check_ready(s, "IBMSolver_init_flow_file") || !ready_preconditioner(s)) return;
     const std::string st = std::string(name) + ".ibm3d", nc = std::string(name) + ".nc";
     int r = read_state(s, st);
     const std::string used = r != 0 ? st : nc;
@@ -2304,6 +2340,7 @@ void account_step(ibm3d_device *d) {
 void iterate_prologue(IBMSolver *s) {
     ibm3d_device *d = s->dev;
     d->status = IBM3D_OK;
+    if (!ready_preconditioner(s)) return;
     prepare_samples(s, d->s, s->time, s->time + s->dt);
     fill_outer(s, 0);
     launch_interp_stag(d->s, d->g, d->ax[0], d->ax[1], d->ax[2], d->u, d->U);
@@ -2328,6 +2365,7 @@ void IBMSolver_iterate(IBMSolver *s, int num_time_steps, bool verbose) {
     ibm3d_device *d = s->dev;
     const double start_time = s->time;
     iterate_prologue(s);
+    if (d->status == IBM3D_ECUDA) return;
     struct timespec t0, t1;
     clock_gettime(CLOCK_REALTIME, &t0);
     for (int i = 1; i <= num_time_steps; i++) {
@@ -2551,6 +2589,7 @@ void IBMSolver_set_precision(IBMSolver *s, int mode) {
         return;
     }
     s->dev->precision = mode;
+    if (s->dev->assembled) ready_preconditioner(s);
 }
 
 void IBMSolver_get_field(IBMSolver *s, int field, double *out) {
@@ -2713,7 +2752,7 @@ double IBMSolver_time_iterate(IBMSolver *s, int nsteps) {
 // after each trial and at the end, so the run continues exactly as if the
 // tuner had not run.
 double IBMSolver_autotune(IBMSolver *s, int steps, int *best_out) {
-    if (!check_ready(s, "IBMSolver_autotune")) return -1;
+    if (!check_ready(s, "IBMSolver_autotune") || !ready_preconditioner(s)) return -1;
     ibm3d_device *d = s->dev;
     if (steps < 1) steps = 1;
     static const int cand[][5] = {{5, 5, 1, 1, 8},  {4, 4, 1, 1, 8},  {6, 6, 1, 1, 8},  {3, 3, 1, 1, 8},
@@ -2775,7 +2814,7 @@ double IBMSolver_autotune(IBMSolver *s, int steps, int *best_out) {
 }
 
 double IBMSolver_time_kernel(IBMSolver *s, int which, int reps, double *bytes) {
-    if (!check_ready(s, "IBMSolver_time_kernel")) return -1;
+    if (!check_ready(s, "IBMSolver_time_kernel") || !ready_preconditioner(s)) return -1;
     ibm3d_device *d = s->dev;
     const bool cold = (which & IBM3D_K_COLD) != 0;
     which &= ~IBM3D_K_COLD;
@@ -3044,6 +3083,7 @@ int IBMBatch_add(IBMBatch *b, IBMSolver *s) {
         fprintf(stderr, "error: IBMBatch_add: the solver must be assembled first\n");
         return -1;
     }
+    if (!ready_preconditioner(s)) return -1;
     for (IBMSolver *m : b->members)
         if (m == s) return 0;
     cudaEvent_t e;
@@ -3091,6 +3131,7 @@ bool batch_launch(IBMBatch *b) {
             b->run_start[q] = m->time;
             b->run_steps[q] = 0;
             iterate_prologue(m);
+            if (m->dev->status == IBM3D_ECUDA) return false;
             b->next_iter[q] = m->iter;
         }
         m->dev->status = IBM3D_OK;
@@ -3221,4 +3262,8 @@ void IBMBatch_set_combined(IBMBatch *b, int on) {
     batch_drop(b);
 }
 
-size_t IBMSolver_device_bytes(const IBMSolver *s) { return s && s->dev ? s->dev->dev_bytes : 0; }
+size_t IBMSolver_device_bytes(const IBMSolver *s) {
+    if (!s || !s->dev) return 0;
+    if (s->dev->assembled) ready_preconditioner(const_cast<IBMSolver *>(s));
+    return s->dev->dev_bytes;
+}

@@ -284,8 +284,11 @@ long long IBMSolver_kernel_launches(void);
 int IBMSolver_host_register(void *ptr, size_t bytes);
 int IBMSolver_host_unregister(void *ptr);
 
-/* Device memory the solver's assembly took (bytes; the drop in free device
-   memory across IBMSolver_assemble), for admission by HBM footprint. */
+/* Device memory the solver's assembly and the preconditioners set up so far
+   took (bytes; the drop in free device memory across them), for admission by
+   HBM footprint.  The pressure preconditioner of a precision is set up once, by
+   IBMSolver_set_precision after assembly, else by the first call that sets the
+   state, steps or asks for this figure. */
 size_t IBMSolver_device_bytes(const IBMSolver *);
 
 /* Device name of the solver's GPU (for logs). */
