@@ -507,29 +507,42 @@ __device__ inline bool publish_partials(const double (&v)[NV], double *partials,
 
 // Reduces every block's partials inside the last block: entries [0, NS)
 // are summed, entries [NS, NV) maxed (all maxed quantities are >= 0, so 0
-// is their identity).  Warp q takes entry q (q + the warps, ...): lane t
-// folds blocks t, t + 32, ... in that order and a fixed-shape tree combines
-// the lanes, so the result does not depend on block scheduling (bitwise
-// reproducible).  One warp per entry, not all of them for each: a warp's
-// FP64 addition takes the SM's FP64 unit 16 cycles, and 608 blocks' three
-// entries take 72 of them instead of 190.  Valid in thread 0; smem holds NV
-// doubles and must be free on entry.
+// is their identity).  Fixed orders and trees, so the result does not depend
+// on block scheduling (bitwise reproducible).  Up to RP_BLOCKS blocks warp q
+// takes entry q (q + the warps, ...): a warp's FP64 addition takes the SM's
+// FP64 unit 16 cycles, and 608 blocks' three entries take 72 of them instead
+// of 190.  Past that one warp's chain of loads is the longer part, and with
+// few entries all threads fold all of them (2 entries of 1,216, 2,200 and
+// 65,536 blocks: 7.2 against 6.1 us, 10.2 against 6.2, 172 against 59; 3
+// entries: 6.2 and 6.1, 8.2 and 6.7, 139 and 72; 608 blocks: 4.1 and 6.1).
+// From 6 entries on the two are within a tenth up to 17,600 blocks.  Valid in
+// thread 0; smem holds 8 * NV doubles, at most 8 warps a block, and must be
+// free on entry.
+constexpr int RP_BLOCKS = 1024;
+
 template <int NV, int NS>
 __device__ inline void reduce_partials(const double *partials, int nblocks, double (&out)[NV], double *smem) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    auto fold = [](int q, double x, double y) { return q < NS ? x + y : nanmax(x, y); };
+    if (NV <= 4 && nblocks > RP_BLOCKS) {
+        double v[NV];
+#pragma unroll
+        for (int q = 0; q < NV; q++) v[q] = 0.0;
+#pragma unroll 4
+        for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
+#pragma unroll
+            for (int q = 0; q < NV; q++) v[q] = fold(q, v[q], __ldcg(partials + (size_t)b * NV + q));
+        }
+        block_reduce<NV, NS>(v, out, smem);
+        return;
+    }
     for (int q = warp; q < NV; q += nw) {
         double x = 0.0;
         const double *p = partials + q;
 #pragma unroll 8
-        for (int b = lane; b < nblocks; b += 32) {
-            const double y = __ldcg(p + (size_t)b * NV);
-            x = q < NS ? x + y : nanmax(x, y);
-        }
+        for (int b = lane; b < nblocks; b += 32) x = fold(q, x, __ldcg(p + (size_t)b * NV));
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double y = __shfl_down_sync(0xffffffffu, x, o);
-            x = q < NS ? x + y : nanmax(x, y);
-        }
+        for (int o = 16; o > 0; o >>= 1) x = fold(q, x, __shfl_down_sync(0xffffffffu, x, o));
         if (lane == 0) smem[q] = x;
     }
     __syncthreads();
