@@ -505,48 +505,46 @@ __device__ inline bool publish_partials(const double (&v)[NV], double *partials,
     return last;
 }
 
-// Reduces every block's partials inside the last block: entries [0, NS)
-// are summed, entries [NS, NV) maxed (all maxed quantities are >= 0, so 0
-// is their identity).  Fixed orders and trees, so the result does not depend
-// on block scheduling (bitwise reproducible).  Up to RP_BLOCKS blocks warp q
-// takes entry q (q + the warps, ...): a warp's FP64 addition takes the SM's
-// FP64 unit 16 cycles, and 608 blocks' three entries take 72 of them instead
-// of 190.  Past that one warp's chain of loads is the longer part, and with
-// few entries all threads fold all of them (2 entries of 1,216, 2,200 and
-// 65,536 blocks: 7.2 against 6.1 us, 10.2 against 6.2, 172 against 59; 3
-// entries: 6.2 and 6.1, 8.2 and 6.7, 139 and 72; 608 blocks: 4.1 and 6.1).
-// From 6 entries on the two are within a tenth up to 17,600 blocks.  Valid in
-// thread 0; smem holds 8 * NV doubles, at most 8 warps a block, and must be
-// free on entry.
-constexpr int RP_BLOCKS = 1024;
+// Reduces every block's partials inside the last block (of RP_WARPS warps):
+// entries [0, NS) are summed, entries [NS, NV) maxed (all maxed quantities are
+// >= 0, so 0 is their identity).  Each entry has a share of the warps: lane t
+// of the share's warp s folds blocks 32 s + t, that plus 32 times the share,
+// ... in that order, and fixed-shape trees combine the lanes and the warps, so
+// the result does not depend on block scheduling (bitwise reproducible).  Not
+// all warps for each entry, since a warp's FP64 addition takes the SM's FP64
+// unit 16 cycles and every warp would run every entry's tree; not one warp
+// each, a chain of loads that grows with the blocks (2 entries of 608, 2,200 and
+// 65,536 blocks: 5.1, 9.7 and 170 us with a warp each, 4.1, 5.1 and 41 with
+// four; 3 entries: 4.1, 8.2 and 139, with two 4.1, 6.1 and 62).  Valid in thread 0;
+// smem holds 8 * NV doubles and must be free on entry.
+constexpr int RP_WARPS = 8;
 
 template <int NV, int NS>
 __device__ inline void reduce_partials(const double *partials, int nblocks, double (&out)[NV], double *smem) {
+    constexpr int SHARE = NV < RP_WARPS ? RP_WARPS / NV : 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     auto fold = [](int q, double x, double y) { return q < NS ? x + y : nanmax(x, y); };
-    if (NV <= 4 && nblocks > RP_BLOCKS) {
-        double v[NV];
-#pragma unroll
-        for (int q = 0; q < NV; q++) v[q] = 0.0;
-#pragma unroll 4
-        for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-#pragma unroll
-            for (int q = 0; q < NV; q++) v[q] = fold(q, v[q], __ldcg(partials + (size_t)b * NV + q));
-        }
-        block_reduce<NV, NS>(v, out, smem);
-        return;
-    }
-    for (int q = warp; q < NV; q += nw) {
+#pragma unroll 1
+    for (int w = warp; w < NV * SHARE; w += nw) {   // once; unrolled, it took 10 to 30 registers of every caller
+        const int q = w / SHARE, s = w % SHARE;
         double x = 0.0;
         const double *p = partials + q;
 #pragma unroll 8
-        for (int b = lane; b < nblocks; b += 32) x = fold(q, x, __ldcg(p + (size_t)b * NV));
+        for (int b = 32 * s + lane; b < nblocks; b += 32 * SHARE) x = fold(q, x, __ldcg(p + (size_t)b * NV));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) x = fold(q, x, __shfl_down_sync(0xffffffffu, x, o));
-        if (lane == 0) smem[q] = x;
+        if (lane == 0) smem[w] = x;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if constexpr (SHARE > 1) {   // 2, 4 or 8 warps each: the first lanes combine them
+        if (warp == 0) {
+            double x = lane < NV * SHARE ? smem[lane] : 0.0;
+#pragma unroll
+            for (int o = SHARE / 2; o > 0; o >>= 1) x = fold(lane / SHARE, x, __shfl_down_sync(0xffffffffu, x, o));
+#pragma unroll
+            for (int q = 0; q < NV; q++) out[q] = __shfl_sync(0xffffffffu, x, q * SHARE);
+        }
+    } else if (threadIdx.x == 0) {
 #pragma unroll
         for (int q = 0; q < NV; q++) out[q] = smem[q];
     }

@@ -1,5 +1,5 @@
 """reduce_partials (csrc/common.cuh) against sums and maxima on the host, exact in
-any order, below and past the number of blocks at which its form changes."""
+any order, from one block to many more than one warp folds at once."""
 import importlib
 import os
 import subprocess
