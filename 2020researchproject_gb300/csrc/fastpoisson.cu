@@ -631,14 +631,15 @@ __global__ void k_fp_sums(const double *__restrict__ l0, const double *__restric
 // identity rows of solid cells, and the swept values of the cells near the
 // body (cell[q] takes val[q]).  The three lists write different cells, and no
 // outer row reads a cell that another thread of the launch writes: a partner
-// that is solid gives its residual, the value its identity row takes, and a
+// that is solid (partners: there are some) gives its residual, the value its
+// identity row takes, and a
 // body whose swept cells are partners of outer rows gets its outer rows in
 // a launch of their own.
 template <typename T, typename S>
 __global__ void __launch_bounds__(256)
 k_fp_edges(const OpT<T> c, const S *__restrict__ r, T *z, const int *__restrict__ outer, const int nout,
-           const int *__restrict__ solid, const int nsolid, const int *__restrict__ cell, const T *__restrict__ val,
-           const int ncell, const int *gate) {
+           const int *__restrict__ solid, const int nsolid, const int partners, const int *__restrict__ cell,
+           const T *__restrict__ val, const int ncell, const int *gate) {
     const int t = blockIdx.x * 256 + threadIdx.x, ts = t - nout, tc = ts - nsolid;
     const int own = t < nout ? outer[t] : ts < nsolid ? solid[ts] : tc < ncell ? cell[tc] : -1;
     FP_GATE(gate);
@@ -666,7 +667,7 @@ k_fp_edges(const OpT<T> c, const S *__restrict__ r, T *z, const int *__restrict_
             Q += (2 * L - 1) * (face_low(f) ? s : -s);
         }
     }
-    T v = nsolid > 0 && c.flag[Q] == SOLID ? fp_value<T, S>(r[Q]) : z[Q];
+    T v = partners && c.flag[Q] == SOLID ? fp_value<T, S>(r[Q]) : z[Q];
     for (int q = n - 1; q >= 0; q--) {
         const BCRow<T> &F = c.bc[face[q]];
         const T rv = fp_value<T, S>(r[chain[q]]);
@@ -1142,8 +1143,11 @@ int FastPoisson<T>::setup(cudaStream_t s, const OpT<double> &A64, const OpT<T> &
         for (int j = 0; j < n[1]; j++) {
             const long long P0 = cidx(g, i, j, 0);
             for (int k = 0; k < n[2]; k++) {
-                if (h.flag[P0 + k] == SOLID) solid.push_back((int)(P0 + k));
-                else fluid += h.flag[P0 + k] == FLUID;
+                if (h.flag[P0 + k] == SOLID) {
+                    solid.push_back((int)(P0 + k));
+                    if (i < 2 || i >= n[0] - 2 || j < 2 || j >= n[1] - 2 || k < 2 || k >= n[2] - 2) solid_partners_ = 1;
+                }
+                fluid += h.flag[P0 + k] == FLUID;
             }
         }
     nsolid_ = (int)solid.size();
@@ -1526,7 +1530,7 @@ void FastPoisson<T>::run_tiled(cudaStream_t s, const S *r, T *z, const int *gate
     const int nout = A_.sw.nout;
     auto edges = [&](int outer, int solids, int swept) {
         launch_pdl(k_fp_edges<T, S>, (outer + solids + swept + 255) / 256, 256, 0, s, A_, r, z, A_.sw.outer, outer,
-                   (const int *)solid_, solids, patch_.P, (const T *)near_val_, swept, gate);
+                   (const int *)solid_, solids, solid_partners_, patch_.P, (const T *)near_val_, swept, gate);
         k++;
     };
     k += 3;

@@ -98,7 +98,7 @@ template <typename T>
 constexpr int FP_SWEEPS = sizeof(T) == 4 ? 16 : 8;
 // Side of the cubes the cells are cut by, and the cells a patch takes beyond
 // them.  FP64, bound by each SM's two multiply-adds per clock: more and
-// smaller patches (boxes 64x48x40: 3.38 ms per step, with FP32's sizes 3.75);
+// smaller patches (a tenth of the step on boxes 64x48x40 against FP32's sizes);
 // FP32 steps are within 3 % for sides of 6 and 8 and overlaps of 2 to 4.
 template <typename T>
 constexpr int FP_CUBE = sizeof(T) == 4 ? 8 : 5;
@@ -149,6 +149,7 @@ class FastPoisson : public Preconditioner<T> {
     T *near_val_ = nullptr;        // swept values of the cells near the body
     int npatch_ = 0, nghost_ = 0, nsolid_ = 0;
     int *solid_ = nullptr;
+    int solid_partners_ = 0;       // some lie in the two layers that outer rows take their partners from
     bool near_outer_ = false;
     int launches_ = 0;
     bool plane_ = false;           // the slice kernels (fastplane.cuh) take both ends
