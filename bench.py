@@ -304,14 +304,23 @@ def _vel_rel_l2(a, b):
     return (num / den) ** 0.5 if den > 0 else 0.0
 
 
-def step_roofline(ms_per_step, cells, k_u, k_p, mixed, les, peak):
-    """Step-level roofline from the algorithmic-bytes model of the step:
-    B_step = 336 + 3 k_u 144 + k_p B_pois (+ 104 with LES) bytes per cell,
-    B_pois = 492 with the FP64 preconditioner, 318 with the FP32 one, with k_u
-    and k_p the measured iterations per step (momentum per
-    component, pressure)."""
-    b_pois = 318.0 if mixed else 492.0
-    b_step = 336.0 + 3 * k_u * 144.0 + k_p * b_pois + (104.0 if les else 0.0)
+def step_roofline(ms_per_step, cells, k_u, k_p, mode, body, les, peak):
+    """Step-level roofline from the algorithmic bytes per cell of the kernels
+    that run: 336 for the explicit stages (+ 104 with LES); a momentum sweep
+    reads c and x and writes x (3 words per component, FP64 or FP32); a pressure
+    iteration is two operator sweeps and three vector updates (FP64 vectors: 168;
+    double-float ones, whose preconditioned vectors are FP32: 152) and two
+    applications of the preconditioner: the fast diagonalisation's gather, four
+    transforms and tridiagonal solve (56 in FP32, 112 in FP64), or, FP64 on the
+    sphere, a multigrid V-cycle (174).  k_u and k_p are the measured sweeps (per
+    component) and iterations per step.  None for the forms that refine."""
+    model = {"MIXED32": (12.0, 152.0, 56.0), "MIXED_MG": (24.0, 168.0, 56.0),
+             "FP64": (24.0, 168.0, 174.0 if body else 112.0)}.get(mode)
+    if model is None:
+        return None
+    sweep, krylov, application = model
+    b_pois = krylov + 2 * application
+    b_step = 336.0 + 3 * k_u * sweep + k_p * b_pois + (104.0 if les else 0.0)
     ach = b_step * cells / (ms_per_step / 1e3) / 1e9
     return {"B_step": round(b_step, 1), "k_u": round(k_u, 2), "k_p": round(k_p, 2), "achieved": round(ach, 1),
             "peak": peak, "unit": "GB/s", "frac": round(ach / peak, 4)}
@@ -342,7 +351,7 @@ def e2e_loop(ibm, s, steps, world):
 def fp64_step_ops(arm):
     """FP64 operations (FMA = 2) of one step of `arm` (fp64 / mixed) on the
     sphere, from the committed ncu summary (profiles/fp64_step_ops.txt:
-    '<arm> <workload> <ops> <momentum iterations> <pressure iterations>'
+    '<arm> <workload> <ops> <momentum sweeps> <pressure iterations>'
     of the profiled step), or None."""
     path = os.path.join(ROOT, "profiles", "fp64_step_ops.txt")
     try:
@@ -367,7 +376,7 @@ def fp64_roofline(arm, ms_per_step, fp64_tf):
     tf = ops / (ms_per_step / 1e3) / 1e12
     return {"fp64_ops_per_step": ops, "achieved_tflops": round(tf, 3), "peak_tflops": round(fp64_tf, 3),
             "frac": round(tf / fp64_tf, 4), "peak_source": "measured FP64 FMA rate (fma_rate_tflops)",
-            "ops_source": f"ncu, one profiled step ({it_u:g} momentum and {it_p:g} pressure iterations)"}
+            "ops_source": f"ncu, one profiled step ({it_u:g} momentum sweeps, {it_p:g} pressure iterations)"}
 
 
 def fp64_ops_per_launch(kernel):
@@ -455,9 +464,10 @@ def bench_gb300(args):
     mixed_mode = getattr(ibm, (mixed_arm["tuned"] or {}).get("mode", args.mixed_form))
 
     # --- step-level roofline of both arms (measured iterations per step).
+    mixed_name = (mixed_arm["tuned"] or {}).get("mode", args.mixed_form)
     roof_step = {a: step_roofline(arm["ms"] / args.steps, ncell, arm["iters"]["k_u"], arm["iters"]["k_p"],
-                                  a == "mixed", False, peak)
-                 for a, arm in (("mixed", mixed_arm), ("fp64", fp64_arm))}
+                                  mode, "stl" in case, "smag" in case, peak)
+                 for a, arm, mode in (("mixed", mixed_arm, mixed_name), ("fp64", fp64_arm, "FP64"))}
 
     # --- stage profile (host-sequenced step, CUDA events per stage).
     s.set_profiling(True)
