@@ -5,8 +5,12 @@
 // six Crank-Nicolson numbers, so a Jacobi sweep contracts the error by
 // rho = max sum k / (1 + sum k): 0.01-0.1 on the grids and time steps of the
 // workloads, where a sweep gains one or two digits.  A ghost row is solved
-// from the sweep's new fluid values (its ghost partners' old ones), an outer
-// row exactly.  A sweep reads c and x and writes x (12 bytes per cell and
+// from the sweep's new fluid values (its ghost partners' old ones), which
+// contracts by (1 - w_self) / (1 + w_self) at worst, and not at all where a
+// ghost's whole stencil is other ghosts; an outer row exactly (an extrapolated
+// outlet cancels the row's second difference along its axis, so rho still
+// bounds it).  No row's map exceeds 1 in the maximum norm: sweeps that do not
+// converge stall, they do not grow.  A sweep reads c and x and writes x (12 bytes per cell and
 // component in FP32) and reduces the residual of the x it reads, so the
 // stopping test costs no pass of its own; a BiCGSTAB iteration moves 84
 // bytes and gains about what two sweeps do.
